@@ -2,6 +2,7 @@
 #pragma once
 #include <cstring>
 
+#include "conetile.cuh"
 #include "graphloop.hpp"
 #include "icb_internal.hpp"
 
@@ -15,9 +16,12 @@ struct ConeFilter
   double r;
   int nnb = 0;           ///< neighbours in the stencil
   int hx = 0, hy = 0;    ///< the stencil's largest |di|, |dj|
-  DevBuf<int4> offs;     ///< (di,dj,dk, linear offset) per neighbour, element-index order
-  DevBuf<double> wts;    ///< r - distance
+  /// (di,dj,dk, linear offset) per neighbour, element-index order; then the
+  /// groups of columns of `cols`
+  DevBuf<int4> offs;
+  DevBuf<double> wts;    ///< r - distance per neighbour; then the weights of `cols`
   DevBuf<double> aa;     ///< sum of weights per element (dfilters_ds)
+  ConeCols cols;         ///< the stencil as columns (ncol 0: too large for the tiles)
 
   ConeFilter(const Dims &dims, const double *h, double radius, cudaStream_t s);
   /// densityFilter(x, false); with beta > 0 also the threshold projection and
