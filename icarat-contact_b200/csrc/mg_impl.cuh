@@ -247,15 +247,26 @@ __global__ void k_jacobi0(long long n, T c, const T *__restrict__ dinv,
 }
 
 // --------------------------------------------------------- coarse level ----
-/// Dense coarse matrix, row by row: the thread of free DOF (node n, c) adds
-/// the rows of its <= 8 elements in element order.  Each row has one writer,
-/// so the sums are deterministic (no atomics).
-template <typename T>
-__device__ __forceinline__ void dense_assemble_b(Dims d, KMat<double, 24> K, const T *__restrict__ E,
-                                 const int *__restrict__ dense, int n, double *A, const Blk &B)
+/// Dense coarse matrix, a warp per free DOF's row: lane t takes the t-th of
+/// the 3^dim neighbour nodes and adds, in element order, the elements that hold
+/// both nodes.  Each entry has one writer, so the sums are deterministic (no
+/// atomics); entries of the row that couple no element stay 0.  (A thread per
+/// row that added its elements' rows in memory took 53 us on the coarsest 3D
+/// grids, a chain of 8 x 24 dependent updates; a warp takes 5 us.)
+constexpr int kAssembleThreads = 128;
+inline unsigned assemble_blocks(const Dims &d)
 {
-  long long t = B.x * (long long)blockDim.x + threadIdx.x;
-  if(t >= (long long)d.nnode * d.dim)
+  return unsigned((d.nnode * d.dim * 32 + kAssembleThreads - 1) / kAssembleThreads);
+}
+template <typename T>
+__device__ __forceinline__ void dense_assemble_b(const Dims &d, const KMat<double, 24> &K,
+                                                 const T *__restrict__ E,
+                                                 const int *__restrict__ dense, int n, double *A,
+                                                 const Blk &B)
+{
+  const long long t = (B.x * (long long)blockDim.x + threadIdx.x) >> 5;
+  const int lane = threadIdx.x & 31;
+  if(t >= d.nnode * d.dim || lane >= (d.dim == 3 ? 27 : 9))
     return;
   const int c = int(t % d.dim);
   const long long nd = t / d.dim;
@@ -265,29 +276,39 @@ __device__ __forceinline__ void dense_assemble_b(Dims d, KMat<double, 24> K, con
   const int ne = d.dim == 2 ? 4 : 8, ndof = ne * d.dim;
   const long long sxy = (long long)d.sx * d.sy;
   const int i = int(nd % d.sx), j = int((nd / d.sx) % d.sy), k = d.dim == 3 ? int(nd / sxy) : 0;
-  double *Arow = A + (long long)row * n;
+  // the lane's node
+  const int oi = lane % 3 - 1, oj = lane / 3 % 3 - 1, ok = d.dim == 3 ? lane / 9 - 1 : 0;
+  if(unsigned(i + oi) >= unsigned(d.sx) || unsigned(j + oj) >= unsigned(d.sy) ||
+     unsigned(k + ok) >= unsigned(d.sz))
+    return;
+  double s[3] = {0.0, 0.0, 0.0};
   for(int dk = (d.dim == 3 ? -1 : 0); dk <= 0; dk++)
     for(int dj = -1; dj <= 0; dj++)
       for(int di = -1; di <= 0; di++)
       {
-        int ei = i + di, ej = j + dj, ek = k + dk;
+        const int ei = i + di, ej = j + dj, ek = k + dk;
         if(ei < 0 || ej < 0 || ek < 0 || ei >= d.nx || ej >= d.ny || (d.dim == 3 && ek >= d.nz))
           continue;
+        const int li = oi - di, lj = oj - dj, lk = ok - dk; // the node's corner in the element
+        if(unsigned(li) > 1u || unsigned(lj) > 1u || unsigned(lk) > 1u)
+          continue;
         const int a = ((-di) ^ (-dj)) + 2 * (-dj) + (d.dim == 3 ? 4 * (-dk) : 0);
+        const int l = (li ^ lj) + 2 * lj + 4 * lk;
         const double Ee = double(E[ei + (long long)ej * d.nx + (long long)ek * d.nx * d.ny]);
-        const long long base = ei + (long long)ej * d.sx + (long long)ek * sxy;
-        for(int l = 0; l < ne; l++)
-        {
-          int q = l & 3, top = l >> 2;
-          long long node = base + ((q == 1 || q == 2) ? 1 : 0) + (q >= 2 ? d.sx : 0) + top * sxy;
-          for(int c2 = 0; c2 < d.dim; c2++)
-          {
-            int col = dense[c2 * d.ld + node];
-            if(col >= 0)
-              Arow[col] += Ee * K.k[(a * d.dim + c) * ndof + l * d.dim + c2];
-          }
-        }
+#pragma unroll
+        for(int c2 = 0; c2 < 3; c2++)
+          if(c2 < d.dim)
+            s[c2] += Ee * K.k[(a * d.dim + c) * ndof + l * d.dim + c2];
       }
+  const long long node = nd + oi + (long long)oj * d.sx + ok * sxy;
+#pragma unroll
+  for(int c2 = 0; c2 < 3; c2++)
+    if(c2 < d.dim)
+    {
+      const int col = dense[c2 * d.ld + node];
+      if(col >= 0)
+        A[(long long)row * n + col] = s[c2];
+    }
 }
 template <typename T>
 __global__ void k_dense_assemble(Dims d, KMat<double, 24> K, const T *__restrict__ E,
@@ -296,73 +317,170 @@ __global__ void k_dense_assemble(Dims d, KMat<double, 24> K, const T *__restrict
   dense_assemble_b<T>(d, K, E, dense, n, A, this_block());
 }
 
-/// In-place Gauss-Jordan inversion of the SPD coarse matrix (no pivoting is
-/// needed for SPD).  One CTA; a non-positive pivot is recorded in *status
-/// and replaced by a tiny positive value so the preconditioner stays usable.
-/// SMEM: the matrix is worked on in shared memory (n^2 doubles, n <=
-/// kInvSmemMax) and copied back once; otherwise in place in global memory
-/// (L2-resident).  Warp w updates rows w, w + 32, ..., its lanes the columns.
-constexpr int kInvSmemMax = 160;
-template <bool SMEM>
+/// Gauss-Jordan inversion of the SPD coarse matrix (no pivoting is needed for
+/// SPD) by one CTA; a non-positive pivot is recorded in *status and replaced by
+/// a tiny positive value so the preconditioner stays usable.
+constexpr int kInvSmemMax = 160; ///< largest matrix of the register form
+constexpr int kInvThreads = 512; ///< its CTA: 16 warps
+/// The matrix lives in registers: thread (warp, lane) holds rows warp + 16 r
+/// and columns lane + 32 c.  The serial chain of n steps bounds it: a step is
+/// one barrier -- the warp that owns row k divides it by the pivot and puts it
+/// in shared memory, every warp takes column k's entries of its own rows by
+/// shuffle and updates them (with the matrix in shared memory and three
+/// barriers a step it took 333 us at n = 132; now 127 us.  Dividing the next
+/// row ahead of the other rows' updates took 139 us: more registers, spills).
+/// The loops over column blocks and row halves are unrolled, so every index
+/// into a is a constant.
+template <int NB>
+__device__ __forceinline__ void invert_spd_reg(int n, double *A, int *status, double (*srow)[160],
+                                               double *sred)
+{
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  double a[2 * NB][NB];
+#pragma unroll
+  for(int r = 0; r < 2 * NB; r++)
+#pragma unroll
+    for(int c = 0; c < NB; c++)
+    {
+      const int i = warp + 16 * r, j = lane + 32 * c;
+      a[r][c] = i < n && j < n ? A[i * n + j] : 0.0;
+    }
+  double dmax = 0.0;
+  for(int i = threadIdx.x; i < n; i += kInvThreads)
+    dmax = fmax(dmax, A[i * n + i]);
+#pragma unroll
+  for(int o = 16; o > 0; o >>= 1)
+    dmax = fmax(dmax, __shfl_xor_sync(0xffffffffu, dmax, o));
+  if(lane == 0)
+    sred[warp] = dmax;
+  __syncthreads();
+  for(int w = 0; w < kInvThreads / 32; w++)
+    dmax = fmax(dmax, sred[w]);
+#pragma unroll
+  for(int cb = 0; cb < NB; cb++)
+#pragma unroll
+    for(int h = 0; h < 2; h++)
+      for(int q = 0; q < 16; q++)
+      {
+        // k = 32 cb + 16 h + q: row 2 cb + h of warp q, column block cb of lane 16 h + q
+        const int k = 32 * cb + 16 * h + q, kl = 16 * h + q;
+        if(k >= n)
+          break;
+        double *sk = srow[k & 1];
+        if(warp == q)
+        {
+          double p = __shfl_sync(0xffffffffu, a[2 * cb + h][cb], kl);
+          if(!(p > 1e-14 * dmax))
+          {
+            if(lane == 0)
+              status[0] = k + 1;
+            p = fmax(1e-14 * dmax, DBL_MIN);
+          }
+#pragma unroll
+          for(int c = 0; c < NB; c++)
+            sk[lane + 32 * c] = (c == cb && lane == kl ? 1.0 : a[2 * cb + h][c]) / p;
+        }
+        __syncthreads();
+        double rk[NB];
+#pragma unroll
+        for(int c = 0; c < NB; c++)
+          rk[c] = sk[lane + 32 * c];
+#pragma unroll
+        for(int r = 0; r < 2 * NB; r++)
+        {
+          const double f = __shfl_sync(0xffffffffu, a[r][cb], kl);
+          const bool own = warp == q && r == 2 * cb + h;
+#pragma unroll
+          for(int c = 0; c < NB; c++)
+          {
+            const double v = c == cb && lane == kl ? 0.0 : a[r][c];
+            a[r][c] = own ? rk[c] : fma(-f, rk[c], v);
+          }
+        }
+      }
+#pragma unroll
+  for(int r = 0; r < 2 * NB; r++)
+#pragma unroll
+    for(int c = 0; c < NB; c++)
+    {
+      const int i = warp + 16 * r, j = lane + 32 * c;
+      if(i < n && j < n)
+        A[i * n + j] = a[r][c];
+    }
+  __syncthreads(); // srow and sred may be reused by the CTA's next matrix
+}
+/// REG: n <= kInvSmemMax, kInvThreads threads, the matrix in registers;
+/// otherwise 1024 threads, in place in global memory (L2-resident): warp w
+/// updates rows w, w + 32, ..., its lanes the columns.
+template <bool REG>
 __device__ __forceinline__ void invert_spd_b(int n, double *Ag, int *status)
 {
-  extern __shared__ double sA[];
-  __shared__ double rowk[1024];
-  __shared__ double colk[1024];
-  __shared__ double piv;
-  const int tid = threadIdx.x, nth = blockDim.x;
-  const int warp = tid >> 5, lane = tid & 31, nwarp = nth >> 5;
-  double *A = SMEM ? sA : Ag;
-  if(SMEM)
+  if constexpr(REG)
   {
-    for(int t = tid; t < n * n; t += nth)
-      sA[t] = Ag[t];
-    __syncthreads();
+    __shared__ double srow[2][160];
+    __shared__ double sred[kInvThreads / 32];
+    if(n <= 32)
+      invert_spd_reg<1>(n, Ag, status, srow, sred);
+    else if(n <= 64)
+      invert_spd_reg<2>(n, Ag, status, srow, sred);
+    else if(n <= 96)
+      invert_spd_reg<3>(n, Ag, status, srow, sred);
+    else if(n <= 128)
+      invert_spd_reg<4>(n, Ag, status, srow, sred);
+    else
+      invert_spd_reg<5>(n, Ag, status, srow, sred);
   }
-  double dmax = 0.0;
-  for(int i = 0; i < n; i++)
-    dmax = fmax(dmax, A[(long long)i * n + i]);
-  for(int k = 0; k < n; k++)
+  else
   {
-    if(tid == 0)
+    __shared__ double rowk[1024];
+    __shared__ double colk[1024];
+    __shared__ double piv;
+    const int tid = threadIdx.x, nth = blockDim.x;
+    const int warp = tid >> 5, lane = tid & 31, nwarp = nth >> 5;
+    double *A = Ag;
+    double dmax = 0.0;
+    for(int i = 0; i < n; i++)
+      dmax = fmax(dmax, A[(long long)i * n + i]);
+    for(int k = 0; k < n; k++)
     {
-      double p = A[(long long)k * n + k];
-      if(!(p > 1e-14 * dmax))
+      if(tid == 0)
       {
-        status[0] = k + 1;
-        p = fmax(1e-14 * dmax, DBL_MIN);
+        double p = A[(long long)k * n + k];
+        if(!(p > 1e-14 * dmax))
+        {
+          status[0] = k + 1;
+          p = fmax(1e-14 * dmax, DBL_MIN);
+        }
+        piv = p;
       }
-      piv = p;
+      __syncthreads();
+      const double p = piv;
+      for(int j = tid; j < n; j += nth)
+      {
+        rowk[j] = (j == k ? 1.0 : A[(long long)k * n + j]) / p;
+        colk[j] = A[(long long)j * n + k];
+      }
+      __syncthreads();
+      for(int i = warp; i < n; i += nwarp)
+      {
+        double *Ai = A + (long long)i * n;
+        const double f = colk[i];
+        if(i == k)
+          for(int j = lane; j < n; j += 32)
+            Ai[j] = rowk[j];
+        else
+          for(int j = lane; j < n; j += 32)
+            Ai[j] = (j == k ? 0.0 : Ai[j]) - f * rowk[j];
+      }
+      __syncthreads();
     }
-    __syncthreads();
-    const double p = piv;
-    for(int j = tid; j < n; j += nth)
-    {
-      rowk[j] = (j == k ? 1.0 : A[(long long)k * n + j]) / p;
-      colk[j] = A[(long long)j * n + k];
-    }
-    __syncthreads();
-    for(int i = warp; i < n; i += nwarp)
-    {
-      double *Ai = A + (long long)i * n;
-      const double f = colk[i];
-      if(i == k)
-        for(int j = lane; j < n; j += 32)
-          Ai[j] = rowk[j];
-      else
-        for(int j = lane; j < n; j += 32)
-          Ai[j] = (j == k ? 0.0 : Ai[j]) - f * rowk[j];
-    }
-    __syncthreads();
   }
-  if(SMEM)
-    for(int t = tid; t < n * n; t += nth)
-      Ag[t] = sA[t];
 }
-template <bool SMEM>
-__global__ void __launch_bounds__(1024) k_invert_spd(int n, double *Ag, int *status)
+template <bool REG>
+__global__ void __launch_bounds__(REG ? kInvThreads : 1024)
+    k_invert_spd(int n, double *Ag, int *status)
 {
-  invert_spd_b<SMEM>(n, Ag, status);
+  invert_spd_b<REG>(n, Ag, status);
 }
 
 /// x_c = A^-1 b_c over the free coarse DOFs (warp per row)
@@ -859,7 +977,7 @@ template <typename TK, typename TP> struct MgPcg
           fm[nd] |= uint8_t(1u << c);
     const int dim = hs.desc.dim;
     // default: coarsen until the grid has <= 160 DOFs, so the coarsest
-    // matrix is inverted in shared memory (600 DOFs cost 14.6 ms a density)
+    // matrix is inverted in registers (600 DOFs in memory cost 14.6 ms a density)
     const int cd = coarseDofs > 0 ? coarseDofs : kInvSmemMax;
     while(true)
     {
@@ -1012,18 +1130,10 @@ template <typename TK, typename TP> struct MgPcg
       KMat<double, 24> kd;
       for(int i = 0; i < 576; i++)
         kd.k[i] = double(C.K[i]);
-      k_dense_assemble<TP><<<nblocks(C.d.nnode * C.d.dim, 128), 128, 0, s>>>(C.d, kd, C.E,
+      k_dense_assemble<TP><<<assemble_blocks(C.d), kAssembleThreads, 0, s>>>(C.d, kd, C.E,
                                                                             cDense.p, nc, cA.p);
       if(nc <= kInvSmemMax)
-      {
-        // the shared-memory opt-in is a per-device function attribute shared by
-        // every host thread: always set it to the largest size, so threads of
-        // the batch runner never shrink it under one another's launch
-        ICB_CUDA(cudaFuncSetAttribute(k_invert_spd<true>,
-                                      cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      int(sizeof(double)) * kInvSmemMax * kInvSmemMax));
-        k_invert_spd<true><<<1, 1024, int(sizeof(double)) * nc * nc, s>>>(nc, cA.p, cStatus.p);
-      }
+        k_invert_spd<true><<<1, kInvThreads, 0, s>>>(nc, cA.p, cStatus.p);
       else
         k_invert_spd<false><<<1, 1024, 0, s>>>(nc, cA.p, cStatus.p);
       count_launch(2);

@@ -31,8 +31,12 @@ namespace
 {
 /// persistent CTAs take (record, block) items from the queue; block b of a
 /// record is block b of that problem's own launch (its own grid)
+template <class L> struct BatchThreads
+{
+  static constexpr int v = 256; ///< threads of a block at most
+};
 template <class L>
-__global__ void k_batch(const L *__restrict__ D, const int2 *__restrict__ map, BatchQueue q)
+__global__ void __launch_bounds__(BatchThreads<L>::v) k_batch(const L *__restrict__ D, const int2 *__restrict__ map, BatchQueue q)
 {
   batch_queue(
       D, map, q, [](const L &l) { return int(l.g.gx * l.g.gy * l.g.gz); },
@@ -242,14 +246,23 @@ template <typename T> struct AssembleL
   __device__ bool skip() const { return false; }
   __device__ void run(const Blk &B) const { dense_assemble_b<T>(d, K, E, dense, n, A, B); }
 };
-template <bool SMEM> struct InvertL
+template <bool REG> struct InvertL
 {
   Blk g;
   int n;
   double *A;
   int *status;
   __device__ bool skip() const { return false; }
-  __device__ void run(const Blk &) const { invert_spd_b<SMEM>(n, A, status); }
+  __device__ void run(const Blk &) const { invert_spd_b<REG>(n, A, status); }
+};
+
+template <> struct BatchThreads<InvertL<true>>
+{
+  static constexpr int v = kInvThreads;
+};
+template <> struct BatchThreads<InvertL<false>>
+{
+  static constexpr int v = 1024;
 };
 
 /// number of problems whose solve has not stopped
@@ -624,7 +637,6 @@ template <typename TP> struct BatchMg
     Builder<AssembleL<TP>> as;
     Builder<InvertL<true>> invS;
     Builder<InvertL<false>> invG;
-    int smemMax = 0;
     for(MG *m : M)
     {
       if(!m->nc)
@@ -641,23 +653,16 @@ template <typename TP> struct BatchMg
       a.dense = m->cDense.p;
       a.n = m->nc;
       a.A = m->cA.p;
-      as.add(a, nblocks(C.d.nnode * C.d.dim, 128));
+      as.add(a, assemble_blocks(C.d));
       if(m->nc <= kInvSmemMax)
-      {
         invS.add(InvertL<true>{{}, m->nc, m->cA.p, m->cStatus.p}, 1);
-        smemMax = std::max(smemMax, int(sizeof(double)) * m->nc * m->nc);
-      }
       else
         invG.add(InvertL<false>{{}, m->nc, m->cA.p, m->cStatus.p}, 1);
     }
     push(zA.finish(VB, 0, s, qc.p));
     push(zS.finish(VB, 0, s, qc.p));
-    push(as.finish(128, 0, s, qc.p));
-    if(smemMax > 0)
-      ICB_CUDA(cudaFuncSetAttribute(k_batch<InvertL<true>>,
-                                    cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    int(sizeof(double)) * kInvSmemMax * kInvSmemMax));
-    push(invS.finish(1024, smemMax, s, qc.p));
+    push(as.finish(kAssembleThreads, 0, s, qc.p));
+    push(invS.finish(kInvThreads, 0, s, qc.p));
     push(invG.finish(1024, 0, s, qc.p));
   }
 
