@@ -30,8 +30,9 @@
 //    before and after the coarse correction; the first pre-smoothing step
 //    starts from zero and needs no operator;
 //  * coarsest level (<= 160 DOFs by default): dense FP64 inverse built on
-//    the device (one CTA, Gauss-Jordan in shared memory), applied as a
-//    dense product.
+//    the device (one CTA, Gauss-Jordan in registers), applied as a dense
+//    product;
+//  * the levels of a few thousand nodes and fewer run as one launch (mgtail.cu).
 // The whole V-cycle is a fixed kernel sequence, so one PCG iteration with
 // its V-cycle is captured as the body of a CUDA graph's conditional WHILE
 // node, which the device repeats until the stop flag is set.

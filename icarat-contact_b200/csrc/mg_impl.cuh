@@ -10,7 +10,9 @@
 #include "batchq.cuh"
 #include "graphloop.hpp"
 #include "loopcache.hpp"
+#include "hex8modal.cuh"
 #include "mg.hpp"
+#include "mgtail.cuh"
 #include "reduce.cuh"
 
 namespace icb
@@ -936,6 +938,12 @@ template <typename TK, typename TP> struct MgPcg
   DevBuf<unsigned> counter;
   RedScratch red;
   KState *hst = nullptr;
+  /// the levels tail0 .. coarsest as one launch (mgtail.cu): its arguments
+  /// without the gate; tail0 < 0: none
+  int tail0 = -1;
+  TailArgs<TP> tail{};
+  TailK<TP> tailK{};
+  DevBuf<int> tailEntry;
   WhileGraph loop; ///< one FCG iteration, repeated on the device until stop
   GraphKey key;    ///< what `loop` bakes in besides this object's own buffers
 
@@ -1109,6 +1117,111 @@ template <typename TK, typename TP> struct MgPcg
     ICB_CUDA(cudaMemsetAsync(counter.p, 0, sizeof(unsigned), s));
     red = RedScratch{partials.p, counter.p, mb};
     ICB_CUDA(cudaMallocHost(&hst, sizeof(KState)));
+    buildTail(soa, s);
+  }
+
+  /// the tail: from the first level small enough (mgtail.cuh) down, as long as
+  /// the levels' element matrices are powers of two times one another
+  void buildTail(const std::vector<long long> &soa, cudaStream_t s)
+  {
+    tail0 = -1;
+    const int dim = lv[0].d.dim, KN = tail_k(dim), depth = int(lv.size());
+    if(nu > kTailSmooth || depth < 2)
+      return;
+    auto matrix = [&](int l, TailK<TP> &k) {
+      if(dim == 2)
+        std::copy(lv[l].K, lv[l].K + KN, k.v);
+      else
+      {
+        KModal<TP> m;
+        if(!modal_form_cached(lv[l].K, m))
+          return false; // the level runs on the dense kernel
+        std::copy(m.v, m.v + KN, k.v);
+      }
+      return true;
+    };
+    // upwards from the last smoothed level
+    tailK = TailK<TP>{};
+    if(!matrix(depth - 2, tailK) || !(tailK.v[0] > TP(0)))
+      return;
+    std::vector<TP> es(depth, TP(1));
+    int l0 = depth - 2;
+    for(int l = l0; l >= std::max(0, depth - kTailLevels); l--)
+    {
+      TailK<TP> k{};
+      if(lv[l].d.nnode > tail_nodes<TP>(dim) || !matrix(l, k))
+        break;
+      int e = 0;
+      const double q = double(k.v[0]) / double(tailK.v[0]);
+      bool same = std::frexp(q, &e) == 0.5;
+      for(int i = 0; same && i < KN; i++)
+        same = k.v[i] == TP(q * double(tailK.v[i]));
+      if(!same)
+        break;
+      es[l] = TP(q);
+      l0 = l;
+    }
+    // the longest tail that fits one CTA's shared memory
+    for(; l0 <= depth - 2; l0++)
+    {
+      TailArgs<TP> A{};
+      A.dim = dim;
+      A.nlev = depth - l0;
+      A.nu = nu;
+      A.nc = nc;
+      for(int k = 0; k < nu; k++)
+      {
+        A.c1[k] = TP(cc1[k]);
+        A.c2[k] = TP(cc2[k]);
+      }
+      for(int l = l0; l < depth; l++)
+      {
+        Level<TP> &L = lv[l];
+        TailLevel<TP> &t = A.lv[l - l0];
+        t.nx = L.d.nx, t.ny = L.d.ny, t.nz = L.d.nz;
+        t.sx = L.d.sx, t.sy = L.d.sy, t.sz = L.d.sz;
+        t.shx = L.sh.x, t.shy = L.sh.y, t.shz = dim == 3 ? L.sh.z : 0;
+        t.es = es[l];
+        t.ld = L.d.ld;
+        t.E = L.E;
+        t.dinv = L.dinv.p;
+      }
+      A.b = l0 ? lv[l0].b.p : rin();
+      A.out = l0 ? lv[l0].x.p : z.p;
+      A.Ainv = cA.p;
+      if(lv[l0].d.nnode <= tail_nodes<TP>(dim) && tail_plan(A))
+      {
+        std::vector<int> entry(std::max(nc, 1), 0);
+        const Dims &dc = lv.back().d;
+        for(int q = 0; q < nc; q++)
+        {
+          const long long c = soa[q] / dc.ld, nd = soa[q] % dc.ld;
+          entry[q] = tail_entry(A.lv[depth - 1 - l0], dim, int(c), int(nd % dc.sx),
+                                int(nd / dc.sx % dc.sy), int(nd / ((long long)dc.sx * dc.sy)));
+        }
+        tailEntry.alloc(entry.size());
+        ICB_CUDA(cudaMemcpyAsync(tailEntry.p, entry.data(), sizeof(int) * entry.size(),
+                                 cudaMemcpyHostToDevice, s));
+        ICB_CUDA(cudaStreamSynchronize(s));
+        A.entry = tailEntry.p;
+        tail = A;
+        tail0 = l0;
+        return;
+      }
+    }
+  }
+  /// whether the tail stands for its levels' own launches: it runs the
+  /// CUDA-core corner-mode operator, which the process-wide switches may exclude
+  bool useTail() const
+  {
+    return tail0 >= 0 && (lv[0].d.dim == 2 ||
+                          (hex8_modal_enabled() && !(sizeof(TP) == 4 && tc_operator_enabled())));
+  }
+  TailArgs<TP> tailArgs(const KState *gate) const
+  {
+    TailArgs<TP> A = tail;
+    A.gate = gate;
+    return A;
   }
 
   /// per density: coarse moduli, diagonals, coarse inverse
@@ -1158,6 +1271,11 @@ template <typename TK, typename TP> struct MgPcg
   void level(size_t l, const TP *b, TP *out, cudaStream_t s, const KState *gate)
   {
     Level<TP> &L = lv[l];
+    if(int(l) == tail0 && useTail())
+    {
+      launch_mg_tail(tailArgs(gate), tailK, s);
+      return;
+    }
     if(l + 1 == lv.size())
     {
       coarseSolve(b, out, s, gate);

@@ -13,8 +13,9 @@
 // (block_reduce_at) -- so each problem's iterates are bitwise those of its
 // own solve.  A problem that has converged is gated out (its blocks return at
 // once), as in its own solve.  Problems whose hierarchies have fewer levels
-// reach their coarsest solve earlier; a batched launch holds the problems
-// that take that step at that point of the V-cycle.
+// join at a later step of the descent; a batched launch holds the problems
+// that take that step, and the coarse levels of all of them are one launch
+// (mgtail.cu).
 #include <atomic>
 #include <chrono>
 #include <cstring>
@@ -431,15 +432,24 @@ template <typename TP> struct BatchMg
     int i;
     const TP *b;
     TP *out;
+    size_t l; ///< the problem's level
   };
+  /// levels of problem i that run as batched launches of their own (the rest
+  /// is its tail or its coarsest solve)
+  size_t ownLevels(int i) const
+  {
+    return M[i]->useTail() ? size_t(M[i]->tail0) : M[i]->lv.size() - 1;
+  }
 
-  /// append the batched steps of level(l, b, out) for the problems `set`
-  void emitLevel(size_t l, const std::vector<Inst> &set, bool gated, std::vector<Launch> &seq,
+  /// append the batched steps of level(l, b, out) for the problems `set`, `left`
+  /// launch levels above the last: a problem with fewer levels of its own joins
+  /// later, so that every tail is part of one launch
+  void emitLevel(size_t left, const std::vector<Inst> &set, bool gated, std::vector<Launch> &seq,
                  cudaStream_t s)
   {
-    std::vector<Inst> coarse, fine;
+    std::vector<Inst> coarse, fine, wait;
     for(const Inst &I : set)
-      (l + 1 == M[I.i]->lv.size() ? coarse : fine).push_back(I);
+      (ownLevels(I.i) - I.l < left ? wait : (left ? fine : coarse)).push_back(I);
     auto gate = [&](int i) -> const KState * { return gated ? M[i]->st.p : nullptr; };
     auto push = [&](Launch f) {
       if(f)
@@ -447,13 +457,31 @@ template <typename TP> struct BatchMg
     };
     if(!coarse.empty())
     {
-      // MgPcg::coarseSolve
+      // the tails, and MgPcg::coarseSolve of the problems without one
       Builder<FillL<TP>> f;
       Builder<DenseL<TP>> da;
+      struct Group ///< tails of one element matrix
+      {
+        TailK<TP> K;
+        std::vector<TailArgs<TP>> recs;
+        int smem = 0;
+      };
+      std::vector<Group> tails;
       int ncmax = 1;
       for(const Inst &I : coarse)
       {
         MG &m = *M[I.i];
+        if(m.useTail())
+        {
+          size_t g = 0;
+          while(g < tails.size() && std::memcmp(&tails[g].K, &m.tailK, sizeof m.tailK))
+            g++;
+          if(g == tails.size())
+            tails.push_back(Group{m.tailK, {}, 0});
+          tails[g].recs.push_back(m.tailArgs(gate(I.i)));
+          tails[g].smem = std::max(tails[g].smem, m.tail.smem);
+          continue;
+        }
         const Level<TP> &C = m.lv.back();
         const long long n = (long long)C.d.dim * C.d.ld;
         f.add(FillL<TP>{{}, n, TP(0), I.out}, unsigned(vblocks(n)));
@@ -465,9 +493,25 @@ template <typename TP> struct BatchMg
       }
       push(f.finish(VB, 0, s, qc.p));
       push(da.finish(256, int(sizeof(double)) * ncmax, s, qc.p));
+      for(const Group &t : tails)
+      {
+        const int nt = int(t.recs.size()), smem = t.smem;
+        auto D = std::make_shared<DevBuf<TailArgs<TP>>>(t.recs.size());
+        ICB_CUDA(cudaMemcpyAsync(D->p, t.recs.data(), sizeof(TailArgs<TP>) * t.recs.size(),
+                                 cudaMemcpyHostToDevice, s));
+        ICB_CUDA(cudaStreamSynchronize(s));
+        push([D, nt, smem, K = t.K](cudaStream_t cs) {
+          launch_mg_tail_batch<TP>(D->p, nt, 2, smem, K, cs);
+        });
+      }
     }
-    if(fine.empty())
+    if(left == 0)
       return;
+    if(fine.empty())
+    {
+      emitLevel(left - 1, wait, gated, seq, s);
+      return;
+    }
     struct Cur
     {
       TP *cur, *oth;
@@ -482,7 +526,7 @@ template <typename TP> struct BatchMg
       {
         const Inst &I = fine[k];
         MG &m = *M[I.i];
-        Level<TP> &L = m.lv[l];
+        Level<TP> &L = m.lv[I.l];
         const long long n = (long long)L.d.dim * L.d.ld;
         cs[k] = Cur{L.t.p, I.out};
         j0.add(Jacobi0L<TP>{{}, n, TP(m.cc2[0]), L.dinv.p, I.b, cs[k].cur, cs[k].oth, gate(I.i)},
@@ -496,7 +540,7 @@ template <typename TP> struct BatchMg
       {
         const Inst &I = fine[t];
         MG &m = *M[I.i];
-        Level<TP> &L = m.lv[l];
+        Level<TP> &L = m.lv[I.l];
         OpExtras<TP> ch;
         ch.mode = OP_CHEB;
         ch.b = I.b;
@@ -519,7 +563,7 @@ template <typename TP> struct BatchMg
       long long rowsR = 0;
       for(const Inst &I : fine)
       {
-        const dim3 g3 = grid3(M[I.i]->lv[l + 1].d);
+        const dim3 g3 = grid3(M[I.i]->lv[I.l + 1].d);
         rowsR += (long long)g3.x * g3.y * g3.z;
       }
       const unsigned kR = rows_per_item(rowsR, transfer_capacity(), 8);
@@ -527,8 +571,8 @@ template <typename TP> struct BatchMg
       {
         const Inst &I = fine[t];
         MG &m = *M[I.i];
-        Level<TP> &L = m.lv[l];
-        Level<TP> &Cn = m.lv[l + 1];
+        Level<TP> &L = m.lv[I.l];
+        Level<TP> &Cn = m.lv[I.l + 1];
         OpExtras<TP> res;
         res.mode = OP_RESIDUAL;
         res.b = I.b;
@@ -538,18 +582,19 @@ template <typename TP> struct BatchMg
         const dim3 g3 = grid3(Cn.d);
         rs.add(RestrictL<TP>{{}, L.d, Cn.d, Cn.sh, L.r.p, Cn.b.p, Cn.fix, gate(I.i), g3.y}, g3.x,
                transfer_rows(g3.y, kR), g3.z);
-        next.push_back(Inst{I.i, Cn.b.p, Cn.x.p});
+        next.push_back(Inst{I.i, Cn.b.p, Cn.x.p, I.l + 1});
       }
       push(op.finish(s, qc.p));
       push(rs.finish(kTB, 0, s, qc.p));
-      emitLevel(l + 1, next, gated, seq, s);
+      next.insert(next.end(), wait.begin(), wait.end());
+      emitLevel(left - 1, next, gated, seq, s);
     }
     {
       Builder<ProlongL<TP>> pr;
       long long rowsP = 0;
       for(const Inst &I : fine)
       {
-        const Dims &d = M[I.i]->lv[l].d;
+        const Dims &d = M[I.i]->lv[I.l].d;
         const dim3 g3 = grid3(d);
         rowsP += (long long)g3.x * prolong_row_blocks(d) * g3.z;
       }
@@ -559,8 +604,8 @@ template <typename TP> struct BatchMg
       {
         const Inst &I = fine[t];
         MG &m = *M[I.i];
-        Level<TP> &L = m.lv[l];
-        Level<TP> &Cn = m.lv[l + 1];
+        Level<TP> &L = m.lv[I.l];
+        Level<TP> &Cn = m.lv[I.l + 1];
         const dim3 g3 = grid3(L.d);
         const unsigned rows = kP * kProlongRows; // node rows per work item
         pr.add(ProlongL<TP>{{}, L.d, Cn.d, Cn.sh, Cn.x.p, cs[t].cur, L.fix, gate(I.i), rows}, g3.x,
@@ -574,7 +619,7 @@ template <typename TP> struct BatchMg
     for(size_t t = 0; t < fine.size(); t++)
       if(cs[t].cur != fine[t].out)
       {
-        const Level<TP> &L = M[fine[t].i]->lv[l];
+        const Level<TP> &L = M[fine[t].i]->lv[fine[t].l];
         const long long n = (long long)L.d.dim * L.d.ld;
         cp.add(CopyL<TP>{{}, n, cs[t].cur, fine[t].out, gate(fine[t].i)}, unsigned(vblocks(n)));
       }
@@ -696,11 +741,14 @@ template <typename TP> struct BatchMg
         in.add(InitL<double, TP>{{}, m.n, b[i], x[i], m.r.p, MG::same() ? nullptr : m.rP.p, m.red,
                                  m.st.p, tol[i], maxit[i]},
                unsigned(vblocks(m.n)));
-        all.push_back(Inst{i, m.rin(), m.z.p});
+        all.push_back(Inst{i, m.rin(), m.z.p, 0});
       }
       push(init, in.finish(VB, 0, s, qc.p));
     }
-    emitLevel(0, all, false, init, s);
+    size_t depth = 0;
+    for(int i = 0; i < n; i++)
+      depth = std::max(depth, ownLevels(i));
+    emitLevel(depth, all, false, init, s);
     {
       Builder<Init2L<double, TP>> in2;
       for(int i = 0; i < n; i++)
@@ -730,7 +778,7 @@ template <typename TP> struct BatchMg
       push(iter, op.finish(s, qc.p));
       push(iter, rb.finish(VB, 0, s, qc.p));
     }
-    emitLevel(0, all, true, iter, s);
+    emitLevel(depth, all, true, iter, s);
     {
       Builder<RzL<double, TP>> rz;
       Builder<XpL<double, TP>> xp;
