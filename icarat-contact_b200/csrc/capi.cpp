@@ -416,7 +416,7 @@ int icb_solve(icb_problem p, const icb_solve_opts *opts, icb_solve_info *info)
   {
     set_error(st == ICB_ERR_MAXITER     ? "iteration limit reached"
               : st == ICB_ERR_BREAKDOWN ? "CG breakdown (p.Kp <= 0)"
-              : st == ICB_ERR_TIMEOUT   ? "a tensor-core operator wait timed out inside the V-cycle"
+              : st == ICB_ERR_TIMEOUT   ? "a wait inside the solve timed out"
                                         : "non-finite values in the solve");
     return st;
   }

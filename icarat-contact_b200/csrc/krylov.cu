@@ -14,6 +14,7 @@
 #include <functional>
 
 #include "krylov.hpp"
+#include "pcgtile.hpp"
 #include "reduce.cuh"
 
 namespace icb
@@ -252,12 +253,44 @@ int reduction_blocks(const Dims &d)
 }
 
 // ------------------------------------------------------------ JacobiPcg --
+/// device time from construction to seconds(), on one stream
+struct SolveTimer
+{
+  cudaEvent_t e0 = nullptr, e1 = nullptr;
+  cudaStream_t s;
+  explicit SolveTimer(cudaStream_t stream) : s(stream)
+  {
+    ICB_CUDA(cudaEventCreate(&e0));
+    ICB_CUDA(cudaEventCreate(&e1));
+    ICB_CUDA(cudaEventRecord(e0, s));
+  }
+  SolveTimer(const SolveTimer &) = delete;
+  SolveTimer &operator=(const SolveTimer &) = delete;
+  ~SolveTimer()
+  {
+    if(e0)
+      cudaEventDestroy(e0);
+    if(e1)
+      cudaEventDestroy(e1);
+  }
+  double seconds() const
+  {
+    ICB_CUDA(cudaEventRecord(e1, s));
+    ICB_CUDA(cudaEventSynchronize(e1));
+    float ms = 0.f;
+    cudaEventElapsedTime(&ms, e0, e1);
+    return ms * 1e-3;
+  }
+};
+
 template <typename T> JacobiPcg<T>::JacobiPcg(const Dims &dims, cudaStream_t s) : d(dims)
 {
   n = (long long)d.dim * d.ld;
+  if(sizeof(T) == 8)
+    tiles = pcg_tiles(d);
   r.alloc(n);
   p.alloc(n);
-  q.alloc(n);
+  q.alloc(n + pcg_tile_slots(tiles)); // and the one-kernel form's exchange slots
   // every initialisation goes to the owner's stream: the blocking memset
   // would run on the legacy stream, which non-blocking streams do not wait for
   ICB_CUDA(cudaMemsetAsync(r.p, 0, r.bytes(), s));
@@ -286,6 +319,20 @@ int JacobiPcg<T>::solve(const T *K, const T *E, const uint8_t *fix, const T *inv
                         const T *b, T *x, double tol, int maxit, cudaStream_t s,
                         icb_solve_info *info)
 {
+  if constexpr(sizeof(T) == 8)
+  {
+    // a small problem's iterations as one kernel (pcgtile.cu)
+    if(tiles.ctas())
+    {
+      const SolveTimer timer(s);
+      k_pcg_init<T><<<vec_blocks(n), VB, 0, s>>>(n, b, x, r.p, p.p, invdiag, red, st.p, tol, maxit);
+      ICB_CUDA(cudaGetLastError());
+      count_launch();
+      launch_pcg_tiles(tiles, d, K, E, invdiag, x, r.p, p.p, q.p, st.p, s);
+      ICB_CUDA(cudaMemcpyAsync(hst, st.p, sizeof(KState), cudaMemcpyDeviceToHost, s));
+      return report(timer, info);
+    }
+  }
   const Dims dd = d;
   RedScratch *rp = &red;
   double *dp = dots.p;
@@ -302,10 +349,7 @@ int JacobiPcg<T>::solveOp(const std::function<void(cudaStream_t)> &op, const voi
                           const void *opKey1, const void *opKey2, const T *invdiag, const T *b,
                           T *x, double tol, int maxit, cudaStream_t s, icb_solve_info *info)
 {
-  cudaEvent_t e0, e1;
-  ICB_CUDA(cudaEventCreate(&e0));
-  ICB_CUDA(cudaEventCreate(&e1));
-  ICB_CUDA(cudaEventRecord(e0, s));
+  const SolveTimer timer(s);
   const int nb = vec_blocks(n);
   k_pcg_init<T><<<nb, VB, 0, s>>>(n, b, x, r.p, p.p, invdiag, red, st.p, tol, maxit);
   ICB_CUDA(cudaGetLastError());
@@ -345,18 +389,18 @@ int JacobiPcg<T>::solveOp(const std::function<void(cudaStream_t)> &op, const voi
     launched += loop.batch;
     count_launch(loop.graphNodes);
   }
-  ICB_CUDA(cudaEventRecord(e1, s));
-  ICB_CUDA(cudaEventSynchronize(e1));
-  float ms = 0.f;
-  cudaEventElapsedTime(&ms, e0, e1);
-  cudaEventDestroy(e0);
-  cudaEventDestroy(e1);
+  return report(timer, info);
+}
+
+template <typename T> int JacobiPcg<T>::report(const SolveTimer &timer, icb_solve_info *info)
+{
+  const double seconds = timer.seconds(); // waits for the stream
   if(info)
   {
     info->iters = hst->iter;
     info->matvecs = hst->matvecs;
     info->relres = hst->bb > 0 ? std::sqrt(hst->rr / hst->bb) : 0.0;
-    info->seconds = ms * 1e-3;
+    info->seconds = seconds;
     info->status = hst->status;
   }
   return hst->status;

@@ -4,6 +4,7 @@
 
 #include "graphloop.hpp"
 #include "icb_internal.hpp"
+#include "pcgtile.hpp"
 
 namespace icb
 {
@@ -15,6 +16,7 @@ namespace icb
 /// count excludes the converging iteration.  Every scalar stays on the device;
 /// the host only polls the stop flag once per batch of iterations, and a
 /// batch is one CUDA-graph launch.
+struct SolveTimer;
 template <typename T> struct JacobiPcg
 {
   Dims d;
@@ -27,6 +29,7 @@ template <typename T> struct JacobiPcg
   KState *hst = nullptr; ///< pinned mirror
   WhileGraph loop; ///< host form: 16 iterations per launch
   GraphKey graphKey; ///< what `loop` bakes in besides this object's own buffers
+  PcgTiles tiles;    ///< the one-kernel form of solve(), when the grid is small enough
 
   JacobiPcg(const Dims &dims, cudaStream_t s);
   ~JacobiPcg();
@@ -40,6 +43,8 @@ template <typename T> struct JacobiPcg
   int solveOp(const std::function<void(cudaStream_t)> &op, const void *opKey0,
               const void *opKey1, const void *opKey2, const T *invdiag, const T *b, T *x,
               double tol, int maxit, cudaStream_t s, icb_solve_info *info);
+  /// wait for the solve and hand out what it left in hst
+  int report(const SolveTimer &timer, icb_solve_info *info);
 };
 
 /// Jacobi-PCG (FP64) on caller-supplied buffers, no graph, no allocation:

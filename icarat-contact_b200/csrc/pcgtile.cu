@@ -1,0 +1,626 @@
+// pcgtile.cu -- the Jacobi-PCG of a small problem as one cooperative kernel.
+//
+// Three kernels an iteration are bound by their launches when the vectors fit
+// on the chip: 14.8 us an iteration at 10k unknowns, 17.7 us at 81k.  Here every
+// CTA owns a box of nodes for the whole solve, with its part of x, r and D^-1,
+// the search direction on the box and a ring around it, and the moduli in shared
+// memory.  An iteration is two exchanges between the CTAs:
+//   q = K p on the box;                           exchange p.q
+//   r -= alpha q, z = D^-1 r published;           exchange r.r, r.z
+//   x += alpha p, p = z + beta p on the box and, from the neighbours' z, on
+//   the ring
+// An exchange is one store of the CTA's sum and one warp's poll of everybody's:
+// the slots hold a pattern that no sum takes until they are written, so the
+// value is its own flag, and each CTA adds the same values in the same order.
+// The published z are their own flags too, so nobody waits for a fence: what
+// orders the emptying of slots and of z against their next use is one fence an
+// iteration, taken while the second exchange's sums are on their way (see the
+// kernel).  What is left of an iteration is two round trips through L2, four
+// chains of FP64 additions and the element work.  An iteration, three kernels
+// against one: 120 x 40 (9,920 unknowns) 14.9 and 4.7 us, 60 x 20 x 20 (79,380) 17.9
+// and 7.7, 540 x 540 (585,360) 33.0 and 10.1, 48 x 46 x 45 (318,000) 26.5 and 16.4.
+//
+// The launch is cooperative (every CTA is resident), and every poll is bounded:
+// a CTA whose poll runs out marks the solve ICB_ERR_TIMEOUT and returns, and so
+// do the others when theirs run out.
+#include "pcgtile.hpp"
+
+#include <algorithm>
+#include <cfloat>
+#include <climits>
+
+#include "hex8modal.cuh"
+#include "reduce.cuh"
+
+namespace icb
+{
+namespace
+{
+/// threads of a CTA: one a node in 2D; in 3D two, one for the four elements
+/// below the node and one for the four above
+template <int DIM> constexpr int kThreads = DIM == 3 ? 384 : 256;
+template <int DIM> constexpr int kNodeThreads = DIM == 3 ? 192 : 256;
+/// doubles of a CTA's exchange slots: a 128-byte line of its own.  Lines that
+/// several CTAs write while all poll them move between the L2's halves with
+/// every write: an exchange of 117 CTAs takes 4.4 us with packed slots, 2.4 us
+/// with 32 bytes each and 1.6 us with a line each (1.1 us for 20 CTAs).
+constexpr int kSlot = kPcgTileSlot;
+constexpr int kTileSmem = 200 << 10;
+constexpr unsigned kPolls = 1u << 22; // about two seconds
+constexpr unsigned long long kEmpty = ~0ull;
+
+template <int DIM> struct ElemK;
+template <> struct ElemK<2>
+{
+  double k[64];
+  __device__ __forceinline__ double operator()(int r, int c) const { return k[r * 8 + c]; }
+};
+/// upper triangle (the full 24 x 24 matrix exceeds the constant bank's
+/// parameters)
+template <> struct ElemK<3>
+{
+  double k[300];
+  __device__ __forceinline__ double operator()(int r, int c) const
+  {
+    return r <= c ? k[r * 24 - r * (r - 1) / 2 + (c - r)]
+                  : k[c * 24 - c * (c - 1) / 2 + (r - c)];
+  }
+};
+
+/// a CTA's box and the layout of its shared memory
+template <int DIM> struct Box
+{
+  int x0, y0, z0, nx, ny, nz, own; // its nodes
+  int W, WH, pad;                  // padded box: row, plane, all
+  __device__ __forceinline__ int at(int i, int j, int k) const
+  {
+    return i + 1 + (j + 1) * W + (DIM == 3 ? (k + 1) * WH : 0);
+  }
+};
+
+__device__ __forceinline__ void slot_store(double *s, unsigned long long b)
+{
+  asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(s), "l"(b) : "memory");
+}
+__device__ __forceinline__ void slot_put(double *s, double v)
+{
+  // a NaN keeps being one, but not the empty pattern
+  slot_store(s, v != v ? 0x7ff8000000000000ull : (unsigned long long)__double_as_longlong(v));
+}
+/// acquire-release fence at GPU scope (__threadfence is sequentially consistent)
+__device__ __forceinline__ void fence_gpu() { asm volatile("fence.acq_rel.gpu;" ::: "memory"); }
+__device__ __forceinline__ unsigned long long slot_read(const double *s)
+{
+  unsigned long long b;
+  asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(b) : "l"(s) : "memory");
+  return b;
+}
+
+/// Replace v by its sum over all threads of all CTAs, values first .. first + NV
+/// - 1 of slot set `set`.  `clear` (may be NULL): the set to empty.  With it,
+/// a fence follows the CTA's own stores to the slots: whoever sees a later value
+/// of this CTA and fences too sees all its stores before this exchange.  False
+/// when a poll ran out (the same in all threads of the CTA).
+template <int NT, int NV>
+__device__ __forceinline__ bool exchange(double (&v)[NV], int first, double *set, double *clear,
+                                         double (*sw)[2], double *sres)
+{
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int G = gridDim.x, cta = blockIdx.x;
+#pragma unroll
+  for(int o = 16; o > 0; o >>= 1)
+#pragma unroll
+    for(int k = 0; k < NV; k++)
+      v[k] += __shfl_xor_sync(0xffffffffu, v[k], o);
+  if(lane == 0)
+#pragma unroll
+    for(int k = 0; k < NV; k++)
+      sw[warp][k] = v[k];
+  __syncthreads();
+  if(warp == 0)
+  {
+    static_assert(NT / 32 <= 16, "the warps' sums are added by 16 lanes");
+#pragma unroll
+    for(int k = 0; k < NV; k++)
+      v[k] = lane < NT / 32 ? sw[lane][k] : 0.0;
+#pragma unroll
+    for(int o = 8; o > 0; o >>= 1)
+#pragma unroll
+      for(int k = 0; k < NV; k++)
+        v[k] += __shfl_xor_sync(0xffffffffu, v[k], o);
+    if(lane == 0)
+#pragma unroll
+      for(int k = 0; k < NV; k++)
+        slot_put(set + cta * kSlot + first + k, v[k]);
+    if(clear)
+    {
+      if(lane < 3)
+        slot_store(clear + cta * kSlot + lane, kEmpty);
+      fence_gpu();
+    }
+    constexpr int PER = 8; // slots a lane polls: 256 CTAs at most
+    unsigned long long b[PER][NV];
+#pragma unroll
+    for(int q = 0; q < PER; q++)
+#pragma unroll
+      for(int k = 0; k < NV; k++)
+        b[q][k] = lane + 32 * q < G ? kEmpty : 0ull;
+    bool more = true;
+    for(unsigned n = 0; n < kPolls && more; n++)
+    {
+      more = false;
+#pragma unroll
+      for(int q = 0; q < PER; q++)
+#pragma unroll
+        for(int k = 0; k < NV; k++)
+          if(b[q][k] == kEmpty)
+          {
+            b[q][k] = slot_read(set + (lane + 32 * q) * kSlot + first + k);
+            more |= b[q][k] == kEmpty;
+          }
+      more = __any_sync(0xffffffffu, more);
+    }
+#pragma unroll
+    for(int k = 0; k < NV; k++)
+    {
+      double t[PER];
+#pragma unroll
+      for(int q = 0; q < PER; q++)
+        t[q] = __longlong_as_double((long long)b[q][k]);
+#pragma unroll
+      for(int o = PER / 2; o > 0; o >>= 1)
+#pragma unroll
+        for(int q = 0; q < o; q++)
+          t[q] += t[q + o];
+      v[k] = t[0];
+    }
+#pragma unroll
+    for(int o = 16; o > 0; o >>= 1)
+#pragma unroll
+      for(int k = 0; k < NV; k++)
+        v[k] += __shfl_xor_sync(0xffffffffu, v[k], o);
+    if(lane == 0)
+    {
+#pragma unroll
+      for(int k = 0; k < NV; k++)
+        sres[k] = v[k];
+      sres[2] = more ? 1.0 : 0.0;
+    }
+  }
+  __syncthreads();
+#pragma unroll
+  for(int k = 0; k < NV; k++)
+    v[k] = sres[k];
+  return sres[2] == 0.0;
+}
+
+/// q = (K p) at padded entry c0 of the box (2D): its four elements' products
+__device__ __forceinline__ void node_product2(const ElemK<2> &K, const double *p, const double *E,
+                                              const Box<2> &B, int c0, double (&q)[2])
+{
+  q[0] = q[1] = 0.0;
+#pragma unroll
+  for(int e = 0; e < 4; e++)
+  {
+    // element e: low corner at c0 - (ex, ey); the node is its corner (ex, ey)
+    const int ex = e & 1, ey = e >> 1, l = lnode(ex, ey);
+    const int base = c0 - ex - ey * B.W;
+    const double Ee = E[base];
+    double ue[8];
+#pragma unroll
+    for(int m = 0; m < 4; m++)
+#pragma unroll
+      for(int c = 0; c < 2; c++)
+        ue[lnode(m & 1, m >> 1) * 2 + c] = p[c * B.pad + base + (m & 1) + (m >> 1) * B.W];
+#pragma unroll
+    for(int c = 0; c < 2; c++)
+    {
+      double s = 0.0;
+#pragma unroll
+      for(int j = 0; j < 8; j++)
+        s = fma(K(l * 2 + c, j), ue[j], s);
+      q[c] = fma(Ee, s, q[c]);
+    }
+  }
+}
+
+/// q = the share of the four elements below (EZ = 1) or above (EZ = 0) the node
+/// at padded entry c0 in K p (3D), neighbour by neighbour: a neighbour's values
+/// are read once for all elements that hold it.  They are taken relative to the
+/// node's own (a rigid translation has no forces): the sums then do not cancel,
+/// as in the operator's corner-mode form (without that a 33 x 2 x 2 beam needed
+/// 794 iterations instead of 718), and the node's own columns drop out.
+template <int EZ>
+__device__ __forceinline__ void node_product3(const ElemK<3> &K, const double *p, const double *E,
+                                              const Box<3> &B, int c0, double (&q)[3])
+{
+  double u0[3], s[4][3];
+#pragma unroll
+  for(int c = 0; c < 3; c++)
+  {
+    u0[c] = p[c * B.pad + c0];
+#pragma unroll
+    for(int e = 0; e < 4; e++)
+      s[e][c] = 0.0;
+  }
+#pragma unroll
+  for(int mz = 0; mz < 2; mz++)
+#pragma unroll
+    for(int dy = -1; dy <= 1; dy++)
+#pragma unroll
+      for(int dx = -1; dx <= 1; dx++)
+      {
+        const int dz = mz - EZ;
+        if(dx == 0 && dy == 0 && dz == 0)
+          continue;
+        const int at = c0 + dx + dy * B.W + dz * B.WH;
+        double u[3];
+#pragma unroll
+        for(int c = 0; c < 3; c++)
+          u[c] = p[c * B.pad + at] - u0[c];
+#pragma unroll
+        for(int e = 0; e < 4; e++)
+        {
+          // element e: the node is its corner (ex, ey, EZ), the neighbour (mx, my, mz)
+          const int ex = e & 1, ey = e >> 1, mx = dx + ex, my = dy + ey;
+          if(mx < 0 || mx > 1 || my < 0 || my > 1)
+            continue;
+          const int l = lnode(ex, ey) + 4 * EZ, m = lnode(mx, my) + 4 * mz;
+#pragma unroll
+          for(int c = 0; c < 3; c++)
+#pragma unroll
+            for(int c2 = 0; c2 < 3; c2++)
+              s[e][c] = fma(K(l * 3 + c, m * 3 + c2), u[c2], s[e][c]);
+        }
+      }
+#pragma unroll
+  for(int c = 0; c < 3; c++)
+  {
+    q[c] = 0.0;
+#pragma unroll
+    for(int e = 0; e < 4; e++)
+      q[c] = fma(E[c0 - (e & 1) - (e >> 1) * B.W - EZ * B.WH], s[e][c], q[c]);
+  }
+}
+
+template <int DIM>
+__global__ void __launch_bounds__(kThreads<DIM>)
+    k_pcg_tiles(const __grid_constant__ ElemK<DIM> K, const Dims d, const PcgTiles T,
+                const double *__restrict__ E, const double *__restrict__ dinv,
+                double *__restrict__ x, double *__restrict__ r, double *p0, double *z, double *slots,
+                KState *st)
+{
+  constexpr int NT = kThreads<DIM>;
+  extern __shared__ __align__(16) double pcg_dyn[];
+  __shared__ double sw[NT / 32][2], sres[3];
+  __shared__ int nring;
+  const int G = gridDim.x, cta = blockIdx.x, tid = threadIdx.x;
+  // every CTA reads the state before any writes it (the last thing a solve does)
+  if(st->stop)
+    return;
+  const double thr = st->thr;
+  const int maxit = st->maxit;
+  double rz = st->rz, rr = st->rr;
+  Box<DIM> B;
+  const int cx = cta % T.px, cy = cta / T.px % T.py, cz = cta / (T.px * T.py);
+  B.x0 = cx * T.bx, B.y0 = cy * T.by, B.z0 = cz * T.bz;
+  B.nx = min(T.bx, d.sx - B.x0), B.ny = min(T.by, d.sy - B.y0), B.nz = min(T.bz, d.sz - B.z0);
+  B.own = B.nx * B.ny * B.nz;
+  B.W = T.bx + 2;
+  B.WH = DIM == 3 ? B.W * (T.by + 2) : 0;
+  B.pad = B.W * (T.by + 2) * (DIM == 3 ? T.bz + 2 : 1);
+  const int cap = T.bx * T.by * T.bz;
+  double *sp = pcg_dyn, *sE = sp + DIM * B.pad, *sx = sE + B.pad, *sr = sx + DIM * cap,
+         *sd = sr + DIM * cap, *sq = sd + DIM * cap, *sz = sq + DIM * cap;
+  // (padded entry, node) of the box's own nodes and of the ring's
+  int2 *sown = reinterpret_cast<int2 *>(sq + (DIM == 3 ? 2 : 1) * DIM * cap), *sring = sown + cap;
+  if(tid == 0)
+    nring = 0;
+  __syncthreads();
+  // the box and its ring: moduli and direction, 0 outside the grid
+  for(int t = tid; t < B.pad; t += NT)
+  {
+    const int row = t / B.W, i = t - row * B.W - 1;
+    const int k = DIM == 3 ? row / (T.by + 2) - 1 : 0;
+    const int j = row - (DIM == 3 ? (k + 1) * (T.by + 2) : 0) - 1;
+    const int gx = B.x0 + i, gy = B.y0 + j, gz = B.z0 + k;
+    const bool elem = unsigned(gx) < unsigned(d.nx) && unsigned(gy) < unsigned(d.ny) &&
+                      (DIM == 2 || unsigned(gz) < unsigned(d.nz));
+    sE[t] = elem ? E[gx + (long long)d.nx * (gy + (long long)d.ny * gz)] : 0.0;
+    const bool node = unsigned(gx) < unsigned(d.sx) && unsigned(gy) < unsigned(d.sy) &&
+                      unsigned(gz) < unsigned(d.sz);
+    const int g = gx + d.sx * (gy + d.sy * gz);
+#pragma unroll
+    for(int c = 0; c < DIM; c++)
+      sp[c * B.pad + t] = node ? __ldcg(p0 + c * d.ld + g) : 0.0;
+    if(node && !(unsigned(i) < unsigned(B.nx) && unsigned(j) < unsigned(B.ny) &&
+                 unsigned(k) < unsigned(B.nz)))
+      sring[atomicAdd(&nring, 1)] = make_int2(t, g); // any order: the entries are independent
+  }
+  for(int n = tid; n < B.own; n += NT)
+  {
+    const int row = n / B.nx, i = n - row * B.nx, k = row / B.ny, j = row - k * B.ny;
+    const int g = B.x0 + i + d.sx * (B.y0 + j + d.sy * (B.z0 + k));
+    sown[n] = make_int2(B.at(i, j, k), g);
+#pragma unroll
+    for(int c = 0; c < DIM; c++)
+    {
+      sx[c * cap + n] = 0.0;
+      sr[c * cap + n] = r[c * d.ld + g];
+      sd[c * cap + n] = dinv[c * d.ld + g];
+    }
+  }
+  __syncthreads();
+  // the state of the loop, the same in every thread of every CTA
+  int iter = 0, matvecs = 0, status = ICB_OK, conv = 0;
+  double alpha = 0.0, beta = 0.0, pq = 0.0;
+  for(int it = 0;; it++)
+  {
+    // slots: three sets in turn; published z: the buffers z and p0 in turn (p0
+    // was read by all before the first exchange).  Every CTA has read the last
+    // iteration's slots and z before it arrives at this one's first exchange, so
+    // both are emptied after that exchange and before the second one's fence.
+    // The next value this CTA puts (first exchange of it + 1) is read by all
+    // before their own fence (second exchange of it + 1), and only after that
+    // fence do they read the emptied z (end of it + 1) or slots (it + 2) again.
+    double *set = slots + (it % 3) * kSlot * G, *clear = slots + ((it + 2) % 3) * kSlot * G;
+    double *zcur = it & 1 ? p0 : z, *zold = it & 1 ? z : p0;
+    // q = K p and p.q on the box (constrained rows of q are 0)
+    double v[1] = {0.0};
+    if constexpr(DIM == 3)
+    {
+      double q[3];
+      constexpr int NN = kNodeThreads<3>;
+      if(tid >= NN)
+        for(int n = tid - NN; n < B.own; n += NN)
+        {
+          node_product3<1>(K, sp, sE, B, sown[n].x, q);
+#pragma unroll
+          for(int c = 0; c < 3; c++)
+            sq[c * cap + n] = q[c];
+        }
+      else
+        for(int n = tid; n < B.own; n += NN)
+        {
+          node_product3<0>(K, sp, sE, B, sown[n].x, q);
+#pragma unroll
+          for(int c = 0; c < 3; c++)
+            sz[c * cap + n] = q[c];
+        }
+      __syncthreads();
+    }
+    for(int n = tid; n < B.own; n += NT)
+    {
+      const int c0 = sown[n].x;
+      double q[DIM];
+      if constexpr(DIM == 2)
+        node_product2(K, sp, sE, B, c0, q);
+#pragma unroll
+      for(int c = 0; c < DIM; c++)
+      {
+        if constexpr(DIM == 3)
+          q[c] = sz[c * cap + n] + sq[c * cap + n];
+        if(sd[c * cap + n] == 0.0)
+          q[c] = 0.0;
+        sq[c * cap + n] = q[c];
+        v[0] += sp[c * B.pad + c0] * q[c];
+      }
+    }
+    bool ok = exchange<NT, 1>(v, 0, set, nullptr, sw, sres);
+    pq = v[0];
+    if(!ok)
+    {
+      status = ICB_ERR_TIMEOUT;
+      break;
+    }
+    matvecs++;
+    alpha = rz / pq;
+    if(!(pq > 0.0) || !isfinite(alpha))
+    {
+      status = ICB_ERR_BREAKDOWN;
+      break;
+    }
+    // r -= alpha q; z = D^-1 r for the neighbours; r.r and r.z
+    double w[2] = {0.0, 0.0};
+    for(int n = tid; n < B.own; n += NT)
+    {
+      const int g = sown[n].y;
+#pragma unroll
+      for(int c = 0; c < DIM; c++)
+      {
+        const double ri = sr[c * cap + n] - alpha * sq[c * cap + n];
+        sr[c * cap + n] = ri;
+        const double zi = sd[c * cap + n] * ri;
+        slot_put(zcur + c * d.ld + g, zi);
+        slot_store(zold + c * d.ld + g, kEmpty);
+        w[0] += ri * ri;
+        w[1] += ri * zi;
+      }
+    }
+    ok = exchange<NT, 2>(w, 1, set, clear, sw, sres);
+    if(!ok)
+    {
+      status = ICB_ERR_TIMEOUT;
+      break;
+    }
+    rr = w[0];
+    if(!isfinite(rr) || !isfinite(w[1]))
+    {
+      status = ICB_ERR_NAN;
+      break;
+    }
+    conv = rr < thr;
+    if(!conv)
+    {
+      beta = w[1] / rz;
+      rz = w[1];
+    }
+    // x += alpha p; p = z + beta p on the box, then on the ring
+    for(int n = tid; n < B.own; n += NT)
+    {
+      const int c0 = sown[n].x;
+#pragma unroll
+      for(int c = 0; c < DIM; c++)
+      {
+        const double pi = sp[c * B.pad + c0];
+        sx[c * cap + n] += alpha * pi;
+        sp[c * B.pad + c0] = sd[c * cap + n] * sr[c * cap + n] + beta * pi;
+      }
+    }
+    if(conv)
+      break;
+    iter++;
+    if(iter >= maxit)
+    {
+      status = ICB_ERR_MAXITER;
+      break;
+    }
+    bool late = false;
+    for(int t = tid; t < nring; t += NT)
+    {
+      const int2 e = sring[t];
+      unsigned long long b[DIM];
+      bool more = true;
+#pragma unroll
+      for(int c = 0; c < DIM; c++)
+        b[c] = kEmpty;
+      for(unsigned n = 0; n < kPolls && more; n++)
+      {
+        more = false;
+#pragma unroll
+        for(int c = 0; c < DIM; c++)
+          if(b[c] == kEmpty)
+          {
+            b[c] = slot_read(zcur + c * d.ld + e.y);
+            more |= b[c] == kEmpty;
+          }
+      }
+      late |= more;
+#pragma unroll
+      for(int c = 0; c < DIM; c++)
+        sp[c * B.pad + e.x] =
+            __longlong_as_double((long long)b[c]) + beta * sp[c * B.pad + e.x];
+    }
+    if(__syncthreads_or(late))
+    {
+      status = ICB_ERR_TIMEOUT;
+      break;
+    }
+  }
+  for(int n = tid; n < B.own; n += NT)
+  {
+    const int g = sown[n].y;
+#pragma unroll
+    for(int c = 0; c < DIM; c++)
+    {
+      x[c * d.ld + g] = sx[c * cap + n];
+      r[c * d.ld + g] = sr[c * cap + n];
+    }
+  }
+  if(tid == 0 && status == ICB_ERR_TIMEOUT)
+  {
+    st->status = ICB_ERR_TIMEOUT;
+    st->stop = 1;
+  }
+  else if(cta == 0 && tid == 0)
+  {
+    st->pq = pq;
+    st->alpha = alpha;
+    st->beta = beta;
+    st->rr = rr;
+    st->rz = rz;
+    st->iter = iter;
+    st->matvecs = matvecs;
+    st->conv = conv;
+    // a CTA that timed out has set its own status
+    if(st->status != ICB_ERR_TIMEOUT)
+      st->status = status;
+    st->stop = 1;
+  }
+}
+} // namespace
+
+PcgTiles pcg_tiles(const Dims &d)
+{
+  PcgTiles best;
+  long long bestCost = LLONG_MAX;
+  const int G = num_sms(), nc = d.dim;
+  // nodes a CTA takes at most: six (3D) or eight (2D) a thread; its shared memory
+  // ends near there, and 3D is still 1.6 times the three kernels' speed
+  const long long most = d.dim == 3 ? 6 * kNodeThreads<3> : 8 * kNodeThreads<2>;
+  if(G > 256 || d.nnode >= (1LL << 30))
+    return best; // the exchange polls 256 CTAs at most
+  for(int px = 1; px <= std::min(G, d.sx); px++)
+    for(int py = 1; px * py <= G && py <= d.sy; py++)
+    {
+      const int pzMost = d.dim == 3 ? std::min(G / (px * py), d.sz) : 1;
+      for(int pz = 1; pz <= pzMost; pz++)
+      {
+        PcgTiles t;
+        t.bx = (d.sx + px - 1) / px, t.by = (d.sy + py - 1) / py, t.bz = (d.sz + pz - 1) / pz;
+        // boxes that end up empty are not launched
+        t.px = (d.sx + t.bx - 1) / t.bx, t.py = (d.sy + t.by - 1) / t.by;
+        t.pz = (d.sz + t.bz - 1) / t.bz;
+        const long long own = (long long)t.bx * t.by * t.bz;
+        if(own > most)
+          continue;
+        const long long pad =
+            (long long)(t.bx + 2) * (t.by + 2) * (d.dim == 3 ? t.bz + 2 : 1);
+        const long long bytes = 8 * (pad * (nc + 1) + (d.dim == 3 ? 5 : 4) * nc * own) + 8 * pad;
+        if(bytes > kTileSmem)
+          continue;
+        // cycles of an iteration that depend on the cut: the element work, the
+        // ring, and the polls of two exchanges (measured slopes)
+        const long long cost = own * (d.dim == 3 ? 20 : 4) + (pad - own) * 3 + t.ctas() * 12;
+        if(cost < bestCost)
+        {
+          bestCost = cost;
+          best = t;
+          best.smem = int(bytes);
+        }
+      }
+    }
+  return best;
+}
+
+template <int DIM>
+static void run_tiles(const PcgTiles &t, const Dims &d, const ElemK<DIM> &K, const double *E,
+                      const double *invdiag, double *x, double *r, double *p, double *z,
+                      KState *st, cudaStream_t s)
+{
+  const size_t nsoa = size_t(DIM) * size_t(d.ld);
+  // the shared-memory opt-in is a per-device attribute shared by every host
+  // thread: always its largest value
+  ICB_CUDA(cudaFuncSetAttribute(k_pcg_tiles<DIM>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                kTileSmem));
+  double *slots = z + nsoa; // a multiple of 64 doubles past z: line-aligned
+  ICB_CUDA(cudaMemsetAsync(z, 0xff, sizeof(double) * (nsoa + pcg_tile_slots(t)), s)); // kEmpty
+  Dims dd = d;
+  PcgTiles tt = t;
+  ElemK<DIM> kk = K;
+  void *args[] = {&kk, &dd, &tt, &E, &invdiag, &x, &r, &p, &z, &slots, &st};
+  ICB_CUDA(cudaLaunchCooperativeKernel((const void *)k_pcg_tiles<DIM>, dim3(t.ctas()),
+                                       dim3(kThreads<DIM>), args, size_t(t.smem), s));
+  count_launch();
+}
+
+void launch_pcg_tiles(const PcgTiles &t, const Dims &d, const double *K, const double *E,
+                      const double *invdiag, double *x, double *r, double *p, double *z,
+                      KState *st, cudaStream_t s)
+{
+  if(d.dim == 2)
+  {
+    ElemK<2> k;
+    std::copy(K, K + 64, k.k);
+    run_tiles<2>(t, d, k, E, invdiag, x, r, p, z, st, s);
+  }
+  else
+  {
+    ElemK<3> k;
+    for(int i = 0, m = 0; i < 24; i++)
+      for(int j = i; j < 24; j++)
+        k.k[m++] = K[i * 24 + j];
+    run_tiles<3>(t, d, k, E, invdiag, x, r, p, z, st, s);
+  }
+}
+} // namespace icb
