@@ -1,6 +1,8 @@
-// conetile.cuh -- the 3D cone filter's stencil on shared-memory tiles.
+// conetile.cuh -- the cone filter's stencil on shared-memory tiles: the 3D filter
+// and the volume of the 2D OC update (opt.cu).
 //
-// The stencil {|offset * h| <= r} is a set of columns along z: column (di, dj) holds the offsets |dk| <= hk(di, dj)
+// The stencil {|offset * h| <= r} is a set of columns along the last axis (z; y in
+// 2D): column (di, dj) holds the offsets |dk| <= hk(di, dj)
 // with weights that depend on |di|, |dj| and |dk| only.  A thread sums R
 // consecutive outputs of one column of elements: per group of columns
 // (+-di, +-dj) it reads R + 2 hk tile values of each, adds the group's values
@@ -19,10 +21,11 @@ constexpr int kConeSmem = 100 << 10; ///< most shared memory of a tile (two CTAs
 /// the stencil as columns, on the device
 struct ConeCols
 {
-  const int4 *col = nullptr; ///< (di, dj, hk, first weight), di, dj >= 0, per group of columns
+  /// (di, dj, hk, first weight), di, dj >= 0, per group of columns; 2D: dj = 0
+  const int4 *col = nullptr;
   const double *w = nullptr; ///< per group hk + 1 weights, |dk| = 0 .. hk
   int ncol = 0;
-  int hx = 0, hy = 0, hz = 0; ///< halo of the tile
+  int hx = 0, hy = 0, hz = 0; ///< halo of the tile; 2D: hy = 0, hz along y
 };
 
 /// the tile of a 256-thread block: 32 x 8 x R outputs and its halo
@@ -123,6 +126,25 @@ template <int R> struct ConeTile
       column<HK, false, false>(p, di, djW, w, zs, acc);
   }
 
+  /// acc[r] += the stencil's sum around p + r zs in a tile of row width W
+  static __device__ __forceinline__ void sum_columns(const double *p, int W, int zs,
+                                                     const ConeCols &C, double (&acc)[R])
+  {
+    for(int c = 0; c < C.ncol; c++)
+    {
+      const int4 o = __ldg(C.col + c);
+      const double *w = C.w + o.w;
+      static_assert(kConeMaxHz == 4, "one case per half height");
+      switch(o.z)
+      {
+      case 0: columns<0>(p, o.x, o.y * W, w, zs, acc); break;
+      case 1: columns<1>(p, o.x, o.y * W, w, zs, acc); break;
+      case 2: columns<2>(p, o.x, o.y * W, w, zs, acc); break;
+      case 3: columns<3>(p, o.x, o.y * W, w, zs, acc); break;
+      default: columns<4>(p, o.x, o.y * W, w, zs, acc); break;
+      }
+    }
+  }
   /// acc[r] = sum over the stencil at outputs (lane, warp, z0 + r)
   static __device__ __forceinline__ void sums(const double *tile, const ConeCols &C,
                                               double (&acc)[R])
@@ -133,20 +155,7 @@ template <int R> struct ConeTile
 #pragma unroll
     for(int r = 0; r < R; r++)
       acc[r] = 0.0;
-    for(int c = 0; c < C.ncol; c++)
-    {
-      const int4 o = __ldg(C.col + c);
-      const double *w = C.w + o.w;
-      static_assert(kConeMaxHz == 4, "one case per half height");
-      switch(o.z)
-      {
-      case 0: columns<0>(t0, o.x, o.y * W, w, zs, acc); break;
-      case 1: columns<1>(t0, o.x, o.y * W, w, zs, acc); break;
-      case 2: columns<2>(t0, o.x, o.y * W, w, zs, acc); break;
-      case 3: columns<3>(t0, o.x, o.y * W, w, zs, acc); break;
-      default: columns<4>(t0, o.x, o.y * W, w, zs, acc); break;
-      }
-    }
+    sum_columns(t0, W, zs, C, acc);
   }
 
   /// f(r, element index) for this thread's outputs inside the grid

@@ -30,6 +30,7 @@
 #include "graphloop.hpp"
 #include "opt.hpp"
 #include "batchq.cuh"
+#include "exchange.cuh"
 #include "reduce.cuh"
 
 namespace icb
@@ -180,9 +181,9 @@ template <bool SENS>
 bool cone_tiled(const ConeFilter &F, const double *in, double *out, double beta, double T,
                 double *xhat, double *dxhat, cudaStream_t s)
 {
-  if(!F.cols.ncol)
-    return false;
   const Dims &d = F.d;
+  if(!F.cols.ncol || d.dim == 2)
+    return false;
   if((long long)((d.nx + 31) / 32) * ((d.ny + 7) / 8) * ((d.nz + 7) / 8) >= num_sms())
     launch_cone_tile<SENS, 8>(F, in, out, beta, T, xhat, dxhat, s);
   else
@@ -534,6 +535,180 @@ __global__ void k_oc_final(long long n, double *__restrict__ x, const double *__
   // the last evaluated lambda is the one whose result set l0 or l1 last
   double lam = st->lastLam;
   x[e] = oc_candidate(x[e], df[e], dg[e], lam, P.eta, P.move, xmin[e], xmax[e]);
+}
+
+/// The whole OC update of a 2D design as one cooperative kernel: a CTA takes
+/// every gridDim-th tile of 32 x 32 elements for all steps of the bisection.  A
+/// step was two launches inside a WHILE graph; here it is the tiles' work and one
+/// exchange between the CTAs.  An update (37 steps) takes 245 us less on 640 x 320
+/// elements and 105 us less on 120 x 40.
+///
+/// What a step needs of an element is staged once: h = (-df/dg)^eta x, so that the
+/// candidate at lambda is lambda^-eta h between its bounds, and the bounds.  A
+/// volume formed so differs from the element-wise form's in its last bits; the
+/// bisection only compares it with g, and the final design is oc_candidate's.  The
+/// stencil is summed by columns (conetile.cuh), four rows a thread.
+constexpr int kOcUpTiles = 4;           ///< tiles of a CTA at most (its shared memory)
+constexpr int kOcUpSmem = 200 << 10;
+constexpr int kOcUpSets = 4;            ///< slot sets of the exchanges (see the loop)
+__host__ __device__ inline int oc_up_cells(const ConeCols &C)
+{
+  return (kOcTW + 2 * C.hx) * (kOcTH + 2 * C.hz);
+}
+__device__ __forceinline__ double oc_power(double b, double eta)
+{
+  return eta == 0.5 ? sqrt(b) : pow(b, eta);
+}
+/// h and the bounds of element e
+__device__ __forceinline__ void oc_prep(double x, double df, double dg, double xmin, double xmax,
+                                        const OcParams &P, double &h, double &lo, double &hi)
+{
+  h = oc_power(fmax(0.0, -df / dg), P.eta) * x;
+  lo = fmax(xmin, (1.0 - P.move) * x);
+  hi = fmin(xmax, (1.0 + P.move) * x);
+}
+__device__ __forceinline__ double oc_bounded(double w, double lo, double hi)
+{
+  return w < lo ? lo : (w > hi ? hi : w);
+}
+/// this thread's share of the volume of a tile: elements (i, j0 .. j0 + 3), the
+/// candidates with their halo in buf (row width W)
+__device__ __forceinline__ double oc_tile_volume(const double *buf, int W, const ConeCols &C,
+                                                 const double (&aav)[4], const double (&volv)[4],
+                                                 const OcParams &P, double tb)
+{
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  double acc[4] = {0.0, 0.0, 0.0, 0.0}, v = 0.0;
+  ConeTile<4>::sum_columns(buf + (4 * warp + C.hz) * W + lane + C.hx, W, W, C, acc);
+#pragma unroll
+  for(int r = 0; r < 4; r++)
+  {
+    const double xf = acc[r] / aav[r];
+    const double xh = P.beta > 0.0 ? thresh_tb(xf, P.beta, P.T, tb) : xf;
+    v += xh * volv[r];
+  }
+  return v;
+}
+/// weight sums and volumes of the thread's four elements (volume 0 outside)
+__device__ __forceinline__ void oc_tile_weights(const Dims &d, int i, int j0,
+                                                const double *__restrict__ aa,
+                                                const double *__restrict__ vol, double (&aav)[4],
+                                                double (&volv)[4])
+{
+#pragma unroll
+  for(int r = 0; r < 4; r++)
+  {
+    const bool in = i < d.nx && j0 + r < d.ny;
+    const long long e = i + (long long)(j0 + r) * d.nx;
+    aav[r] = in ? __ldg(aa + e) : 1.0;
+    volv[r] = in ? __ldg(vol + e) : 0.0;
+  }
+}
+__global__ void __launch_bounds__(VB)
+    k_oc_update(Dims d, ConeCols C, const double *__restrict__ aa, double *x,
+                const double *__restrict__ df, const double *__restrict__ dg,
+                const double *__restrict__ xmin, const double *__restrict__ xmax,
+                const double *__restrict__ vol, OcParams P, double g, double *slots, OcState *st)
+{
+  extern __shared__ __align__(16) double oc_up_dyn[];
+  __shared__ double sw[VB / 32][2], sres[3];
+  const int G = gridDim.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int ntx = (d.nx + kOcTW - 1) / kOcTW, tiles = ntx * ((d.ny + kOcTH - 1) / kOcTH);
+  const int W = kOcTW + 2 * C.hx, cells = oc_up_cells(C);
+  // two buffers of candidates, then h and the bounds of every tile
+  double *cand = oc_up_dyn, *sh = cand + 2 * cells;
+  int nt = 0;
+  for(int t = blockIdx.x; t < tiles; t += G, nt++)
+  {
+    const int x0 = t % ntx * kOcTW, y0 = t / ntx * kOcTH;
+    double *h = sh + nt * 3 * cells, *lo = h + cells, *hi = lo + cells;
+    for(int q = threadIdx.x; q < cells; q += VB)
+    {
+      const int ty = q / W, i = x0 - C.hx + q - ty * W, j = y0 - C.hz + ty;
+      double hv = 0.0, lv = 0.0, uv = 0.0; // outside the grid: candidate 0
+      if(unsigned(i) < unsigned(d.nx) && unsigned(j) < unsigned(d.ny))
+      {
+        const long long e = i + (long long)j * d.nx;
+        oc_prep(x[e], df[e], dg[e], xmin[e], xmax[e], P, hv, lv, uv);
+      }
+      h[q] = hv;
+      lo[q] = lv;
+      hi[q] = uv;
+    }
+  }
+  // the bisection's state, the same in every thread of every CTA (OCSolver.hpp:33-60)
+  OcState S;
+  S.tanhTb = P.beta > 0.0 ? tanh(P.T * P.beta) : 0.0;
+  S.l0 = 0.0;
+  S.l1 = 1.0e4;
+  S.lambdaeps = 1.0e-5;
+  S.maxiter = 100;
+  S.counter = 0;
+  S.pad = 0;
+  S.g = g;
+  S.vol = 0.0;
+  S.lam = S.lastLam = 0.5 * (S.l1 + S.l0);
+  S.done = !((S.l1 - S.l0) / (S.l1 + S.l0) > S.lambdaeps && S.maxiter > S.counter);
+  bool dead = false;
+  for(int it = 0; !S.done; it++)
+  {
+    const double c = 1.0 / oc_power(S.lam, P.eta);
+    double v[1] = {0.0};
+    for(int k = 0; k < nt; k++)
+    {
+      const int t = blockIdx.x + k * G, x0 = t % ntx * kOcTW, y0 = t / ntx * kOcTH;
+      const double *h = sh + k * 3 * cells, *lo = h + cells, *hi = lo + cells;
+      const int i = x0 + lane, j0 = y0 + 4 * warp;
+      double aav[4], volv[4];
+      oc_tile_weights(d, i, j0, aa, vol, aav, volv);
+      // alternate buffers: the barrier below also frees the one before
+      double *buf = cand + (k & 1) * cells;
+      for(int q = threadIdx.x; q < cells; q += VB)
+        buf[q] = oc_bounded(h[q] * c, lo[q], hi[q]);
+      __syncthreads();
+      v[0] += oc_tile_volume(buf, W, C, aav, volv, P, S.tanhTb);
+    }
+    // set it + 2 was last polled at it - 2, by everyone before it arrived at it - 1:
+    // it is emptied now, this CTA's value of it + 1 comes after the fence, and
+    // everyone reads that value, and fences, before it polls set it + 2
+    if(!exchange<VB, 1>(v, 0, slots + (it % kOcUpSets) * kExSlot * G,
+                        slots + ((it + 2) % kOcUpSets) * kExSlot * G, sw, sres))
+    {
+      dead = true;
+      break;
+    }
+    S.lastLam = S.lam;
+    if(v[0] - S.g > 0.0)
+      S.l0 = S.lam;
+    else
+      S.l1 = S.lam;
+    S.counter++;
+    S.vol = v[0];
+    if(!((S.l1 - S.l0) / (S.l1 + S.l0) > S.lambdaeps && S.maxiter > S.counter))
+      S.done = 1;
+    else
+      S.lam = 0.5 * (S.l1 + S.l0);
+  }
+  // every CTA has staged its tiles, halo and all, before the first exchange
+  if(!dead)
+    for(int k = 0; k < nt; k++)
+    {
+      const int t = blockIdx.x + k * G;
+      const int i = t % ntx * kOcTW + lane, j0 = t / ntx * kOcTH + 4 * warp;
+#pragma unroll
+      for(int r = 0; r < 4; r++)
+        if(i < d.nx && j0 + r < d.ny)
+        {
+          const long long e = i + (long long)(j0 + r) * d.nx;
+          x[e] = oc_candidate(x[e], df[e], dg[e], S.lastLam, P.eta, P.move, xmin[e], xmax[e]);
+        }
+    }
+  if(threadIdx.x == 0 && (dead || blockIdx.x == 0))
+  {
+    S.done = dead ? -1 : 1;
+    if(dead || st->done != -1)
+      *st = S;
+  }
 }
 
 // ----------------------------------------------------------------- MMA ----
@@ -920,17 +1095,17 @@ ConeFilter::ConeFilter(const Dims &dims, const double *h, double radius, cudaStr
     hx = std::max(hx, std::abs(off[3 * t]));
     hy = std::max(hy, std::abs(off[3 * t + 1]));
   }
-  // the same stencil as columns along z (3D), when its tiles fit
+  // the same stencil as columns along the last axis, when its tiles fit
   std::vector<int4> cc;
   std::vector<double> cw;
-  for(int dj = 0; d.dim == 3 && dj <= R[1]; dj++)
+  for(int dj = 0; dj <= (d.dim == 3 ? R[1] : 0); dj++)
     for(int di = 0; di <= R[0]; di++)
     {
       const int first = int(cw.size());
-      for(int dk = 0; dk <= R[2]; dk++)
+      for(int dk = 0; dk <= R[d.dim - 1]; dk++)
       {
-        const double dx = di * h[0], dy = dj * h[1], dz = dk * h[2];
-        const double dist = std::sqrt(dx * dx + dy * dy + dz * dz);
+        const double dx = di * h[0], dy = (d.dim == 3 ? dj : dk) * h[1], dz = dk * h[2];
+        const double dist = std::sqrt(dx * dx + dy * dy + (d.dim == 3 ? dz * dz : 0.0));
         if(dist <= radius)
           cw.push_back(radius - dist);
       }
@@ -942,8 +1117,11 @@ ConeFilter::ConeFilter(const Dims &dims, const double *h, double radius, cudaStr
       cols.hy = std::max(cols.hy, dj);
       cols.hz = std::max(cols.hz, hk);
     }
-  if(cols.hz <= kConeMaxHz && (d.ny + 7) / 8 <= 65535 && (d.nz + 3) / 4 <= 65535 &&
-     ConeTile<8>::cells(cols) * int(sizeof(double)) <= kConeSmem)
+  const bool fits =
+      d.dim == 3 ? (d.ny + 7) / 8 <= 65535 && (d.nz + 3) / 4 <= 65535 &&
+                       ConeTile<8>::cells(cols) * int(sizeof(double)) <= kConeSmem
+                 : cols.hx <= kOcHalo;
+  if(cols.hz <= kConeMaxHz && fits)
   {
     cols.ncol = int(cc.size());
     nb4.insert(nb4.end(), cc.begin(), cc.end());
@@ -1016,6 +1194,23 @@ OcTiling oc_tiling(const Dims &d, const ConeFilter *cone)
   t.blocks = int(t.ntx) * ((d.ny + kOcTH - 1) / kOcTH);
   return t;
 }
+/// CTAs of the one-kernel update on a grid: no more than there are tiles or SMs;
+/// 0 for 3D grids and those with too many tiles a CTA
+int oc_update_ctas(const Dims &d)
+{
+  if(d.dim != 2)
+    return 0;
+  const long long tiles =
+      (long long)((d.nx + kOcTW - 1) / kOcTW) * ((d.ny + kOcTH - 1) / kOcTH);
+  const int G = std::min(num_sms(), kExCtas);
+  return tiles <= (long long)kOcUpTiles * G ? int(std::min<long long>(tiles, G)) : 0;
+}
+/// its shared memory: two buffers of candidates and three values a cell of its tiles
+int oc_update_smem(const Dims &d, const ConeCols &C, int ctas)
+{
+  const int tiles = ((d.nx + kOcTW - 1) / kOcTW) * ((d.ny + kOcTH - 1) / kOcTH);
+  return int(sizeof(double)) * oc_up_cells(C) * (2 + 3 * ((tiles + ctas - 1) / ctas));
+}
 } // namespace
 
 OcUpdater::OcUpdater(const Dims &dims, cudaStream_t s) : d(dims)
@@ -1031,7 +1226,9 @@ OcUpdater::OcUpdater(const Dims &dims, cudaStream_t s) : d(dims)
   counter.alloc(1);
   ICB_CUDA(cudaMemsetAsync(counter.p, 0, sizeof(unsigned), s));
   red = RedScratch{partials.p, counter.p, nb};
-  cand.alloc(std::max<long long>(d.nel, 1));
+  // the candidates; or the one-kernel form's slots
+  const int ctas = oc_update_ctas(d);
+  cand.alloc(std::max<long long>(std::max<long long>(d.nel, 1), kOcUpSets * kExSlot * ctas));
   ICB_CUDA(cudaMallocHost(&hst, sizeof(OcState)));
 }
 OcUpdater::~OcUpdater()
@@ -1051,6 +1248,10 @@ int OcUpdater::update(const ConeFilter *cone, double *x, const double *df, const
 
 int OcUpdater::finish()
 {
+  if(hst->done == -1)
+    throw Error{ICB_ERR_TIMEOUT, "a wait inside the OC update timed out"};
+  if(oneKernel)
+    return hst->counter;
   count_launch(1 + (loop.device ? (long long)hst->pad : 1) * loop.graphNodes);
   return hst->counter;
 }
@@ -1059,6 +1260,28 @@ void OcUpdater::launch(const ConeFilter *cone, double *x, const double *df, cons
                        double g, const double *xmin, const double *xmax, const double *vol,
                        const OcParams &P, cudaStream_t s)
 {
+  const int ctas = cone && cone->cols.ncol ? oc_update_ctas(d) : 0;
+  const int upSmem = ctas ? oc_update_smem(d, cone->cols, ctas) : 0;
+  oneKernel = ctas && upSmem <= kOcUpSmem;
+  if(oneKernel)
+  {
+    ICB_CUDA(cudaFuncSetAttribute(k_oc_update, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  kOcUpSmem));
+    double *slots = cand.p;
+    ICB_CUDA(cudaMemsetAsync(slots, 0xff, sizeof(double) * kOcUpSets * kExSlot * ctas, s));
+    ICB_CUDA(cudaMemsetAsync(st.p, 0, sizeof(OcState), s));
+    Dims dd = d;
+    ConeCols cc = cone->cols;
+    const double *aa = cone->aa.p;
+    OcParams Pu = P;
+    OcState *sp = st.p;
+    void *args[] = {&dd, &cc, &aa, &x, &df, &dg, &xmin, &xmax, &vol, &Pu, &g, &slots, &sp};
+    ICB_CUDA(cudaLaunchCooperativeKernel((const void *)k_oc_update, dim3(unsigned(ctas)), dim3(VB),
+                                         args, size_t(upSmem), s));
+    count_launch();
+    ICB_CUDA(cudaMemcpyAsync(hst, st.p, sizeof(OcState), cudaMemcpyDeviceToHost, s));
+    return;
+  }
   const int nb = vblocks(d.nel);
   k_oc_init<<<1, 1, 0, s>>>(st.p, g, P);
   count_launch();
@@ -1117,6 +1340,10 @@ struct OcBatch::Rec
   double *x;
   const double *df, *dg, *xmin, *xmax, *vol;
   double *xc; ///< the candidates of the step (the problem's OcUpdater::cand)
+  /// column form (cols.ncol > 0): h and the bounds of every element, nel each, and
+  /// one step item per tile that forms its candidates itself
+  ConeCols cols;
+  double *prep;
   OcParams P;
   RedScratch red;
   OcState *st;
@@ -1126,6 +1353,69 @@ struct OcBatch::Rec
 namespace
 {
 constexpr int kOcStepsPerLaunch = 8;
+
+/// the column form's h and bounds, once per update (work items as the candidates')
+__global__ void __launch_bounds__(VB)
+    k_oc_prep_batch(const OcBatch::Rec *__restrict__ R, const int2 *__restrict__ map, BatchQueue q)
+{
+  batch_queue(
+      R, map, q, [](const OcBatch::Rec &r) { return int(r.gxc); },
+      [](const OcBatch::Rec &r) { return !r.cols.ncol; },
+      [](const OcBatch::Rec &r, int b, bool) {
+        const long long nel = r.d.nel, base = (long long)b * VB * kCandPerThread + threadIdx.x;
+#pragma unroll 4
+        for(int k = 0; k < kCandPerThread; k++)
+        {
+          const long long e = base + (long long)k * VB;
+          if(e < nel)
+          {
+            double h, lo, hi;
+            oc_prep(r.x[e], r.df[e], r.dg[e], r.xmin[e], r.xmax[e], r.P, h, lo, hi);
+            r.prep[e] = h;
+            r.prep[nel + e] = lo;
+            r.prep[2 * nel + e] = hi;
+          }
+        }
+      });
+}
+/// one bisection step on a tile in the column form (k_oc_update's arithmetic):
+/// the candidates of the tile and its halo into shared memory, the volume, and
+/// in a problem's last block its bisection logic
+__device__ __forceinline__ void oc_step_cols_b(const OcBatch::Rec &r, int b, double *buf)
+{
+  if(r.st->done)
+    return;
+  const Dims &d = r.d;
+  const ConeCols &C = r.cols;
+  const double c = 1.0 / oc_power(r.st->lam, r.P.eta), tb = r.st->tanhTb;
+  const int x0 = int(unsigned(b) % r.ntx) * kOcTW, y0 = int(unsigned(b) / r.ntx) * kOcTH;
+  const int W = kOcTW + 2 * C.hx, cells = oc_up_cells(C);
+  double aav[4], volv[4];
+  oc_tile_weights(d, x0 + int(threadIdx.x & 31), y0 + 4 * int(threadIdx.x >> 5), r.aa, r.vol, aav,
+                  volv);
+  constexpr int U = 4;
+  for(int q0 = threadIdx.x; q0 < cells; q0 += VB * U)
+  {
+    double h[U], lo[U], hi[U];
+#pragma unroll
+    for(int u = 0; u < U; u++)
+    {
+      const int q = q0 + u * VB, ty = q / W, i = x0 - C.hx + q - ty * W, j = y0 - C.hz + ty;
+      const bool in = q < cells && unsigned(i) < unsigned(d.nx) && unsigned(j) < unsigned(d.ny);
+      const long long e = i + (long long)j * d.nx;
+      h[u] = in ? __ldg(r.prep + e) : 0.0;
+      lo[u] = in ? __ldg(r.prep + d.nel + e) : 0.0;
+      hi[u] = in ? __ldg(r.prep + 2 * d.nel + e) : 0.0;
+    }
+#pragma unroll
+    for(int u = 0; u < U; u++)
+      if(q0 + u * VB < cells)
+        buf[q0 + u * VB] = oc_bounded(h[u] * c, lo[u], hi[u]);
+  }
+  __syncthreads();
+  double v[1] = {oc_tile_volume(buf, W, C, aav, volv, r.P, tb)};
+  block_reduce_at<1>(v, r.red, FinOc{r.st, LoopCtl{}}, b, int(r.gx));
+}
 
 __global__ void k_oc_init_batch(const OcBatch::Rec *__restrict__ R, int n)
 {
@@ -1138,7 +1428,7 @@ __global__ void __launch_bounds__(VB, 4)
 {
   batch_queue(
       R, map, q, [](const OcBatch::Rec &r) { return int(r.gxc); },
-      [](const OcBatch::Rec &r) { return r.st->done != 0 || !r.P.useFilter; },
+      [](const OcBatch::Rec &r) { return r.st->done != 0 || !r.P.useFilter || r.cols.ncol; },
       [](const OcBatch::Rec &r, int b, bool) {
         oc_cand_chunk(r.d.nel, r.x, r.df, r.dg, r.xmin, r.xmax, r.P, r.st, r.xc,
                       (long long)b * VB * kCandPerThread);
@@ -1153,7 +1443,9 @@ __global__ void __launch_bounds__(VB, 4)
       [](const OcBatch::Rec &r) { return r.st->done != 0; },
       [](const OcBatch::Rec &r, int b, bool) {
         const Blk B{unsigned(b), 0, 0, r.gx, 1, 1};
-        if(r.tiled)
+        if(r.cols.ncol)
+          oc_step_cols_b(r, b, reinterpret_cast<double *>(oc_batch_dyn));
+        else if(r.tiled)
           oc_step_tile_b(r.d, r.hx, r.hy, r.ntx, r.off, r.w, r.nnb, r.aa, r.vol, r.xc, r.P, r.red,
                          r.st, LoopCtl{}, B, oc_batch_dyn);
         else
@@ -1209,8 +1501,14 @@ void OcBatch::build(const std::vector<OcBatchItem> &items, cudaStream_t s)
   n = int(items.size());
   recsHost.assign(sizeof(Rec) * std::max(n, 1), 0);
   Rec *R = reinterpret_cast<Rec *>(recsHost.data());
-  std::vector<int2> ms, mc, mf;
+  std::vector<int2> ms, mc, mp, mf;
   smemStep = 0;
+  size_t np = 0;
+  auto columns = [](const OcBatchItem &it) { return it.cone && it.cone->cols.ncol; };
+  for(const OcBatchItem &it : items)
+    np += columns(it) ? 3 * size_t(it.oc->d.nel) : 0;
+  prep.alloc(std::max<size_t>(np, 1));
+  np = 0;
   for(int i = 0; i < n; i++)
   {
     const OcBatchItem &it = items[i];
@@ -1223,7 +1521,17 @@ void OcBatch::build(const std::vector<OcBatchItem> &items, cudaStream_t s)
     r.hx = tl.hx;
     r.hy = tl.hy;
     r.ntx = tl.ntx;
-    smemStep = std::max(smemStep, tl.smem);
+    r.cols = ConeCols{};
+    r.prep = nullptr;
+    if(tl.tiled && columns(it))
+    {
+      r.cols = it.cone->cols;
+      r.prep = prep.p + np;
+      np += 3 * size_t(r.d.nel);
+      smemStep = std::max(smemStep, int(sizeof(double)) * oc_up_cells(r.cols));
+    }
+    else
+      smemStep = std::max(smemStep, tl.smem);
     r.off = it.cone ? it.cone->offs.p : nullptr;
     r.w = it.cone ? it.cone->wts.p : nullptr;
     r.nnb = it.cone ? it.cone->nnb : 0;
@@ -1240,7 +1548,7 @@ void OcBatch::build(const std::vector<OcBatchItem> &items, cudaStream_t s)
     for(unsigned b = 0; b < r.gx; b++)
       ms.push_back(make_int2(i, int(b)));
     for(unsigned b = 0; b < r.gxc; b++)
-      mc.push_back(make_int2(i, int(b)));
+      (r.cols.ncol ? mp : mc).push_back(make_int2(i, int(b)));
     for(long long b = 0; b < (r.d.nel + 255) / 256; b++)
       mf.push_back(make_int2(i, int(b)));
   }
@@ -1249,6 +1557,9 @@ void OcBatch::build(const std::vector<OcBatchItem> &items, cudaStream_t s)
   mapCand.alloc(std::max<size_t>(mc.size(), 1));
   if(!mc.empty())
     ICB_CUDA(cudaMemcpyAsync(mapCand.p, mc.data(), sizeof(int2) * mc.size(), cudaMemcpyHostToDevice, s));
+  mapPrep.alloc(std::max<size_t>(mp.size(), 1));
+  if(!mp.empty())
+    ICB_CUDA(cudaMemcpyAsync(mapPrep.p, mp.data(), sizeof(int2) * mp.size(), cudaMemcpyHostToDevice, s));
   mapFinal.alloc(std::max<size_t>(mf.size(), 1));
   if(!ms.empty())
     ICB_CUDA(cudaMemcpyAsync(mapStep.p, ms.data(), sizeof(int2) * ms.size(), cudaMemcpyHostToDevice, s));
@@ -1267,8 +1578,12 @@ void OcBatch::build(const std::vector<OcBatchItem> &items, cudaStream_t s)
   if(!hNotDone)
     ICB_CUDA(cudaMallocHost(&hNotDone, sizeof(int)));
   BatchQueue qs{qc.p, qc.p + 1, int(ms.size())}, qf{qc.p, qc.p + 1, int(mf.size())};
-  BatchQueue qa{qc.p, qc.p + 1, int(mc.size())};
+  BatchQueue qa{qc.p, qc.p + 1, int(mc.size())}, qp{qc.p, qc.p + 1, int(mp.size())};
+  itemsPrep = qp.items;
+  gridPrep = queue_grid((const void *)k_oc_prep_batch, VB, 0, qp);
+  chunkPrep = qp.chunk;
   itemsStep = qs.items;
+  candLaunched = qa.items > 0;
   itemsFinal = qf.items;
   gridCand = queue_grid((const void *)k_oc_cand_batch, VB, 0, qa);
   chunkCand = qa.chunk;
@@ -1288,7 +1603,8 @@ void OcBatch::build(const std::vector<OcBatchItem> &items, cudaStream_t s)
   const Rec *Rd = reinterpret_cast<const Rec *>(recs.p);
   for(int k = 0; k < kOcStepsPerLaunch; k++)
   {
-    k_oc_cand_batch<<<gridCand, VB, 0, cs>>>(Rd, mapCand.p, qa);
+    if(qa.items)
+      k_oc_cand_batch<<<gridCand, VB, 0, cs>>>(Rd, mapCand.p, qa);
     k_oc_step_batch<<<gridStep, VB, smemStep, cs>>>(Rd, mapStep.p, qs);
   }
   k_oc_gather<<<1, 256, 0, cs>>>(Rd, n, states.p, notDone.p);
@@ -1315,11 +1631,18 @@ void OcBatch::update(const std::vector<double> &g, const std::vector<OcParams> &
   k_oc_init_batch<<<(n + 127) / 128, 128, 0, s>>>(Rd, n);
   ICB_CUDA(cudaGetLastError());
   count_launch();
+  if(itemsPrep)
+  {
+    BatchQueue qp{qc.p, qc.p + 1, itemsPrep, chunkPrep};
+    k_oc_prep_batch<<<gridPrep, VB, 0, s>>>(Rd, mapPrep.p, qp);
+    ICB_CUDA(cudaGetLastError());
+    count_launch();
+  }
   // at most ICARAT's 100 bisection steps (the updates stop themselves)
   for(int steps = 0; steps <= 100; steps += kOcStepsPerLaunch)
   {
     ICB_CUDA(cudaGraphLaunch(exec, s));
-    count_launch(2 * kOcStepsPerLaunch + 1);
+    count_launch((candLaunched ? 2 : 1) * kOcStepsPerLaunch + 1);
     ICB_CUDA(cudaStreamSynchronize(s));
     if(*hNotDone == 0)
       break;

@@ -63,6 +63,7 @@ struct OcUpdater
   OcState *hst = nullptr;
   WhileGraph loop; ///< one bisection step, repeated on the device until done
   GraphKey key;     ///< what `loop` bakes in
+  bool oneKernel = false; ///< the last launch was the one-kernel form
 
   OcUpdater(const Dims &dims, cudaStream_t s);
   ~OcUpdater();
@@ -96,7 +97,8 @@ struct OcBatch
   int n = 0;
   std::vector<unsigned char> recsHost; ///< n records
   DevBuf<unsigned char> recs;
-  DevBuf<int2> mapStep, mapCand, mapFinal;
+  DevBuf<int2> mapStep, mapCand, mapPrep, mapFinal;
+  DevBuf<double> prep; ///< the column-form problems' h and bounds
   int smemStep = 0; ///< dynamic shared memory of the step launch (tiled problems)
   DevBuf<unsigned> qc;
   DevBuf<OcState> states;
@@ -104,7 +106,8 @@ struct OcBatch
   OcState *hst = nullptr;
   int *hNotDone = nullptr;
   int gridCand = 0, gridStep = 0, gridFinal = 0, chunkCand = 1, chunkStep = 1, chunkFinal = 1,
-      itemsStep = 0, itemsFinal = 0;
+      itemsStep = 0, itemsFinal = 0, gridPrep = 0, chunkPrep = 1, itemsPrep = 0;
+  bool candLaunched = false; ///< some problem is not in the column form
   cudaGraphExec_t exec = nullptr; ///< kStepsPerLaunch steps and the done count
   OcBatch() = default;
   OcBatch(const OcBatch &) = delete;

@@ -29,8 +29,8 @@
 #include <cfloat>
 #include <climits>
 
+#include "exchange.cuh"
 #include "hex8modal.cuh"
-#include "reduce.cuh"
 
 namespace icb
 {
@@ -40,14 +40,7 @@ namespace
 /// below the node and one for the four above
 template <int DIM> constexpr int kThreads = DIM == 3 ? 384 : 256;
 template <int DIM> constexpr int kNodeThreads = DIM == 3 ? 192 : 256;
-/// doubles of a CTA's exchange slots: a 128-byte line of its own.  Lines that
-/// several CTAs write while all poll them move between the L2's halves with
-/// every write: an exchange of 117 CTAs takes 4.4 us with packed slots, 2.4 us
-/// with 32 bytes each and 1.6 us with a line each (1.1 us for 20 CTAs).
-constexpr int kSlot = kPcgTileSlot;
 constexpr int kTileSmem = 200 << 10;
-constexpr unsigned kPolls = 1u << 22; // about two seconds
-constexpr unsigned long long kEmpty = ~0ull;
 
 template <int DIM> struct ElemK;
 template <> struct ElemK<2>
@@ -77,122 +70,6 @@ template <int DIM> struct Box
     return i + 1 + (j + 1) * W + (DIM == 3 ? (k + 1) * WH : 0);
   }
 };
-
-__device__ __forceinline__ void slot_store(double *s, unsigned long long b)
-{
-  asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(s), "l"(b) : "memory");
-}
-__device__ __forceinline__ void slot_put(double *s, double v)
-{
-  // a NaN keeps being one, but not the empty pattern
-  slot_store(s, v != v ? 0x7ff8000000000000ull : (unsigned long long)__double_as_longlong(v));
-}
-/// acquire-release fence at GPU scope (__threadfence is sequentially consistent)
-__device__ __forceinline__ void fence_gpu() { asm volatile("fence.acq_rel.gpu;" ::: "memory"); }
-__device__ __forceinline__ unsigned long long slot_read(const double *s)
-{
-  unsigned long long b;
-  asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(b) : "l"(s) : "memory");
-  return b;
-}
-
-/// Replace v by its sum over all threads of all CTAs, values first .. first + NV
-/// - 1 of slot set `set`.  `clear` (may be NULL): the set to empty.  With it,
-/// a fence follows the CTA's own stores to the slots: whoever sees a later value
-/// of this CTA and fences too sees all its stores before this exchange.  False
-/// when a poll ran out (the same in all threads of the CTA).
-template <int NT, int NV>
-__device__ __forceinline__ bool exchange(double (&v)[NV], int first, double *set, double *clear,
-                                         double (*sw)[2], double *sres)
-{
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int G = gridDim.x, cta = blockIdx.x;
-#pragma unroll
-  for(int o = 16; o > 0; o >>= 1)
-#pragma unroll
-    for(int k = 0; k < NV; k++)
-      v[k] += __shfl_xor_sync(0xffffffffu, v[k], o);
-  if(lane == 0)
-#pragma unroll
-    for(int k = 0; k < NV; k++)
-      sw[warp][k] = v[k];
-  __syncthreads();
-  if(warp == 0)
-  {
-    static_assert(NT / 32 <= 16, "the warps' sums are added by 16 lanes");
-#pragma unroll
-    for(int k = 0; k < NV; k++)
-      v[k] = lane < NT / 32 ? sw[lane][k] : 0.0;
-#pragma unroll
-    for(int o = 8; o > 0; o >>= 1)
-#pragma unroll
-      for(int k = 0; k < NV; k++)
-        v[k] += __shfl_xor_sync(0xffffffffu, v[k], o);
-    if(lane == 0)
-#pragma unroll
-      for(int k = 0; k < NV; k++)
-        slot_put(set + cta * kSlot + first + k, v[k]);
-    if(clear)
-    {
-      if(lane < 3)
-        slot_store(clear + cta * kSlot + lane, kEmpty);
-      fence_gpu();
-    }
-    constexpr int PER = 8; // slots a lane polls: 256 CTAs at most
-    unsigned long long b[PER][NV];
-#pragma unroll
-    for(int q = 0; q < PER; q++)
-#pragma unroll
-      for(int k = 0; k < NV; k++)
-        b[q][k] = lane + 32 * q < G ? kEmpty : 0ull;
-    bool more = true;
-    for(unsigned n = 0; n < kPolls && more; n++)
-    {
-      more = false;
-#pragma unroll
-      for(int q = 0; q < PER; q++)
-#pragma unroll
-        for(int k = 0; k < NV; k++)
-          if(b[q][k] == kEmpty)
-          {
-            b[q][k] = slot_read(set + (lane + 32 * q) * kSlot + first + k);
-            more |= b[q][k] == kEmpty;
-          }
-      more = __any_sync(0xffffffffu, more);
-    }
-#pragma unroll
-    for(int k = 0; k < NV; k++)
-    {
-      double t[PER];
-#pragma unroll
-      for(int q = 0; q < PER; q++)
-        t[q] = __longlong_as_double((long long)b[q][k]);
-#pragma unroll
-      for(int o = PER / 2; o > 0; o >>= 1)
-#pragma unroll
-        for(int q = 0; q < o; q++)
-          t[q] += t[q + o];
-      v[k] = t[0];
-    }
-#pragma unroll
-    for(int o = 16; o > 0; o >>= 1)
-#pragma unroll
-      for(int k = 0; k < NV; k++)
-        v[k] += __shfl_xor_sync(0xffffffffu, v[k], o);
-    if(lane == 0)
-    {
-#pragma unroll
-      for(int k = 0; k < NV; k++)
-        sres[k] = v[k];
-      sres[2] = more ? 1.0 : 0.0;
-    }
-  }
-  __syncthreads();
-#pragma unroll
-  for(int k = 0; k < NV; k++)
-    v[k] = sres[k];
-  return sres[2] == 0.0;
-}
 
 /// q = (K p) at padded entry c0 of the box (2D): its four elements' products
 __device__ __forceinline__ void node_product2(const ElemK<2> &K, const double *p, const double *E,
@@ -363,7 +240,7 @@ __global__ void __launch_bounds__(kThreads<DIM>)
     // The next value this CTA puts (first exchange of it + 1) is read by all
     // before their own fence (second exchange of it + 1), and only after that
     // fence do they read the emptied z (end of it + 1) or slots (it + 2) again.
-    double *set = slots + (it % 3) * kSlot * G, *clear = slots + ((it + 2) % 3) * kSlot * G;
+    double *set = slots + (it % 3) * kExSlot * G, *clear = slots + ((it + 2) % 3) * kExSlot * G;
     double *zcur = it & 1 ? p0 : z, *zold = it & 1 ? z : p0;
     // q = K p and p.q on the box (constrained rows of q are 0)
     double v[1] = {0.0};
@@ -432,7 +309,7 @@ __global__ void __launch_bounds__(kThreads<DIM>)
         sr[c * cap + n] = ri;
         const double zi = sd[c * cap + n] * ri;
         slot_put(zcur + c * d.ld + g, zi);
-        slot_store(zold + c * d.ld + g, kEmpty);
+        slot_store(zold + c * d.ld + g, kExEmpty);
         w[0] += ri * ri;
         w[1] += ri * zi;
       }
@@ -483,16 +360,16 @@ __global__ void __launch_bounds__(kThreads<DIM>)
       bool more = true;
 #pragma unroll
       for(int c = 0; c < DIM; c++)
-        b[c] = kEmpty;
-      for(unsigned n = 0; n < kPolls && more; n++)
+        b[c] = kExEmpty;
+      for(unsigned n = 0; n < kExPolls && more; n++)
       {
         more = false;
 #pragma unroll
         for(int c = 0; c < DIM; c++)
-          if(b[c] == kEmpty)
+          if(b[c] == kExEmpty)
           {
             b[c] = slot_read(zcur + c * d.ld + e.y);
-            more |= b[c] == kEmpty;
+            more |= b[c] == kExEmpty;
           }
       }
       late |= more;
@@ -548,8 +425,8 @@ PcgTiles pcg_tiles(const Dims &d)
   // nodes a CTA takes at most: six (3D) or eight (2D) a thread; its shared memory
   // ends near there, and 3D is still 1.6 times the three kernels' speed
   const long long most = d.dim == 3 ? 6 * kNodeThreads<3> : 8 * kNodeThreads<2>;
-  if(G > 256 || d.nnode >= (1LL << 30))
-    return best; // the exchange polls 256 CTAs at most
+  if(G > kExCtas || d.nnode >= (1LL << 30))
+    return best;
   for(int px = 1; px <= std::min(G, d.sx); px++)
     for(int py = 1; px * py <= G && py <= d.sy; py++)
     {
@@ -594,7 +471,7 @@ static void run_tiles(const PcgTiles &t, const Dims &d, const ElemK<DIM> &K, con
   ICB_CUDA(cudaFuncSetAttribute(k_pcg_tiles<DIM>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 kTileSmem));
   double *slots = z + nsoa; // a multiple of 64 doubles past z: line-aligned
-  ICB_CUDA(cudaMemsetAsync(z, 0xff, sizeof(double) * (nsoa + pcg_tile_slots(t)), s)); // kEmpty
+  ICB_CUDA(cudaMemsetAsync(z, 0xff, sizeof(double) * (nsoa + pcg_tile_slots(t)), s)); // kExEmpty
   Dims dd = d;
   PcgTiles tt = t;
   ElemK<DIM> kk = K;

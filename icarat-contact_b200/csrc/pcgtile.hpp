@@ -1,7 +1,7 @@
 // pcgtile.hpp -- the Jacobi-PCG of a small problem as one cooperative kernel
 // (pcgtile.cu).
 #pragma once
-#include "icb_internal.hpp"
+#include "exchange.cuh"
 
 namespace icb
 {
@@ -15,9 +15,8 @@ struct PcgTiles
 };
 /// the cut for a grid, or ctas() == 0 when the problem is too large for it
 PcgTiles pcg_tiles(const Dims &d);
-/// doubles of the exchange buffer of a cut: three sets of a line a CTA
-constexpr int kPcgTileSlot = 16;
-inline int pcg_tile_slots(const PcgTiles &t) { return 3 * kPcgTileSlot * t.ctas(); }
+/// doubles of the exchange slots of a cut: three sets
+inline int pcg_tile_slots(const PcgTiles &t) { return 3 * kExSlot * t.ctas(); }
 /// Iterate from the state k_pcg_init left (r, p, KState) until the solve
 /// stops: x, r, and the final KState; p is overwritten.  z: scratch of the
 /// vectors' length plus pcg_tile_slots() doubles.
