@@ -246,17 +246,89 @@ template <typename T> struct EpiIn
   T b[3], dinv[3], d[3], us[3];
 };
 
+/// 16-byte vectors of T and a component's four x-y modes in them
+template <typename T> struct Vec16;
+template <> struct Vec16<float>
+{
+  using V = float4;
+  static constexpr int PER = 1; ///< vectors per four values
+  static __device__ __forceinline__ void get(const V *p, int, float (&m)[4])
+  {
+    const V a = *p;
+    m[0] = a.x, m[1] = a.y, m[2] = a.z, m[3] = a.w;
+  }
+  static __device__ __forceinline__ void put(V *p, int, const float (&m)[4])
+  {
+    *p = make_float4(m[0], m[1], m[2], m[3]);
+  }
+};
+template <> struct Vec16<double>
+{
+  using V = double2;
+  static constexpr int PER = 2;
+  static __device__ __forceinline__ void get(const V *p, int stride, double (&m)[4])
+  {
+    const V a = p[0], b = p[stride];
+    m[0] = a.x, m[1] = a.y, m[2] = b.x, m[3] = b.y;
+  }
+  static __device__ __forceinline__ void put(V *p, int stride, const double (&m)[4])
+  {
+    p[0] = make_double2(m[0], m[1]);
+    p[stride] = make_double2(m[2], m[3]);
+  }
+};
+
+/// three values of a thread in a 32-byte (FP64) or 16-byte slot
+__device__ __forceinline__ void row_put(float (&p)[4], const float (&v)[3])
+{
+  *reinterpret_cast<float4 *>(p) = make_float4(v[0], v[1], v[2], 0.f);
+}
+__device__ __forceinline__ void row_get(const float (&p)[4], float (&v)[3])
+{
+  const float4 a = *reinterpret_cast<const float4 *>(p);
+  v[0] = a.x, v[1] = a.y, v[2] = a.z;
+}
+__device__ __forceinline__ void row_put(double (&p)[4], const double (&v)[3])
+{
+  *reinterpret_cast<double2 *>(p) = make_double2(v[0], v[1]);
+  p[2] = v[2];
+}
+__device__ __forceinline__ void row_get(const double (&p)[4], double (&v)[3])
+{
+  const double2 a = *reinterpret_cast<const double2 *>(p);
+  v[0] = a.x, v[1] = a.y, v[2] = p[2];
+}
+
 /// dynamic shared memory of k_matvec_h8m: the carry, and for FP64 the
 /// bottom plane's modes (12 values per thread each)
 template <typename T, int TYK> constexpr int h8m_smem_bytes()
 {
   return int(sizeof(T)) * 12 * TYK * TX * (sizeof(T) == 8 ? 2 : 1);
 }
+/// whether a grid's vectors can be addressed by 32-bit byte offsets per component
+template <typename T> inline bool h8m_offsets_fit(const Dims &d)
+{
+  return (unsigned long long)d.nnode * sizeof(T) < (1ull << 32);
+}
+/// base[off bytes]: a base all threads share and a 32-bit offset (one register
+/// serves every component and vector at the same node)
+template <typename T> __device__ __forceinline__ const T *at_byte(const T *base, unsigned off)
+{
+  return reinterpret_cast<const T *>(reinterpret_cast<const char *>(base) + off);
+}
+template <typename T> __device__ __forceinline__ T *at_byte(T *base, unsigned off)
+{
+  return reinterpret_cast<T *>(reinterpret_cast<char *>(base) + off);
+}
 
 /// Each layer issues the loads of the next layer's top plane and modulus
 /// ahead of its own element work, so the arithmetic covers their latency.
 /// The carried top-face result lives in shared memory (each thread its own
-/// 12 values), which keeps the registers for the prefetched plane.
+/// 12 values, in 16-byte vectors), which keeps the registers for the prefetched
+/// plane.  The kernel is bound by issue slots, so what is not arithmetic is kept
+/// small: one 32-bit byte offset per node row serves all components (instead of
+/// twelve 64-bit addresses), and columns and planes outside the grid read the
+/// nearest inside with a zero modulus instead of selecting zeros.
 template <typename T, int TYK, bool DOT, int MODE, int MINB>
 __global__ void __launch_bounds__(TX *TYK, MINB)
     k_matvec_h8m(const KModal<T> K, const Dims d, const int zchunk,
@@ -269,55 +341,68 @@ __global__ void __launch_bounds__(TX *TYK, MINB)
   // FP64 also keeps the bottom plane's modes in shared memory (kSmemModes);
   // carry and modes take h8m_smem_bytes of dynamic shared memory
   constexpr bool kSmemModes = sizeof(T) == 8;
+  using V = typename Vec16<T>::V;
+  constexpr int PER = Vec16<T>::PER, NT = TX * TYK;
   extern __shared__ __align__(16) unsigned char h8m_dyn[];
-  auto sC = reinterpret_cast<T(*)[TYK][TX]>(h8m_dyn);
-  auto sH = reinterpret_cast<T(*)[TYK][TX]>(h8m_dyn + sizeof(T) * 12 * TYK * TX);
-  __shared__ T sB[2][3][TYK][TX];
   const int lx = threadIdx.x, ly = threadIdx.y;
+  // component c's modes: vectors (c PER + 0 .. PER - 1) NT + thread
+  V *sC = reinterpret_cast<V *>(h8m_dyn) + ly * TX + lx, *sH = sC + 3 * PER * NT;
+  // the row below's corner sums: three values a thread
+  __shared__ __align__(16) T sB[2][TYK][TX][4];
   const int X0 = blockIdx.x * (TX - 1), Y0 = blockIdx.y * (TYK - 1);
   const int ei = X0 - 1 + lx, ej = Y0 - 1 + ly;
   const int Z0 = blockIdx.z * zchunk;
   const int Z1 = min(Z0 + zchunk, d.sz) - 1;
   const bool col = ei >= 0 && ei < d.nx && ej >= 0 && ej < d.ny;
-  const long long sxy = (long long)d.sx * d.sy, exy = (long long)d.nx * d.ny;
+  const unsigned sxy = unsigned(d.sx) * unsigned(d.sy) * unsigned(sizeof(T));
+  const unsigned exy = unsigned(d.nx) * unsigned(d.ny) * unsigned(sizeof(T));
   const long long ld = d.ld;
-  // component c of this column's corner q in node plane k: u[c*ld + nb + qoff[q] + k*sxy]
-  const long long nb = col ? (long long)ei + (long long)ej * d.sx : 0;
-  const long long qoff[4] = {0, 1, 1 + (long long)d.sx, (long long)d.sx};
-  const long long eb = col ? (long long)ei + (long long)ej * d.nx : 0;
-  auto load_plane = [&](int k, T (&v)[3][4]) {
-    const bool ok = col && k >= 0 && k <= d.nz;
-    const T *p = u + nb + (long long)k * sxy;
+  // byte offsets of the column's low corners in the two node rows, of the next
+  // plane to load (planes outside the grid: the nearest)
+  const int cx = min(max(ei, 0), d.nx - 1), cy = min(max(ej, 0), d.ny - 1);
+  unsigned o0 = (unsigned(cx) + unsigned(cy) * unsigned(d.sx)) * unsigned(sizeof(T)) +
+                unsigned(max(Z0 - 1, 0)) * sxy;
+  const unsigned rowb = unsigned(d.sx) * unsigned(sizeof(T));
+  auto load_plane = [&](T(&v)[3][4]) {
+    const unsigned o1 = o0 + rowb;
 #pragma unroll
     for(int c = 0; c < 3; c++)
-#pragma unroll
-      for(int q = 0; q < 4; q++)
-        v[c][q] = ok ? __ldg(p + c * ld + qoff[q]) : T(0);
+    {
+      const T *p = u + c * ld;
+      v[c][0] = __ldg(at_byte(p, o0));
+      v[c][1] = __ldg(at_byte(p, o0) + 1);
+      v[c][2] = __ldg(at_byte(p, o1) + 1);
+      v[c][3] = __ldg(at_byte(p, o1));
+    }
   };
-  auto load_E = [&](int k) {
-    return col && k >= 0 && k < d.nz ? __ldg(E + eb + (long long)k * exy) : T(0);
-  };
+  unsigned eo = (unsigned(cx) + unsigned(cy) * unsigned(d.nx)) * unsigned(sizeof(T)) +
+                unsigned(max(Z0 - 1, 0)) * exy;
+  auto load_E = [&](int k) { return col && k >= 0 && k < d.nz ? __ldg(at_byte(E, eo)) : T(0); };
 
   // the bottom plane's x-y modes; the top-face result carried up (sC)
   T bh[3][4], nxt[3][4];
   {
     T v[3][4];
-    load_plane(Z0 - 1, v);
+    load_plane(v);
 #pragma unroll
     for(int c = 0; c < 3; c++)
     {
       plane_modes(v[c], bh[c]);
-#pragma unroll
-      for(int q = 0; q < 4; q++)
-      {
-        sC[c * 4 + q][ly][lx] = T(0);
-        if(kSmemModes)
-          sH[c * 4 + q][ly][lx] = bh[c][q];
-      }
+      const T zero[4] = {T(0), T(0), T(0), T(0)};
+      Vec16<T>::put(sC + c * PER * NT, NT, zero);
+      if(kSmemModes)
+        Vec16<T>::put(sH + c * PER * NT, NT, bh[c]);
     }
   }
-  load_plane(Z0, nxt);
+  if(Z0 > 0)
+    o0 += sxy;
+  load_plane(nxt);
   T Enxt = load_E(Z0 - 1);
+  // this thread's output node: byte offset in plane Z0 - 1, advanced a plane a layer
+  const int ni = ei + 1, nj = ej + 1;
+  const bool ownCol = lx < TX - 1 && ly < TYK - 1 && ni < d.sx && nj < d.sy;
+  unsigned node = (unsigned(ni) + unsigned(nj) * unsigned(d.sx)) * unsigned(sizeof(T)) +
+                  (unsigned(Z0) - 1u) * sxy; // wraps below plane 0, where it is not used
   double dot = 0.0;
   for(int ek = Z0 - 1; ek <= Z1; ++ek)
   {
@@ -329,32 +414,35 @@ __global__ void __launch_bounds__(TX *TYK, MINB)
     // next layer's inputs: FP32 at the top of the layer, FP64 after the
     // element product (its registers are the limit)
     constexpr bool kLateNext = sizeof(T) == 8;
-    if(!kLateNext)
-    {
-      load_plane(ek + 2, nxt);
+    auto load_next = [&]() {
+      if(ek + 2 <= d.nz)
+        o0 += sxy;
+      load_plane(nxt);
+      if(ek >= 0)
+        eo += exy;
       Enxt = load_E(ek + 1);
-    }
+    };
+    if(!kLateNext)
+      load_next();
     const bool out = ek >= Z0;
-    const int ni = ei + 1, nj = ej + 1;
-    const bool own = out && lx < TX - 1 && ly < TYK - 1 && ni < d.sx && nj < d.sy;
-    const long long node = (long long)ni + (long long)nj * d.sx + (long long)ek * sxy;
+    const bool own = out && ownCol;
     unsigned f = 0;
     EpiIn<T> in;
     auto load_in = [&]() {
       if(own)
       {
-        f = __ldg(fix + node);
+        f = __ldg(fix + node / unsigned(sizeof(T)));
 #pragma unroll
         for(int c = 0; c < 3; c++)
         {
           if(DOT || MODE >= OP_JACOBI)
-            in.us[c] = __ldg(u + c * ld + node);
+            in.us[c] = __ldg(at_byte(u + c * ld, node));
           if(MODE != OP_APPLY)
-            in.b[c] = __ldg(ep.b + c * ld + node);
+            in.b[c] = __ldg(at_byte(ep.b + c * ld, node));
           if(MODE >= OP_JACOBI)
-            in.dinv[c] = __ldg(ep.dinv + c * ld + node);
+            in.dinv[c] = __ldg(at_byte(ep.dinv + c * ld, node));
           if(MODE == OP_CHEB)
-            in.d[c] = ep.c1 != T(0) ? y[c * ld + node] : T(0); // the previous iterate
+            in.d[c] = ep.c1 != T(0) ? *at_byte(y + c * ld, node) : T(0); // the previous iterate
         }
       }
     };
@@ -367,35 +455,38 @@ __global__ void __launch_bounds__(TX *TYK, MINB)
     // element modes: z butterfly of the two planes' x-y modes
     T uh[24], yh[24];
 #pragma unroll
-    for(int s = 0; s < 4; s++)
-#pragma unroll
-      for(int c = 0; c < 3; c++)
+    for(int c = 0; c < 3; c++)
+    {
+      if(kSmemModes)
       {
-        const T b = kSmemModes ? sH[c * 4 + s][ly][lx] : bh[c][s];
-        uh[s * 3 + c] = b + th[c][s];
-        uh[(s + 4) * 3 + c] = b - th[c][s];
-        if(kSmemModes)
-          sH[c * 4 + s][ly][lx] = th[c][s];
+        Vec16<T>::get(sH + c * PER * NT, NT, bh[c]);
+        Vec16<T>::put(sH + c * PER * NT, NT, th[c]);
       }
+#pragma unroll
+      for(int s = 0; s < 4; s++)
+      {
+        uh[s * 3 + c] = bh[c][s] + th[c][s];
+        uh[(s + 4) * 3 + c] = bh[c][s] - th[c][s];
+      }
+    }
     yh[0] = yh[1] = yh[2] = T(0); // rigid translations
     modal_blocks_apply<0, 0>(K, uh, yh);
     if(kLateNext)
-    {
-      load_plane(ek + 2, nxt);
-      Enxt = load_E(ek + 1);
-    }
+      load_next();
     // inverse z butterfly: bottom face completes plane ek, top face is carried
     T acc[3][4];
 #pragma unroll
     for(int c = 0; c < 3; c++)
     {
-      T hb[4];
+      T hb[4], carry[4];
+      Vec16<T>::get(sC + c * PER * NT, NT, carry);
 #pragma unroll
       for(int s = 0; s < 4; s++)
       {
-        hb[s] = fma(Ee, yh[s * 3 + c] + yh[(s + 4) * 3 + c], sC[c * 4 + s][ly][lx]);
-        sC[c * 4 + s][ly][lx] = Ee * (yh[s * 3 + c] - yh[(s + 4) * 3 + c]);
+        hb[s] = fma(Ee, yh[s * 3 + c] + yh[(s + 4) * 3 + c], carry[s]);
+        carry[s] = Ee * (yh[s * 3 + c] - yh[(s + 4) * 3 + c]);
       }
+      Vec16<T>::put(sC + c * PER * NT, NT, carry);
       plane_corners(hb, acc[c]);
     }
     if(!kSmemModes)
@@ -408,28 +499,28 @@ __global__ void __launch_bounds__(TX *TYK, MINB)
       load_in();
     if(out)
     {
-      T A[3];
+      T A[3], S[3];
       const int buf = ek & 1;
 #pragma unroll
       for(int c = 0; c < 3; c++)
       {
         A[c] = acc[c][lnode(1, 1)] + __shfl_down_sync(0xffffffffu, acc[c][lnode(0, 1)], 1);
-        sB[buf][c][ly][lx] =
-            acc[c][lnode(1, 0)] + __shfl_down_sync(0xffffffffu, acc[c][lnode(0, 0)], 1);
+        S[c] = acc[c][lnode(1, 0)] + __shfl_down_sync(0xffffffffu, acc[c][lnode(0, 0)], 1);
       }
+      row_put(sB[buf][ly][lx], S);
       __syncthreads();
       if(own)
       {
+        row_get(sB[buf][ly + 1][lx], S);
 #pragma unroll
         for(int c = 0; c < 3; c++)
         {
-          T o = A[c] + sB[buf][c][ly + 1][lx];
+          T o = A[c] + S[c];
           if((f >> c) & 1u)
             o = T(0);
           const T us = in.us[c];
           if(DOT)
             dot += double(us) * double(o);
-          const long long i = c * ld + node;
           T w;
           if(MODE == OP_APPLY)
             w = o;
@@ -448,10 +539,11 @@ __global__ void __launch_bounds__(TX *TYK, MINB)
               w = us + dn;
             }
           }
-          y[i] = w;
+          *at_byte(y + c * ld, node) = w;
         }
       }
     }
+    node += sxy;
   }
   if(DOT)
   {
@@ -1484,7 +1576,7 @@ static void launch_op_mode(const Dims &d, const T *K, const T *E, const T *u, T 
         return;
       }
     }
-    if(g_hex8_modal && modal_form_cached(K, kmod))
+    if(g_hex8_modal && h8m_offsets_fit<T>(d) && modal_form_cached(K, kmod))
     {
       // 3 (FP32) CTAs of 256 threads per SM; FP64 2 with the fused dot and 1
       // without (no register cap short of the kernel's own: the FP64 V-cycle
