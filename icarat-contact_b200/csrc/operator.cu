@@ -299,11 +299,11 @@ __device__ __forceinline__ void row_get(const double (&p)[4], double (&v)[3])
   v[0] = a.x, v[1] = a.y, v[2] = p[2];
 }
 
-/// dynamic shared memory of k_matvec_h8m: the carry, and for FP64 the
-/// bottom plane's modes (12 values per thread each)
-template <typename T, int TYK> constexpr int h8m_smem_bytes()
+/// dynamic shared memory of k_matvec_h8m: the carry, and for FP64 with two CTAs
+/// an SM the bottom plane's modes (12 values per thread each)
+template <typename T, int TYK, int MINB> constexpr int h8m_smem_bytes()
 {
-  return int(sizeof(T)) * 12 * TYK * TX * (sizeof(T) == 8 ? 2 : 1);
+  return int(sizeof(T)) * 12 * TYK * TX * (sizeof(T) == 8 && MINB > 1 ? 2 : 1);
 }
 /// whether a grid's vectors can be addressed by 32-bit byte offsets per component
 template <typename T> inline bool h8m_offsets_fit(const Dims &d)
@@ -338,9 +338,10 @@ __global__ void __launch_bounds__(TX *TYK, MINB)
 {
   if(gate && (gate->stop || (gateConv && gate->conv)))
     return;
-  // FP64 also keeps the bottom plane's modes in shared memory (kSmemModes);
-  // carry and modes take h8m_smem_bytes of dynamic shared memory
-  constexpr bool kSmemModes = sizeof(T) == 8;
+  // FP64 with two CTAs an SM (the fused dot): the registers end at 128, so the
+  // bottom plane's modes live in shared memory too and the loads wait until the
+  // element product's registers are free
+  constexpr bool kTight = sizeof(T) == 8 && MINB > 1;
   using V = typename Vec16<T>::V;
   constexpr int PER = Vec16<T>::PER, NT = TX * TYK;
   extern __shared__ __align__(16) unsigned char h8m_dyn[];
@@ -390,7 +391,7 @@ __global__ void __launch_bounds__(TX *TYK, MINB)
       plane_modes(v[c], bh[c]);
       const T zero[4] = {T(0), T(0), T(0), T(0)};
       Vec16<T>::put(sC + c * PER * NT, NT, zero);
-      if(kSmemModes)
+      if(kTight)
         Vec16<T>::put(sH + c * PER * NT, NT, bh[c]);
     }
   }
@@ -411,9 +412,7 @@ __global__ void __launch_bounds__(TX *TYK, MINB)
     for(int c = 0; c < 3; c++)
       plane_modes(nxt[c], th[c]);
     const T Ee = Enxt;
-    // next layer's inputs: FP32 at the top of the layer, FP64 after the
-    // element product (its registers are the limit)
-    constexpr bool kLateNext = sizeof(T) == 8;
+    // next layer's inputs
     auto load_next = [&]() {
       if(ek + 2 <= d.nz)
         o0 += sxy;
@@ -422,7 +421,7 @@ __global__ void __launch_bounds__(TX *TYK, MINB)
         eo += exy;
       Enxt = load_E(ek + 1);
     };
-    if(!kLateNext)
+    if(!kTight)
       load_next();
     const bool out = ek >= Z0;
     const bool own = out && ownCol;
@@ -446,18 +445,14 @@ __global__ void __launch_bounds__(TX *TYK, MINB)
         }
       }
     };
-    // FP32: before the element work; FP64: after it, where the registers
-    // of the element work are free again (the exchange barrier covers part
-    // of the latency)
-    constexpr bool kEarly = sizeof(T) == 4;
-    if(kEarly)
+    if(!kTight)
       load_in();
     // element modes: z butterfly of the two planes' x-y modes
     T uh[24], yh[24];
 #pragma unroll
     for(int c = 0; c < 3; c++)
     {
-      if(kSmemModes)
+      if(kTight)
       {
         Vec16<T>::get(sH + c * PER * NT, NT, bh[c]);
         Vec16<T>::put(sH + c * PER * NT, NT, th[c]);
@@ -471,7 +466,7 @@ __global__ void __launch_bounds__(TX *TYK, MINB)
     }
     yh[0] = yh[1] = yh[2] = T(0); // rigid translations
     modal_blocks_apply<0, 0>(K, uh, yh);
-    if(kLateNext)
+    if(kTight)
       load_next();
     // inverse z butterfly: bottom face completes plane ek, top face is carried
     T acc[3][4];
@@ -489,13 +484,13 @@ __global__ void __launch_bounds__(TX *TYK, MINB)
       Vec16<T>::put(sC + c * PER * NT, NT, carry);
       plane_corners(hb, acc[c]);
     }
-    if(!kSmemModes)
+    if(!kTight)
 #pragma unroll
       for(int c = 0; c < 3; c++)
 #pragma unroll
         for(int q = 0; q < 4; q++)
           bh[c][q] = th[c][q];
-    if(!kEarly)
+    if(kTight)
       load_in();
     if(out)
     {
@@ -1430,10 +1425,10 @@ int matvec_blocks(const Dims &d)
   if(d.dim == 3)
   {
     // the largest CTA count h8_zchunk picks for any occupancy of 1..8 CTAs/SM,
-    // for the one-row tiles (31 x 7 nodes) and the paired ones (31 x 15)
+    // for the one-row tiles (31 x 7 nodes, FP64 31 x 11) and the paired ones (31 x 15)
     const long long bx = (d.sx + TX - 2) / (TX - 1);
     long long most = 0;
-    for(int rows : {TY3 - 1, 2 * kPairWarps - 1})
+    for(int rows : {TY3 - 1, TY3 + 3, 2 * kPairWarps - 1})
     {
       const long long tiles = bx * ((d.sy + rows - 1) / rows);
       for(int k = 1; k <= 8; k++)
@@ -1540,18 +1535,25 @@ static void launch_op_mode(const Dims &d, const T *K, const T *E, const T *u, T 
   Epi<T> ep{x.b, x.dinv, T(x.omega), T(x.c1), T(x.c2)};
   if(d.dim == 3)
   {
-    // 8 element rows per tile for FP64 and FP32 (16-row FP64 tiles were
-    // measured: faster at 384x128x128, slower at 192x64x64)
-    constexpr int TYK = TY3;
-    const int bx = (d.sx + TX - 2) / (TX - 1), by = (d.sy + TYK - 2) / (TYK - 1);
-    auto run = [&](auto kern, const auto &kp, int smem) {
+    // element rows per tile: 8; 12 for the FP64 product and residual without a
+    // dot, whose registers (168) still fit 384 threads without spills: 12 warps
+    // an SM and a smaller halo (y = K u at 384x128x128 183 us, with 8 rows 198,
+    // with 8 rows and the fused dot's form 211; the Chebyshev step spills at 12
+    // rows, 288 against 285 us).  12 rows for FP32 measured 89.6 against 88.2 us.
+    // The dot keeps 8 rows: its sum is cut by tiles, and a mixed solve follows
+    // every bit of it
+    constexpr int TYK0 = TY3;
+    constexpr int TYK1 = sizeof(T) == 8 && MODE <= OP_RESIDUAL ? TY3 + 4 : TY3;
+    const int bx = (d.sx + TX - 2) / (TX - 1);
+    auto run = [&](auto kern, const auto &kp, int smem, int rows) {
+      const int by = (d.sy + rows - 2) / (rows - 1);
       const int zchunk =
-          h8_zchunk(d, (long long)bx * by, resident_ctas((const void *)kern, TX * TYK, smem));
+          h8_zchunk(d, (long long)bx * by, resident_ctas((const void *)kern, TX * rows, smem));
       const int bz = (d.sz + zchunk - 1) / zchunk;
       if(x.dotRed)
         ICB_REQUIRE((long long)bx * by * bz <= red.maxBlocks, "reduction scratch too small");
-      kern<<<dim3(bx, by, bz), dim3(TX, TYK), smem, s>>>(kp, d, zchunk, E, u, y, fix, red,
-                                                         x.dotOut, x.gate, x.gateConv, ep);
+      kern<<<dim3(bx, by, bz), dim3(TX, rows), smem, s>>>(kp, d, zchunk, E, u, y, fix, red,
+                                                          x.dotOut, x.gate, x.gateConv, ep);
     };
     KModal<T> kmod;
     if constexpr(std::is_same<T, float>::value)
@@ -1578,18 +1580,15 @@ static void launch_op_mode(const Dims &d, const T *K, const T *E, const T *u, T 
     }
     if(g_hex8_modal && h8m_offsets_fit<T>(d) && modal_form_cached(K, kmod))
     {
-      // 3 (FP32) CTAs of 256 threads per SM; FP64 2 with the fused dot and 1
-      // without (no register cap short of the kernel's own: the FP64 V-cycle
-      // took 58.3 against 59.4 ms at 384x128x128, the dot-fused form was
-      // unchanged).  The carry (and for FP64 the bottom plane's modes) live
-      // in shared memory: FP64 with both in registers spills, and the
-      // dot-fused FP64 Jacobi-PCG on halfmbb3d 192x64x64 took 208 ms against
-      // 172 ms for 2374 iterations
+      // 3 (FP32) CTAs of 256 threads per SM; FP64 two with the fused dot and one
+      // without, whose registers let the next plane's loads go out a whole layer
+      // ahead and keep the bottom plane's modes (only the carry in shared memory)
       constexpr int MB = sizeof(T) == 8 ? 2 : 3, MBnodot = sizeof(T) == 8 ? 1 : 3;
       if(x.dotRed)
-        run(k_matvec_h8m<T, TYK, true, MODE, MB>, kmod, h8m_smem_bytes<T, TYK>());
+        run(k_matvec_h8m<T, TYK0, true, MODE, MB>, kmod, h8m_smem_bytes<T, TYK0, MB>(), TYK0);
       else
-        run(k_matvec_h8m<T, TYK, false, MODE, MBnodot>, kmod, h8m_smem_bytes<T, TYK>());
+        run(k_matvec_h8m<T, TYK1, false, MODE, MBnodot>, kmod,
+            h8m_smem_bytes<T, TYK1, MBnodot>(), TYK1);
     }
     else if constexpr(std::is_same<T, double>::value)
     {
@@ -1598,18 +1597,18 @@ static void launch_op_mode(const Dims &d, const T *K, const T *E, const T *u, T 
         for(int c = r; c < 24; c++)
           ks.k[symIdx(r, c)] = K[r * 24 + c];
       if(x.dotRed)
-        run(k_matvec_h8<T, KSym24, TYK, true, MODE>, ks, 0);
+        run(k_matvec_h8<T, KSym24, TYK0, true, MODE>, ks, 0, TYK0);
       else
-        run(k_matvec_h8<T, KSym24, TYK, false, MODE>, ks, 0);
+        run(k_matvec_h8<T, KSym24, TYK0, false, MODE>, ks, 0, TYK0);
     }
     else
     {
       KMat<T, 24> km;
       std::copy(K, K + 576, km.k);
       if(x.dotRed)
-        run(k_matvec_h8<T, KMat<T, 24>, TYK, true, MODE>, km, 0);
+        run(k_matvec_h8<T, KMat<T, 24>, TYK0, true, MODE>, km, 0, TYK0);
       else
-        run(k_matvec_h8<T, KMat<T, 24>, TYK, false, MODE>, km, 0);
+        run(k_matvec_h8<T, KMat<T, 24>, TYK0, false, MODE>, km, 0, TYK0);
     }
   }
   else
