@@ -179,6 +179,7 @@ template <typename T> struct Epi
   const T *dinv;
   T omega;
   T c1, c2;
+  int prev0; ///< OP_CHEB: the iterate before is 0 (y is not read)
 };
 template <typename T> struct OpExtras
 {
@@ -187,6 +188,7 @@ template <typename T> struct OpExtras
   const T *dinv = nullptr;
   double omega = 0.0;
   double c1 = 0.0, c2 = 0.0;
+  int prev0 = 0;
   RedScratch *dotRed = nullptr; ///< fused u.y reduction (OP_APPLY) into *dotOut
   double *dotOut = nullptr;
   const KState *gate = nullptr; ///< skip when gate->stop (or gate->conv if gateConv)

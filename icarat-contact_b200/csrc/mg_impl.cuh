@@ -79,6 +79,24 @@ __global__ void k_coarsen_E(Dims df, Dims dc, int3 sh, const T *__restrict__ Ef,
   coarsen_E_b<T>(df, dc, sh, Ef, Ec, this_block());
 }
 
+/// A level's first smoothing step from a zero guess, x = c D^-1 b, taken by the
+/// kernel that writes b (x NULL: none).  As a kernel of its own it read D^-1 and b
+/// again and cleared the iterate before, 38 us of an iteration at 384x128x128, and one
+/// launch of eight on every level.
+template <typename T> struct FirstStep
+{
+  T c;
+  const T *dinv;
+  T *x;
+  /// D^-1 at entry i, loaded ahead of the b it scales
+  __device__ __forceinline__ T load(long long i) const { return x ? __ldg(dinv + i) : T(0); }
+  __device__ __forceinline__ void store(long long i, T d, T b) const
+  {
+    if(x)
+      x[i] = c * d * b;
+  }
+};
+
 /// b_c = R r_f (R = P^T), constrained coarse DOFs zeroed.  One thread per
 /// coarse node (x along threads, y and z along the grid, so no index
 /// division): along a halved axis the 1-D weights of the fine neighbours
@@ -87,7 +105,7 @@ __global__ void k_coarsen_E(Dims df, Dims dc, int3 sh, const T *__restrict__ Ef,
 template <typename T>
 __device__ __forceinline__ void restrict_b(Dims df, Dims dc, int3 sh, const T *__restrict__ rf,
                            T *__restrict__ bc, const uint8_t *__restrict__ fixc,
-                           const KState *gate, const Blk &B)
+                           const KState *gate, const FirstStep<T> &first, const Blk &B)
 {
   if(gated(gate))
     return;
@@ -97,7 +115,12 @@ __device__ __forceinline__ void restrict_b(Dims df, Dims dc, int3 sh, const T *_
   const long long fsxy = (long long)df.sx * df.sy;
   const int kr = df.dim == 3 ? sh.z : 0;
   const T h = T(0.5);
-  T s[3] = {T(0), T(0), T(0)};
+  T s[3] = {T(0), T(0), T(0)}, dv[3];
+  const long long n = I + (long long)J * dc.sx + (long long)K * dc.sx * dc.sy;
+  const unsigned fx = fixc[n];
+#pragma unroll
+  for(int c = 0; c < 3; c++)
+    dv[c] = c < dc.dim ? first.load(c * dc.ld + n) : T(0);
   for(int dk = -kr; dk <= kr; dk++)
   {
     const int k = (K << sh.z) + dk;
@@ -125,19 +148,21 @@ __device__ __forceinline__ void restrict_b(Dims df, Dims dc, int3 sh, const T *_
     for(int c = 0; c < 3; c++)
       s[c] = dk ? fma(h, sk[c], s[c]) : s[c] + sk[c];
   }
-  const long long n = I + (long long)J * dc.sx + (long long)K * dc.sx * dc.sy;
-  const unsigned fx = fixc[n];
 #pragma unroll
   for(int c = 0; c < 3; c++)
     if(c < dc.dim)
-      bc[c * dc.ld + n] = ((fx >> c) & 1u) ? T(0) : s[c];
+    {
+      const T v = ((fx >> c) & 1u) ? T(0) : s[c];
+      bc[c * dc.ld + n] = v;
+      first.store(c * dc.ld + n, dv[c], v);
+    }
 }
 template <typename T>
 __global__ void k_restrict(Dims df, Dims dc, int3 sh, const T *__restrict__ rf,
                            T *__restrict__ bc, const uint8_t *__restrict__ fixc,
-                           const KState *gate)
+                           const KState *gate, const FirstStep<T> first)
 {
-  restrict_b<T>(df, dc, sh, rf, bc, fixc, gate, this_block());
+  restrict_b<T>(df, dc, sh, rf, bc, fixc, gate, first, this_block());
 }
 
 /// x_f += P x_c, constrained fine DOFs untouched (they stay 0).  One thread
@@ -207,45 +232,6 @@ __global__ void k_prolong_add(Dims df, Dims dc, int3 sh, const T *__restrict__ x
     return;
   prolong_rows_b<T>(df, dc, sh, xc, xf, fixf, blockIdx.x * blockDim.x + threadIdx.x,
                     blockIdx.y * kProlongRows, blockIdx.z);
-}
-
-/// first smoothing step from a zero guess: x = c D^-1 b, x0 = 0
-template <typename T>
-__device__ __forceinline__ void jacobi0_b(long long n, T c, const T *__restrict__ dinv,
-                          const T *__restrict__ b, T *__restrict__ x, T *__restrict__ x0,
-                          const KState *gate, const Blk &B)
-{
-  if(gated(gate))
-    return;
-  const long long st = (long long)B.gx * blockDim.x;
-  for(long long i0 = B.x * (long long)blockDim.x + threadIdx.x; i0 < n; i0 += kGroup * st)
-  {
-    T dv[kGroup], bv[kGroup];
-#pragma unroll
-    for(int g = 0; g < kGroup; g++)
-    {
-      const long long i = i0 + g * st;
-      dv[g] = i < n ? dinv[i] : T(0);
-      bv[g] = i < n ? b[i] : T(0);
-    }
-#pragma unroll
-    for(int g = 0; g < kGroup; g++)
-    {
-      const long long i = i0 + g * st;
-      if(i < n)
-      {
-        x[i] = c * dv[g] * bv[g];
-        x0[i] = T(0); // the iterate before x, for the next three-term step
-      }
-    }
-  }
-}
-template <typename T>
-__global__ void k_jacobi0(long long n, T c, const T *__restrict__ dinv,
-                          const T *__restrict__ b, T *__restrict__ x, T *__restrict__ x0,
-                          const KState *gate)
-{
-  jacobi0_b<T>(n, c, dinv, b, x, x0, gate, this_block());
 }
 
 // --------------------------------------------------------- coarse level ----
@@ -568,16 +554,20 @@ struct FinInitMg
 template <typename TK, typename TP>
 __device__ __forceinline__ void mg_init_b(long long n, const TK *__restrict__ b, TK *__restrict__ x,
                           TK *__restrict__ r, TP *__restrict__ rP, RedScratch red, KState *st,
-                          double tol, int maxit, const Blk &B)
+                          double tol, int maxit, const FirstStep<TP> &first, const Blk &B)
 {
   double v[1] = {0.0};
   const long long sd = (long long)B.gx * blockDim.x;
   for(long long i0 = B.x * (long long)blockDim.x + threadIdx.x; i0 < n; i0 += kGroup * sd)
   {
     TK bv[kGroup];
+    TP dv[kGroup];
 #pragma unroll
     for(int g = 0; g < kGroup; g++)
+    {
       bv[g] = i0 + g * sd < n ? b[i0 + g * sd] : TK(0);
+      dv[g] = i0 + g * sd < n ? first.load(i0 + g * sd) : TP(0);
+    }
 #pragma unroll
     for(int g = 0; g < kGroup; g++)
     {
@@ -588,6 +578,7 @@ __device__ __forceinline__ void mg_init_b(long long n, const TK *__restrict__ b,
         r[i] = bi;
         if(rP)
           rP[i] = TP(bi);
+        first.store(i, dv[g], TP(bi));
         x[i] = TK(0);
         v[0] += double(bi) * double(bi);
       }
@@ -598,9 +589,9 @@ __device__ __forceinline__ void mg_init_b(long long n, const TK *__restrict__ b,
 template <typename TK, typename TP>
 __global__ void k_mg_init(long long n, const TK *__restrict__ b, TK *__restrict__ x,
                           TK *__restrict__ r, TP *__restrict__ rP, RedScratch red, KState *st,
-                          double tol, int maxit)
+                          double tol, int maxit, const FirstStep<TP> first)
 {
-  mg_init_b<TK, TP>(n, b, x, r, rP, red, st, tol, maxit, this_block());
+  mg_init_b<TK, TP>(n, b, x, r, rP, red, st, tol, maxit, first, this_block());
 }
 
 struct FinRz0
@@ -691,7 +682,8 @@ struct FinRmg
 template <typename TK, typename TP>
 __device__ __forceinline__ void mg_r_b(long long n, TK *__restrict__ r, TP *__restrict__ rP,
                        const TK *__restrict__ q, const TP *__restrict__ zold,
-                       const double *__restrict__ pq, RedScratch red, KState *st, const Blk &B)
+                       const double *__restrict__ pq, RedScratch red, KState *st,
+                       const FirstStep<TP> &first, const Blk &B)
 {
   if(st->stop)
     return;
@@ -706,7 +698,7 @@ __device__ __forceinline__ void mg_r_b(long long n, TK *__restrict__ r, TP *__re
     for(long long i0 = B.x * (long long)blockDim.x + threadIdx.x; i0 < n; i0 += kGroup * sd)
     {
       TK rv[kGroup], qv[kGroup];
-      TP zv[kGroup];
+      TP zv[kGroup], dv[kGroup];
 #pragma unroll
       for(int g = 0; g < kGroup; g++)
       {
@@ -714,6 +706,7 @@ __device__ __forceinline__ void mg_r_b(long long n, TK *__restrict__ r, TP *__re
         rv[g] = i < n ? r[i] : TK(0);
         qv[g] = i < n ? q[i] : TK(0);
         zv[g] = i < n ? zold[i] : TP(0);
+        dv[g] = i < n ? first.load(i) : TP(0);
       }
 #pragma unroll
       for(int g = 0; g < kGroup; g++)
@@ -725,6 +718,7 @@ __device__ __forceinline__ void mg_r_b(long long n, TK *__restrict__ r, TP *__re
           r[i] = ri;
           if(rP)
             rP[i] = TP(ri);
+          first.store(i, dv[g], TP(ri));
           v[0] += double(ri) * double(ri);
           v[1] += double(ri) * double(zv[g]);
         }
@@ -736,9 +730,10 @@ __device__ __forceinline__ void mg_r_b(long long n, TK *__restrict__ r, TP *__re
 template <typename TK, typename TP>
 __global__ void k_mg_r(long long n, TK *__restrict__ r, TP *__restrict__ rP,
                        const TK *__restrict__ q, const TP *__restrict__ zold,
-                       const double *__restrict__ pq, RedScratch red, KState *st)
+                       const double *__restrict__ pq, RedScratch red, KState *st,
+                       const FirstStep<TP> first)
 {
-  mg_r_b<TK, TP>(n, r, rP, q, zold, pq, red, st, this_block());
+  mg_r_b<TK, TP>(n, r, rP, q, zold, pq, red, st, first, this_block());
 }
 
 struct FinRz
@@ -1267,7 +1262,15 @@ template <typename TK, typename TP> struct MgPcg
     }
   }
 
-  /// out = V-cycle(b) on level l
+  /// level l's first smoothing step, when it runs as launches of its own
+  FirstStep<TP> firstStep(size_t l)
+  {
+    if(l + 1 >= lv.size() || (int(l) == tail0 && useTail()))
+      return FirstStep<TP>{TP(0), nullptr, nullptr};
+    return FirstStep<TP>{TP(cc2[0]), lv[l].dinv.p, lv[l].t.p};
+  }
+
+  /// out = V-cycle(b) on level l; firstStep(l) is done
   void level(size_t l, const TP *b, TP *out, cudaStream_t s, const KState *gate)
   {
     Level<TP> &L = lv[l];
@@ -1282,11 +1285,9 @@ template <typename TK, typename TP> struct MgPcg
       return;
     }
     long long m = (long long)L.d.dim * L.d.ld;
-    // step 0 from zero, then 2nu-1 operator steps: an odd number of
-    // ping-pongs ends in out
+    // step 0 from zero (taken where b was written, firstStep(l)), then 2nu-1
+    // operator steps: an odd number of ping-pongs ends in out
     TP *cur = L.t.p, *oth = out;
-    k_jacobi0<TP><<<vblocks(m), VB, 0, s>>>(m, TP(cc2[0]), L.dinv.p, b, cur, oth, gate);
-    count_launch();
     OpExtras<TP> ch;
     ch.mode = OP_CHEB;
     ch.b = b;
@@ -1297,9 +1298,11 @@ template <typename TK, typename TP> struct MgPcg
     {
       ch.c1 = cc1[k];
       ch.c2 = cc2[k];
+      ch.prev0 = k == 1;
       launch_op<TP>(L.d, L.K, L.E, cur, oth, L.fix, s, ch);
       std::swap(cur, oth);
     }
+    ch.prev0 = 0;
     OpExtras<TP> res;
     res.mode = OP_RESIDUAL;
     res.b = b;
@@ -1307,7 +1310,8 @@ template <typename TK, typename TP> struct MgPcg
     res.gateConv = 1;
     launch_op<TP>(L.d, L.K, L.E, cur, L.r.p, L.fix, s, res);
     Level<TP> &Cn = lv[l + 1];
-    k_restrict<TP><<<grid3(Cn.d), kTB, 0, s>>>(L.d, Cn.d, Cn.sh, L.r.p, Cn.b.p, Cn.fix, gate);
+    k_restrict<TP><<<grid3(Cn.d), kTB, 0, s>>>(L.d, Cn.d, Cn.sh, L.r.p, Cn.b.p, Cn.fix, gate,
+                                                  firstStep(l + 1));
     count_launch();
     level(l + 1, Cn.b.p, Cn.x.p, s, gate);
     dim3 gp = grid3(L.d);
@@ -1334,7 +1338,8 @@ template <typename TK, typename TP> struct MgPcg
     a.dotOut = dots.p;
     a.gate = st.p;
     launch_op<TK>(d, Kk, Ek, p.p, q.p, lv[0].fix, s, a);
-    k_mg_r<TK, TP><<<nb, VB, 0, s>>>(n, r.p, same() ? nullptr : rP.p, q.p, z.p, dots.p, red, st.p);
+    k_mg_r<TK, TP><<<nb, VB, 0, s>>>(n, r.p, same() ? nullptr : rP.p, q.p, z.p, dots.p, red, st.p,
+                                      firstStep(0));
     level(0, rin(), z.p, s, st.p);
     k_mg_rz<TK, TP><<<nb, VB, 0, s>>>(n, r.p, z.p, red, st.p);
     k_mg_xp<TK, TP><<<nb, VB, 0, s>>>(n, x, p.p, z.p, red, st.p, L);
@@ -1345,7 +1350,7 @@ template <typename TK, typename TP> struct MgPcg
   {
     int nb = vblocks(n);
     k_mg_init<TK, TP><<<nb, VB, 0, s>>>(n, b, x, r.p, same() ? nullptr : rP.p, red, st.p, tol,
-                                         maxit);
+                                         maxit, firstStep(0));
     count_launch();
     level(0, rin(), z.p, s, nullptr);
     k_mg_init2<TK, TP><<<nb, VB, 0, s>>>(n, r.p, z.p, p.p, red, st.p);

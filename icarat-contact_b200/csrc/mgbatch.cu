@@ -62,8 +62,12 @@ template <typename TK, typename TP> struct InitL
   KState *st;
   double tol;
   int maxit;
+  FirstStep<TP> first;
   __device__ bool skip() const { return false; }
-  __device__ void run(const Blk &B) const { mg_init_b<TK, TP>(n, b, x, r, rP, red, st, tol, maxit, B); }
+  __device__ void run(const Blk &B) const
+  {
+    mg_init_b<TK, TP>(n, b, x, r, rP, red, st, tol, maxit, first, B);
+  }
 };
 template <typename TK, typename TP> struct Init2L
 {
@@ -88,8 +92,9 @@ template <typename TK, typename TP> struct RL
   const double *pq;
   RedScratch red;
   KState *st;
+  FirstStep<TP> first;
   __device__ bool skip() const { return st->stop != 0; }
-  __device__ void run(const Blk &B) const { mg_r_b<TK, TP>(n, r, rP, q, z, pq, red, st, B); }
+  __device__ void run(const Blk &B) const { mg_r_b<TK, TP>(n, r, rP, q, z, pq, red, st, first, B); }
 };
 template <typename TK, typename TP> struct RzL
 {
@@ -113,17 +118,6 @@ template <typename TK, typename TP> struct XpL
   __device__ bool skip() const { return st->stop != 0; }
   __device__ void run(const Blk &B) const { mg_xp_b<TK, TP>(n, x, p, z, red, st, LoopCtl{}, B); }
 };
-template <typename T> struct Jacobi0L
-{
-  Blk g;
-  long long n;
-  T c;
-  const T *dinv, *b;
-  T *x, *x0;
-  const KState *gate;
-  __device__ bool skip() const { return gated(gate); }
-  __device__ void run(const Blk &B) const { jacobi0_b<T>(n, c, dinv, b, x, x0, gate, B); }
-};
 /// the transfers write each node from its own reads only, so a batched
 /// launch may give a block several node rows: g.gy blocks take the ry rows
 /// of the per-problem grid (same results, far fewer tiny blocks)
@@ -137,13 +131,14 @@ template <typename T> struct RestrictL
   const uint8_t *fixc;
   const KState *gate;
   unsigned ry;
+  FirstStep<T> first;
   __device__ bool skip() const { return gated(gate); }
   __device__ void run(const Blk &B) const
   {
     Blk b = B;
 #pragma unroll 2
     for(b.y = B.y; b.y < ry; b.y += B.gy)
-      restrict_b<T>(df, dc, sh, rf, bc, fixc, gate, b);
+      restrict_b<T>(df, dc, sh, rf, bc, fixc, gate, first, b);
   }
 };
 /// g.gy blocks along y, each ry node rows from its first, kProlongRows at a
@@ -343,7 +338,7 @@ template <typename T> struct Q4Builder
     q.dotOut = x.dotOut;
     q.gate = x.gate;
     q.gateConv = x.gateConv;
-    q.ep = Epi<T>{x.b, x.dinv, T(x.omega), T(x.c1), T(x.c2)};
+    q.ep = Epi<T>{x.b, x.dinv, T(x.omega), T(x.c1), T(x.c2), x.prev0};
     if(x.dotRed)
       ICB_REQUIRE(q4_dot_slots(d) <= x.dotRed->maxBlocks, "reduction scratch too small");
     mode = x.mode;
@@ -520,21 +515,9 @@ template <typename TP> struct BatchMg
     const int nu = M[fine[0].i]->nu;
     for(const Inst &I : fine)
       ICB_REQUIRE(M[I.i]->nu == nu, "batched problems need the same smoothing degree");
-    {
-      Builder<Jacobi0L<TP>> j0;
-      for(size_t k = 0; k < fine.size(); k++)
-      {
-        const Inst &I = fine[k];
-        MG &m = *M[I.i];
-        Level<TP> &L = m.lv[I.l];
-        const long long n = (long long)L.d.dim * L.d.ld;
-        cs[k] = Cur{L.t.p, I.out};
-        j0.add(Jacobi0L<TP>{{}, n, TP(m.cc2[0]), L.dinv.p, I.b, cs[k].cur, cs[k].oth, gate(I.i)},
-               unsigned(vblocks(n)));
-      }
-      push(j0.finish(VB, 0, s, qc.p));
-    }
-    auto cheb = [&](int k) {
+    for(size_t k = 0; k < fine.size(); k++)
+      cs[k] = Cur{M[fine[k].i]->lv[fine[k].l].t.p, fine[k].out};
+    auto cheb = [&](int k, bool pre) {
       Q4Builder<TP> op;
       for(size_t t = 0; t < fine.size(); t++)
       {
@@ -549,13 +532,14 @@ template <typename TP> struct BatchMg
         ch.gateConv = 1;
         ch.c1 = m.cc1[k];
         ch.c2 = m.cc2[k];
+        ch.prev0 = pre && k == 1;
         op.add(L.d, L.K, L.E, cs[t].cur, cs[t].oth, L.fix, ch);
         std::swap(cs[t].cur, cs[t].oth);
       }
       push(op.finish(s, qc.p));
     };
     for(int k = 1; k < nu; k++)
-      cheb(k);
+      cheb(k, true);
     {
       Q4Builder<TP> op;
       Builder<RestrictL<TP>> rs;
@@ -580,7 +564,9 @@ template <typename TP> struct BatchMg
         res.gateConv = 1;
         op.add(L.d, L.K, L.E, cs[t].cur, L.r.p, L.fix, res);
         const dim3 g3 = grid3(Cn.d);
-        rs.add(RestrictL<TP>{{}, L.d, Cn.d, Cn.sh, L.r.p, Cn.b.p, Cn.fix, gate(I.i), g3.y}, g3.x,
+        rs.add(RestrictL<TP>{{}, L.d, Cn.d, Cn.sh, L.r.p, Cn.b.p, Cn.fix, gate(I.i), g3.y,
+                            m.firstStep(I.l + 1)},
+               g3.x,
                transfer_rows(g3.y, kR), g3.z);
         next.push_back(Inst{I.i, Cn.b.p, Cn.x.p, I.l + 1});
       }
@@ -614,7 +600,7 @@ template <typename TP> struct BatchMg
       push(pr.finish(kTB, 0, s, qc.p));
     }
     for(int k = 0; k < nu; k++)
-      cheb(k);
+      cheb(k, false);
     Builder<CopyL<TP>> cp;
     for(size_t t = 0; t < fine.size(); t++)
       if(cs[t].cur != fine[t].out)
@@ -739,7 +725,7 @@ template <typename TP> struct BatchMg
       {
         MG &m = *M[i];
         in.add(InitL<double, TP>{{}, m.n, b[i], x[i], m.r.p, MG::same() ? nullptr : m.rP.p, m.red,
-                                 m.st.p, tol[i], maxit[i]},
+                                 m.st.p, tol[i], maxit[i], m.firstStep(0)},
                unsigned(vblocks(m.n)));
         all.push_back(Inst{i, m.rin(), m.z.p, 0});
       }
@@ -772,7 +758,7 @@ template <typename TP> struct BatchMg
         a.gate = m.st.p;
         op.add(m.lv[0].d, m.Kk, m.Ek, m.p.p, m.q.p, m.lv[0].fix, a);
         rb.add(RL<double, TP>{{}, m.n, m.r.p, MG::same() ? nullptr : m.rP.p, m.q.p, m.z.p,
-                              m.dots.p, m.red, m.st.p},
+                              m.dots.p, m.red, m.st.p, m.firstStep(0)},
                unsigned(vblocks(m.n)));
       }
       push(iter, op.finish(s, qc.p));

@@ -59,7 +59,7 @@ __device__ __forceinline__ T epilogue(T Au, T uself, long long i, const Epi<T> &
     return uself + ep.omega * __ldg(ep.dinv + i) * r;
   T dn = ep.c2 * __ldg(ep.dinv + i) * r;
   if(ep.c1 != T(0))
-    dn += ep.c1 * (uself - y[i]);
+    dn += ep.c1 * (uself - (ep.prev0 ? T(0) : y[i]));
   return uself + dn;
 }
 
@@ -441,7 +441,7 @@ __global__ void __launch_bounds__(TX *TYK, MINB)
           if(MODE >= OP_JACOBI)
             in.dinv[c] = __ldg(at_byte(ep.dinv + c * ld, node));
           if(MODE == OP_CHEB)
-            in.d[c] = ep.c1 != T(0) ? *at_byte(y + c * ld, node) : T(0); // the previous iterate
+            in.d[c] = ep.c1 != T(0) && !ep.prev0 ? *at_byte(y + c * ld, node) : T(0); // the previous iterate
         }
       }
     };
@@ -750,8 +750,8 @@ __global__ void __launch_bounds__(TX *TW, MINB)
         }
         if(MODE == OP_CHEB)
         {
-          pv1[c] = (own1 && ep.c1 != T(0)) ? y[i1] : T(0);
-          pv2[c] = (own2 && ep.c1 != T(0)) ? y[i2] : T(0);
+          pv1[c] = (own1 && ep.c1 != T(0) && !ep.prev0) ? y[i1] : T(0);
+          pv2[c] = (own2 && ep.c1 != T(0) && !ep.prev0) ? y[i2] : T(0);
         }
       }
     }
@@ -940,7 +940,7 @@ __device__ __forceinline__ void q4_body(const KMat<T, 8> &K, const Dims &d, cons
           bv[c] = __ldg(ep.b + i);
         if(MODE >= OP_JACOBI)
           dv[c] = __ldg(ep.dinv + i);
-        if(MODE == OP_CHEB && ep.c1 != T(0))
+        if(MODE == OP_CHEB && ep.c1 != T(0) && !ep.prev0)
           yp[c] = y[i];
       }
     }
@@ -1532,7 +1532,7 @@ static void launch_op_mode(const Dims &d, const T *K, const T *E, const T *u, T 
 {
   RedScratch red = x.dotRed ? *x.dotRed : RedScratch{};
   const int target = num_sms() * 4;
-  Epi<T> ep{x.b, x.dinv, T(x.omega), T(x.c1), T(x.c2)};
+  Epi<T> ep{x.b, x.dinv, T(x.omega), T(x.c1), T(x.c2), x.prev0};
   if(d.dim == 3)
   {
     // element rows per tile: 8; 12 for the FP64 product and residual without a

@@ -260,7 +260,7 @@ template <bool DOT, int MODE> struct LayerOps
         bb[c] = __ldg(ep.b + c * ld + node);
       if(MODE >= OP_JACOBI)
         dv[c] = __ldg(ep.dinv + c * ld + node);
-      if(MODE == OP_CHEB && ep.c1 != 0.f)
+      if(MODE == OP_CHEB && ep.c1 != 0.f && !ep.prev0)
         dp[c] = y[c * ld + node]; // the previous iterate (y is written after)
     }
   }
@@ -570,7 +570,7 @@ void launch_tc_mode(const Dims &d, const float *K, const float *E, const float *
   w.spin = tc_spin_limit();
   const int grid = std::min(w.items, slots);
   RedScratch red = x.dotRed ? *x.dotRed : RedScratch{};
-  Epi<float> ep{x.b, x.dinv, float(x.omega), float(x.c1), float(x.c2)};
+  Epi<float> ep{x.b, x.dinv, float(x.omega), float(x.c1), float(x.c2), x.prev0};
   if(x.dotRed)
     ICB_REQUIRE(grid <= red.maxBlocks, "reduction scratch too small");
   kern<<<grid, dim3(TX, TY), smem, s>>>(km, d, w, E, u, y, fix, red, x.dotOut, x.gate,
