@@ -918,9 +918,9 @@ __device__ __forceinline__ void q4_body(const KMat<T, 8> &K, const Dims &d, cons
   // its strip of that row, so the total does not depend on how the rows are
   // cut into blocks
   const int strips = nbx * TY2, strip = bxi * TY2 + w;
-  // the inputs of the update of row ej's output node (FP32: loaded a row
-  // ahead, with the next node row; the previous iterate in y is read before
-  // this thread, its only writer, overwrites it)
+  // the inputs of the update of row ej's output node (FP32, and FP64 where the
+  // registers allow: loaded a row ahead, with the next node row; the previous
+  // iterate in y is read before this thread, its only writer, overwrites it)
   auto load_inp = [&](int ej, unsigned &f, T(&us)[2], T(&bv)[2], T(&dv)[2], T(&yp)[2]) {
     f = 0;
 #pragma unroll
@@ -945,7 +945,7 @@ __device__ __forceinline__ void q4_body(const KMat<T, 8> &K, const Dims &d, cons
       }
     }
   };
-  constexpr bool kAhead = sizeof(T) == 4;
+  constexpr bool kAhead = sizeof(T) == 4 || MODE == OP_APPLY;
   unsigned nf = 0;
   T nus[2], nbv[2], ndv[2], nyp[2];
   if(kAhead)
