@@ -15,6 +15,7 @@
 #include <algorithm>
 
 #include "icb_internal.hpp"
+#include "reduce.cuh"
 
 namespace icb
 {
@@ -39,18 +40,18 @@ struct BatchQueue
 /// items per chunk: 1 while every item gets a CTA of its own in one wave
 /// (small launches stay fully parallel), more for launches many waves long,
 /// so a converged problem's items are skipped several at a time
+constexpr int kMaxChunk = 16;
 inline int queue_chunk(int items, int capacity)
 {
-  return std::max(1, std::min(16, items / std::max(1, 2 * capacity)));
+  return std::max(1, std::min(kMaxChunk, items / std::max(1, 2 * capacity)));
 }
 
 /// nb(rec): blocks of a record's own grid; skip(rec): the record's blocks
 /// have nothing to do (read by one thread, the same for the whole record
-/// while any of its blocks is pending); run(rec, b, fresh): block b of the
-/// record, fresh when the CTA's previous item was of another record (what
-/// a body stages per record in shared memory survives until then)
+/// while any of its blocks is pending); run(rec, b, n): blocks b .. b + n - 1
+/// of the record, at most a chunk
 template <class Rec, class Nb, class Skip, class Run>
-__device__ __forceinline__ void batch_queue(const Rec *__restrict__ D, const int2 *__restrict__ map,
+__device__ __forceinline__ void batch_runs(const Rec *__restrict__ D, const int2 *__restrict__ map,
                                             const BatchQueue &q, Nb nb, Skip skip, Run run)
 {
   __shared__ int base, jump;
@@ -65,37 +66,33 @@ __device__ __forceinline__ void batch_queue(const Rec *__restrict__ D, const int
     if(b0 >= q.items)
       break;
     const int b1 = min(b0 + q.chunk, q.items);
-    int running = -1; // the record of the last item run: not skipped
     for(int it = b0; it < b1;)
     {
       const int2 m = map[it];
       const Rec &r = D[m.x];
+      const int left = nb(r) - m.y;
       // a record found running stays so while any of its items is pending
-      const bool fresh = m.x != running;
-      if(fresh)
+      if(lead)
       {
-        if(lead)
-        {
-          jump = skip(r) ? nb(r) - m.y : 0;
-          // the record's items are contiguous in the map: move the queue
-          // past its last one, so no CTA takes another chunk of it (chunks
-          // already taken skip it here)
-          if(jump > 0)
-            atomicMax(q.next, unsigned(it + jump));
-        }
-        __syncthreads();
-        const int j = jump;
-        __syncthreads();
-        if(j > 0)
-        {
-          it += j;
-          continue;
-        }
-        running = m.x;
+        jump = skip(r) ? left : 0;
+        // the record's items are contiguous in the map: move the queue
+        // past its last one, so no CTA takes another chunk of it (chunks
+        // already taken skip it here)
+        if(jump > 0)
+          atomicMax(q.next, unsigned(it + jump));
       }
-      run(r, m.y, fresh);
-      __syncthreads(); // the bodies' shared memory is reused by the next item
-      ++it;
+      __syncthreads();
+      const int j = jump;
+      __syncthreads();
+      if(j > 0)
+      {
+        it += j;
+        continue;
+      }
+      const int n = min(b1 - it, left);
+      run(r, m.y, n);
+      __syncthreads(); // the bodies' shared memory is reused by the next run
+      it += n;
     }
   }
   if(lead)
@@ -108,6 +105,69 @@ __device__ __forceinline__ void batch_queue(const Rec *__restrict__ D, const int
       *q.done = 0u;
     }
   }
+}
+
+/// the items one at a time: run(rec, b, fresh), block b of the record, fresh
+/// when it is the first of its run (what a body stages per record in shared
+/// memory survives from there)
+template <class Rec, class Nb, class Skip, class Run>
+__device__ __forceinline__ void batch_queue(const Rec *__restrict__ D, const int2 *__restrict__ map,
+                                            const BatchQueue &q, Nb nb, Skip skip, Run run)
+{
+  batch_runs(D, map, q, nb, skip, [&](const Rec &r, int b, int n) {
+    for(int t = 0; t < n; t++)
+    {
+      if(t)
+        __syncthreads();
+      run(r, b + t, t == 0);
+    }
+  });
+}
+
+/// Blocks b0 .. b0 + n - 1 of a launch with a grid-wide sum (T threads, gx
+/// blocks): acc(B, v) does block B's work and adds to v.  The blocks' partials,
+/// and so the total, are those of their own launch; but the run has one
+/// barrier, one fence and one ticket, where a block at a time takes those after
+/// its few entries a thread -- a chain of latencies that bounded these kernels
+/// (32 designs of 6.1M DOFs, a block at a time and in runs: residual update 96
+/// and 66 us, r.z 49 and 35, x and p 76 and 50).
+template <int NV, int T, class Acc, class Fin>
+__device__ __forceinline__ void sum_runs(int b0, int n, unsigned gx, const RedScratch &red,
+                                         const Acc &acc, const Fin &fin)
+{
+  __shared__ double part[kMaxChunk][T / 32][NV], sw[32][NV];
+  __shared__ int last;
+  const int tid = threadIdx.x;
+  for(int t = 0; t < n; t++)
+  {
+    double v[NV] = {};
+    acc(Blk{unsigned(b0 + t), 0, 0, gx, 1, 1}, v);
+#pragma unroll
+    for(int k = 0; k < NV; k++)
+      v[k] = warp_sum_d(v[k]);
+    if((tid & 31) == 0)
+#pragma unroll
+      for(int k = 0; k < NV; k++)
+        part[t][tid >> 5][k] = v[k];
+  }
+  __syncthreads();
+  static_assert(kMaxChunk * NV <= T, "a partial a thread");
+  if(tid < n * NV)
+  {
+    double s = 0.0;
+    for(int w = 0; w < T / 32; w++)
+      s += part[tid / NV][w][tid % NV];
+    red.partials[(long long)b0 * NV + tid] = s;
+    __threadfence();
+  }
+  __syncthreads();
+  if(tid == 0)
+    last = ticket_acq_rel(red.counter, unsigned(n)) + unsigned(n) == gx;
+  __syncthreads();
+  if(!last)
+    return;
+  __threadfence();
+  partials_finish<NV>(sw, red, fin, int(gx));
 }
 
 /// CTAs of a persistent batched launch (the kernel's residency on every SM,

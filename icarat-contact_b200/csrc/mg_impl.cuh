@@ -102,7 +102,7 @@ template <typename T> struct FirstStep
 /// division): along a halved axis the 1-D weights of the fine neighbours
 /// 2I-1, 2I, 2I+1 are 1/2, 1, 1/2 (those inside the fine grid), along a kept
 /// axis (shift 0) the fine node I alone has weight 1; applied row by row.
-template <typename T>
+template <typename T, int DIM>
 __device__ __forceinline__ void restrict_b(Dims df, Dims dc, int3 sh, const T *__restrict__ rf,
                            T *__restrict__ bc, const uint8_t *__restrict__ fixc,
                            const KState *gate, const FirstStep<T> &first, const Blk &B)
@@ -113,14 +113,42 @@ __device__ __forceinline__ void restrict_b(Dims df, Dims dc, int3 sh, const T *_
   if(I >= dc.sx)
     return;
   const long long fsxy = (long long)df.sx * df.sy;
-  const int kr = df.dim == 3 ? sh.z : 0;
+  const int kr = DIM == 3 ? sh.z : 0;
   const T h = T(0.5);
   T s[3] = {T(0), T(0), T(0)}, dv[3];
   const long long n = I + (long long)J * dc.sx + (long long)K * dc.sx * dc.sy;
   const unsigned fx = fixc[n];
 #pragma unroll
   for(int c = 0; c < 3; c++)
-    dv[c] = c < dc.dim ? first.load(c * dc.ld + n) : T(0);
+    dv[c] = c < DIM ? first.load(c * dc.ld + n) : T(0);
+  if(DIM == 2 && sh.x && sh.y)
+  {
+    // a 2D grid halved on both axes: the nine fine values of both components
+    // loaded before any is summed (a row past the grid adds +0), in the
+    // general form's order
+    T v[2][3];
+#pragma unroll
+    for(int r = 0; r < 3; r++)
+    {
+      const int j = 2 * J + r - 1, i = 2 * I;
+      const bool in = j >= 0 && j < df.sy;
+      const bool lo = in && i >= 1, mid = in && i < df.sx, hi = in && i + 1 < df.sx;
+#pragma unroll
+      for(int c = 0; c < 2; c++)
+      {
+        const T *q = rf + c * df.ld + (long long)j * df.sx;
+        v[c][r] = (mid ? q[i] : T(0)) + h * ((lo ? q[i - 1] : T(0)) + (hi ? q[i + 1] : T(0)));
+      }
+    }
+#pragma unroll
+    for(int c = 0; c < 2; c++)
+    {
+      T sk = fma(h, v[c][0], T(0));
+      sk = sk + v[c][1];
+      s[c] = T(0) + fma(h, v[c][2], sk);
+    }
+  }
+  else
   for(int dk = -kr; dk <= kr; dk++)
   {
     const int k = (K << sh.z) + dk;
@@ -137,7 +165,7 @@ __device__ __forceinline__ void restrict_b(Dims df, Dims dc, int3 sh, const T *_
       const bool lo = sh.x && i - 1 >= 0, mid = i < df.sx, hi = sh.x && i + 1 < df.sx;
 #pragma unroll
       for(int c = 0; c < 3; c++)
-        if(c < df.dim)
+        if(c < DIM)
         {
           const T *r = rf + c * df.ld + row;
           const T v = (mid ? r[i] : T(0)) + h * ((lo ? r[i - 1] : T(0)) + (hi ? r[i + 1] : T(0)));
@@ -150,19 +178,19 @@ __device__ __forceinline__ void restrict_b(Dims df, Dims dc, int3 sh, const T *_
   }
 #pragma unroll
   for(int c = 0; c < 3; c++)
-    if(c < dc.dim)
+    if(c < DIM)
     {
       const T v = ((fx >> c) & 1u) ? T(0) : s[c];
       bc[c * dc.ld + n] = v;
       first.store(c * dc.ld + n, dv[c], v);
     }
 }
-template <typename T>
+template <typename T, int DIM>
 __global__ void k_restrict(Dims df, Dims dc, int3 sh, const T *__restrict__ rf,
                            T *__restrict__ bc, const uint8_t *__restrict__ fixc,
                            const KState *gate, const FirstStep<T> first)
 {
-  restrict_b<T>(df, dc, sh, rf, bc, fixc, gate, first, this_block());
+  restrict_b<T, DIM>(df, dc, sh, rf, bc, fixc, gate, first, this_block());
 }
 
 /// x_f += P x_c, constrained fine DOFs untouched (they stay 0).  One thread
@@ -173,7 +201,7 @@ __global__ void k_restrict(Dims df, Dims dc, int3 sh, const T *__restrict__ rf,
 /// thread loads its rows' fine values and flags first and then the coarse
 /// values, so the loads of all its rows are in flight together.
 constexpr int kProlongRows = 4;
-template <typename T>
+template <typename T, int DIM>
 __device__ __forceinline__ void prolong_rows_b(const Dims &df, const Dims &dc, const int3 &sh,
                                                const T *__restrict__ xc, T *__restrict__ xf,
                                                const uint8_t *__restrict__ fixf, int i, int j0,
@@ -193,10 +221,35 @@ __device__ __forceinline__ void prolong_rows_b(const Dims &df, const Dims &dc, c
     fx[r] = j < df.sy ? unsigned(fixf[n]) : 7u; // a row past the grid: nothing to do
 #pragma unroll
     for(int c = 0; c < 3; c++)
-      old[r][c] = c < df.dim && !((fx[r] >> c) & 1u) ? xf[c * df.ld + n] : T(0);
+      old[r][c] = c < DIM && !((fx[r] >> c) & 1u) ? xf[c * df.ld + n] : T(0);
+  }
+  if(DIM == 2 && sh.x && sh.y)
+  {
+    // a 2D grid halved on both axes: the R rows lie between R/2 + 1 coarse rows
+    // (j0 is a multiple of R), whose midpoints along x they share; a midpoint of
+    // equal values is that value, so the two of the general form along z drop out
+    static_assert(R % 2 == 0, "a group of fine rows starts on a coarse row");
+    const int I0 = i >> 1, I1 = (i + 1) >> 1, J = j0 >> 1;
+    T a[R / 2 + 1][2];
+#pragma unroll
+    for(int q = 0; q <= R / 2; q++)
+    {
+      const T *x = xc + (long long)min(J + q, dc.sy - 1) * dc.sx; // (the clamped row is not used)
+#pragma unroll
+      for(int c = 0; c < 2; c++)
+        a[q][c] = T(0.5) * (x[c * dc.ld + I0] + x[c * dc.ld + I1]);
+    }
+#pragma unroll
+    for(int r = 0; r < R; r++)
+#pragma unroll
+      for(int c = 0; c < 2; c++)
+        if(!((fx[r] >> c) & 1u))
+          xf[c * df.ld + i + (long long)(j0 + r) * df.sx] =
+              old[r][c] + T(0.5) * (a[r / 2][c] + a[(r + 1) / 2][c]);
+    return;
   }
   const int I0 = i >> sh.x, I1 = (i + sh.x) >> sh.x;
-  const int K0 = k >> sh.z, K1 = df.dim == 3 ? (k + sh.z) >> sh.z : K0;
+  const int K0 = k >> sh.z, K1 = DIM == 3 ? (k + sh.z) >> sh.z : K0;
   const long long csxy = (long long)dc.sx * dc.sy;
   const T h = T(0.5);
 #pragma unroll
@@ -209,7 +262,7 @@ __device__ __forceinline__ void prolong_rows_b(const Dims &df, const Dims &dc, c
     const long long n = i + (long long)j * df.sx + (long long)k * fsxy;
 #pragma unroll
     for(int c = 0; c < 3; c++)
-      if(c < df.dim && !((fx[r] >> c) & 1u))
+      if(c < DIM && !((fx[r] >> c) & 1u))
       {
         const T *x = xc + c * dc.ld;
         const T a = h * (x[r00 + I0] + x[r00 + I1]), b = h * (x[r10 + I0] + x[r10 + I1]);
@@ -223,14 +276,14 @@ inline unsigned prolong_row_blocks(const Dims &d)
 {
   return unsigned((d.sy + kProlongRows - 1) / kProlongRows);
 }
-template <typename T>
+template <typename T, int DIM>
 __global__ void k_prolong_add(Dims df, Dims dc, int3 sh, const T *__restrict__ xc,
                               T *__restrict__ xf, const uint8_t *__restrict__ fixf,
                               const KState *gate)
 {
   if(gated(gate))
     return;
-  prolong_rows_b<T>(df, dc, sh, xc, xf, fixf, blockIdx.x * blockDim.x + threadIdx.x,
+  prolong_rows_b<T, DIM>(df, dc, sh, xc, xf, fixf, blockIdx.x * blockDim.x + threadIdx.x,
                     blockIdx.y * kProlongRows, blockIdx.z);
 }
 
@@ -686,10 +739,9 @@ struct FinInitMg
 
 template <typename TK, typename TP>
 __device__ __forceinline__ void mg_init_b(long long n, const TK *__restrict__ b, TK *__restrict__ x,
-                          TK *__restrict__ r, TP *__restrict__ rP, RedScratch red, KState *st,
-                          double tol, int maxit, const FirstStep<TP> &first, const Blk &B)
+                          TK *__restrict__ r, TP *__restrict__ rP,
+                          const FirstStep<TP> &first, const Blk &B, double (&v)[1])
 {
-  double v[1] = {0.0};
   const long long sd = (long long)B.gx * blockDim.x;
   for(long long i0 = B.x * (long long)blockDim.x + threadIdx.x; i0 < n; i0 += kGroup * sd)
   {
@@ -717,14 +769,15 @@ __device__ __forceinline__ void mg_init_b(long long n, const TK *__restrict__ b,
       }
     }
   }
-  block_reduce_at<1>(v, red, FinInitMg{st, tol, maxit}, int(B.x), int(B.gx));
 }
 template <typename TK, typename TP>
 __global__ void k_mg_init(long long n, const TK *__restrict__ b, TK *__restrict__ x,
                           TK *__restrict__ r, TP *__restrict__ rP, RedScratch red, KState *st,
                           double tol, int maxit, const FirstStep<TP> first)
 {
-  mg_init_b<TK, TP>(n, b, x, r, rP, red, st, tol, maxit, first, this_block());
+  double v[1] = {0.0};
+  mg_init_b<TK, TP>(n, b, x, r, rP, first, this_block(), v);
+  block_reduce<1>(v, red, FinInitMg{st, tol, maxit});
 }
 
 struct FinRz0
@@ -744,11 +797,8 @@ struct FinRz0
 /// p = z; rz = r.z
 template <typename TK, typename TP>
 __device__ __forceinline__ void mg_init2_b(long long n, const TK *__restrict__ r, const TP *__restrict__ z,
-                           TK *__restrict__ p, RedScratch red, KState *st, const Blk &B)
+                           TK *__restrict__ p, const Blk &B, double (&v)[1])
 {
-  if(st->stop)
-    return;
-  double v[1] = {0.0};
   const long long sd = (long long)B.gx * blockDim.x;
   for(long long i0 = B.x * (long long)blockDim.x + threadIdx.x; i0 < n; i0 += kGroup * sd)
   {
@@ -773,13 +823,16 @@ __device__ __forceinline__ void mg_init2_b(long long n, const TK *__restrict__ r
       }
     }
   }
-  block_reduce_at<1>(v, red, FinRz0{st}, int(B.x), int(B.gx));
 }
 template <typename TK, typename TP>
 __global__ void k_mg_init2(long long n, const TK *__restrict__ r, const TP *__restrict__ z,
                            TK *__restrict__ p, RedScratch red, KState *st)
 {
-  mg_init2_b<TK, TP>(n, r, z, p, red, st, this_block());
+  if(st->stop)
+    return;
+  double v[1] = {0.0};
+  mg_init2_b<TK, TP>(n, r, z, p, this_block(), v);
+  block_reduce<1>(v, red, FinRz0{st});
 }
 
 struct FinRmg
@@ -810,55 +863,56 @@ struct FinRmg
   }
 };
 
+/// alpha = rz / p.q, read before the sweep that uses it
+struct StepLen
+{
+  double pq, alpha;
+  bool bad;
+  __device__ __forceinline__ StepLen(const KState *st, const double *q)
+      : pq(*q), alpha(st->rz / pq), bad(!(pq > 0.0) || !isfinite(alpha))
+  {
+  }
+};
 /// r -= alpha q (and rP = TP(r)); sums r.r and r.z_old (z still holds the
 /// previous preconditioned residual) for the flexible beta
 template <typename TK, typename TP>
 __device__ __forceinline__ void mg_r_b(long long n, TK *__restrict__ r, TP *__restrict__ rP,
-                       const TK *__restrict__ q, const TP *__restrict__ zold,
-                       const double *__restrict__ pq, RedScratch red, KState *st,
-                       const FirstStep<TP> &first, const Blk &B)
+                       const TK *__restrict__ q, const TP *__restrict__ zold, const StepLen &L,
+                       const FirstStep<TP> &first, const Blk &B, double (&v)[2])
 {
-  if(st->stop)
+  if(L.bad)
     return;
-  const double pqv = *pq;
-  const double alpha = st->rz / pqv;
-  const bool bad = !(pqv > 0.0) || !isfinite(alpha);
-  double v[2] = {0.0, 0.0};
-  if(!bad)
+  const TK a = TK(L.alpha);
+  const long long sd = (long long)B.gx * blockDim.x;
+  for(long long i0 = B.x * (long long)blockDim.x + threadIdx.x; i0 < n; i0 += kGroup * sd)
   {
-    const TK a = TK(alpha);
-    const long long sd = (long long)B.gx * blockDim.x;
-    for(long long i0 = B.x * (long long)blockDim.x + threadIdx.x; i0 < n; i0 += kGroup * sd)
+    TK rv[kGroup], qv[kGroup];
+    TP zv[kGroup], dv[kGroup];
+#pragma unroll
+    for(int g = 0; g < kGroup; g++)
     {
-      TK rv[kGroup], qv[kGroup];
-      TP zv[kGroup], dv[kGroup];
+      const long long i = i0 + g * sd;
+      rv[g] = i < n ? r[i] : TK(0);
+      qv[g] = i < n ? q[i] : TK(0);
+      zv[g] = i < n ? zold[i] : TP(0);
+      dv[g] = i < n ? first.load(i) : TP(0);
+    }
 #pragma unroll
-      for(int g = 0; g < kGroup; g++)
+    for(int g = 0; g < kGroup; g++)
+    {
+      const long long i = i0 + g * sd;
+      if(i < n)
       {
-        const long long i = i0 + g * sd;
-        rv[g] = i < n ? r[i] : TK(0);
-        qv[g] = i < n ? q[i] : TK(0);
-        zv[g] = i < n ? zold[i] : TP(0);
-        dv[g] = i < n ? first.load(i) : TP(0);
-      }
-#pragma unroll
-      for(int g = 0; g < kGroup; g++)
-      {
-        const long long i = i0 + g * sd;
-        if(i < n)
-        {
-          TK ri = rv[g] - a * qv[g];
-          r[i] = ri;
-          if(rP)
-            rP[i] = TP(ri);
-          first.store(i, dv[g], TP(ri));
-          v[0] += double(ri) * double(ri);
-          v[1] += double(ri) * double(zv[g]);
-        }
+        TK ri = rv[g] - a * qv[g];
+        r[i] = ri;
+        if(rP)
+          rP[i] = TP(ri);
+        first.store(i, dv[g], TP(ri));
+        v[0] += double(ri) * double(ri);
+        v[1] += double(ri) * double(zv[g]);
       }
     }
   }
-  block_reduce_at<2>(v, red, FinRmg{st, pqv, alpha, bad}, int(B.x), int(B.gx));
 }
 template <typename TK, typename TP>
 __global__ void k_mg_r(long long n, TK *__restrict__ r, TP *__restrict__ rP,
@@ -866,7 +920,12 @@ __global__ void k_mg_r(long long n, TK *__restrict__ r, TP *__restrict__ rP,
                        const double *__restrict__ pq, RedScratch red, KState *st,
                        const FirstStep<TP> first)
 {
-  mg_r_b<TK, TP>(n, r, rP, q, zold, pq, red, st, first, this_block());
+  if(st->stop)
+    return;
+  const StepLen L(st, pq);
+  double v[2] = {0.0, 0.0};
+  mg_r_b<TK, TP>(n, r, rP, q, zold, L, first, this_block(), v);
+  block_reduce<2>(v, red, FinRmg{st, L.pq, L.alpha, L.bad});
 }
 
 struct FinRz
@@ -889,11 +948,8 @@ struct FinRz
 
 template <typename TK, typename TP>
 __device__ __forceinline__ void mg_rz_b(long long n, const TK *__restrict__ r, const TP *__restrict__ z,
-                        RedScratch red, KState *st, const Blk &B)
+                        const Blk &B, double (&v)[1])
 {
-  if(st->stop || st->conv)
-    return;
-  double v[1] = {0.0};
   const long long sd = (long long)B.gx * blockDim.x;
   for(long long i0 = B.x * (long long)blockDim.x + threadIdx.x; i0 < n; i0 += kGroup * sd)
   {
@@ -911,13 +967,16 @@ __device__ __forceinline__ void mg_rz_b(long long n, const TK *__restrict__ r, c
       if(i0 + g * sd < n)
         v[0] += double(rv[g]) * double(zv[g]);
   }
-  block_reduce_at<1>(v, red, FinRz{st}, int(B.x), int(B.gx));
 }
 template <typename TK, typename TP>
 __global__ void k_mg_rz(long long n, const TK *__restrict__ r, const TP *__restrict__ z,
                         RedScratch red, KState *st)
 {
-  mg_rz_b<TK, TP>(n, r, z, red, st, this_block());
+  if(st->stop || st->conv)
+    return;
+  double v[1] = {0.0};
+  mg_rz_b<TK, TP>(n, r, z, this_block(), v);
+  block_reduce<1>(v, red, FinRz{st});
 }
 
 struct FinXPmg
@@ -945,16 +1004,9 @@ struct FinXPmg
 /// whether the device runs the next one
 template <typename TK, typename TP>
 __device__ __forceinline__ void mg_xp_b(long long n, TK *__restrict__ x, TK *__restrict__ p,
-                        const TP *__restrict__ z, RedScratch red, KState *st, LoopCtl L, const Blk &B)
+                        const TP *__restrict__ z, const TK a, const TK bt, const bool conv,
+                        const Blk &B)
 {
-  if(st->stop)
-  {
-    if(B.x == 0 && threadIdx.x == 0)
-      loop_stop(L);
-    return;
-  }
-  const TK a = TK(st->alpha), bt = TK(st->beta);
-  const bool conv = st->conv;
   const long long sd = (long long)B.gx * blockDim.x;
   for(long long i0 = B.x * (long long)blockDim.x + threadIdx.x; i0 < n; i0 += kGroup * sd)
   {
@@ -981,14 +1033,20 @@ __device__ __forceinline__ void mg_xp_b(long long n, TK *__restrict__ x, TK *__r
       }
     }
   }
-  double v[1] = {0.0};
-  block_reduce_at<1>(v, red, FinXPmg{st, L}, int(B.x), int(B.gx));
 }
 template <typename TK, typename TP>
 __global__ void k_mg_xp(long long n, TK *__restrict__ x, TK *__restrict__ p,
                         const TP *__restrict__ z, RedScratch red, KState *st, LoopCtl L)
 {
-  mg_xp_b<TK, TP>(n, x, p, z, red, st, L, this_block());
+  if(st->stop)
+  {
+    if(blockIdx.x == 0 && threadIdx.x == 0)
+      loop_stop(L);
+    return;
+  }
+  mg_xp_b<TK, TP>(n, x, p, z, TK(st->alpha), TK(st->beta), st->conv != 0, this_block());
+  double v[1] = {0.0};
+  block_reduce<1>(v, red, FinXPmg{st, L});
 }
 } // namespace
 
@@ -1453,8 +1511,8 @@ template <typename TK, typename TP> struct MgPcg
       k_restrict3<TP><<<gr, kTB, 0, s>>>(L.d, Cn.d, planes, L.r.p, Cn.b.p, Cn.fix, gate, firstStep(l + 1));
     }
     else
-      k_restrict<TP><<<gr, kTB, 0, s>>>(L.d, Cn.d, Cn.sh, L.r.p, Cn.b.p, Cn.fix, gate,
-                                        firstStep(l + 1));
+      (L.d.dim == 2 ? k_restrict<TP, 2> : k_restrict<TP, 3>)<<<gr, kTB, 0, s>>>(
+          L.d, Cn.d, Cn.sh, L.r.p, Cn.b.p, Cn.fix, gate, firstStep(l + 1));
     count_launch();
     level(l + 1, Cn.b.p, Cn.x.p, s, gate);
     dim3 gp = grid3(L.d);
@@ -1467,7 +1525,8 @@ template <typename TK, typename TP> struct MgPcg
     else
     {
       gp.y = prolong_row_blocks(L.d);
-      k_prolong_add<TP><<<gp, kTB, 0, s>>>(L.d, Cn.d, Cn.sh, Cn.x.p, cur, L.fix, gate);
+      (L.d.dim == 2 ? k_prolong_add<TP, 2> : k_prolong_add<TP, 3>)<<<gp, kTB, 0, s>>>(
+          L.d, Cn.d, Cn.sh, Cn.x.p, cur, L.fix, gate);
     }
     count_launch();
     for(int k = 0; k < nu; k++)

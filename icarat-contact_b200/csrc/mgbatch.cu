@@ -35,19 +35,29 @@ namespace
 template <class L> struct BatchThreads
 {
   static constexpr int v = 256; ///< threads of a block at most
+  static constexpr int ctas = 1; ///< CTAs of an SM that registers are kept for
+};
+template <class L, class = void> struct TakesRuns : std::false_type
+{
+};
+template <class L> struct TakesRuns<L, std::void_t<decltype(&L::runs)>> : std::true_type
+{
 };
 template <class L>
-__global__ void __launch_bounds__(BatchThreads<L>::v) k_batch(const L *__restrict__ D, const int2 *__restrict__ map, BatchQueue q)
+__global__ void __launch_bounds__(BatchThreads<L>::v, BatchThreads<L>::ctas)
+    k_batch(const L *__restrict__ D, const int2 *__restrict__ map, BatchQueue q)
 {
-  batch_queue(
-      D, map, q, [](const L &l) { return int(l.g.gx * l.g.gy * l.g.gz); },
-      [](const L &l) { return l.skip(); },
-      [](const L &l, int bi, bool) {
-        const unsigned b = unsigned(bi);
-        const Blk B{b % l.g.gx, (b / l.g.gx) % l.g.gy, b / (l.g.gx * l.g.gy), l.g.gx, l.g.gy,
-                    l.g.gz};
-        l.run(B);
-      });
+  const auto nb = [](const L &l) { return int(l.g.gx * l.g.gy * l.g.gz); };
+  const auto skip = [](const L &l) { return l.skip(); };
+  if constexpr(TakesRuns<L>::value)
+    batch_runs(D, map, q, nb, skip, [](const L &l, int b, int n) { l.runs(b, n); });
+  else
+    batch_queue(D, map, q, nb, skip, [](const L &l, int bi, bool) {
+      const unsigned b = unsigned(bi);
+      const Blk B{b % l.g.gx, (b / l.g.gx) % l.g.gy, b / (l.g.gx * l.g.gy), l.g.gx, l.g.gy,
+                  l.g.gz};
+      l.run(B);
+    });
 }
 
 // the per-problem launches as records: the kernel's arguments and its grid
@@ -64,9 +74,12 @@ template <typename TK, typename TP> struct InitL
   int maxit;
   FirstStep<TP> first;
   __device__ bool skip() const { return false; }
-  __device__ void run(const Blk &B) const
+  __device__ void runs(int b0, int nr) const
   {
-    mg_init_b<TK, TP>(n, b, x, r, rP, red, st, tol, maxit, first, B);
+    sum_runs<1, VB>(
+        b0, nr, g.gx, red,
+        [&](const Blk &B, double(&v)[1]) { mg_init_b<TK, TP>(n, b, x, r, rP, first, B, v); },
+        FinInitMg{st, tol, maxit});
   }
 };
 template <typename TK, typename TP> struct Init2L
@@ -79,7 +92,12 @@ template <typename TK, typename TP> struct Init2L
   RedScratch red;
   KState *st;
   __device__ bool skip() const { return st->stop != 0; }
-  __device__ void run(const Blk &B) const { mg_init2_b<TK, TP>(n, r, z, p, red, st, B); }
+  __device__ void runs(int b0, int nr) const
+  {
+    sum_runs<1, VB>(
+        b0, nr, g.gx, red,
+        [&](const Blk &B, double(&v)[1]) { mg_init2_b<TK, TP>(n, r, z, p, B, v); }, FinRz0{st});
+  }
 };
 template <typename TK, typename TP> struct RL
 {
@@ -94,7 +112,14 @@ template <typename TK, typename TP> struct RL
   KState *st;
   FirstStep<TP> first;
   __device__ bool skip() const { return st->stop != 0; }
-  __device__ void run(const Blk &B) const { mg_r_b<TK, TP>(n, r, rP, q, z, pq, red, st, first, B); }
+  __device__ void runs(int b0, int nr) const
+  {
+    const StepLen a(st, pq);
+    sum_runs<2, VB>(
+        b0, nr, g.gx, red,
+        [&](const Blk &B, double(&v)[2]) { mg_r_b<TK, TP>(n, r, rP, q, z, a, first, B, v); },
+        FinRmg{st, a.pq, a.alpha, a.bad});
+  }
 };
 template <typename TK, typename TP> struct RzL
 {
@@ -105,7 +130,12 @@ template <typename TK, typename TP> struct RzL
   RedScratch red;
   KState *st;
   __device__ bool skip() const { return st->stop || st->conv; }
-  __device__ void run(const Blk &B) const { mg_rz_b<TK, TP>(n, r, z, red, st, B); }
+  __device__ void runs(int b0, int nr) const
+  {
+    sum_runs<1, VB>(
+        b0, nr, g.gx, red,
+        [&](const Blk &B, double(&v)[1]) { mg_rz_b<TK, TP>(n, r, z, B, v); }, FinRz{st});
+  }
 };
 template <typename TK, typename TP> struct XpL
 {
@@ -116,7 +146,36 @@ template <typename TK, typename TP> struct XpL
   RedScratch red;
   KState *st;
   __device__ bool skip() const { return st->stop != 0; }
-  __device__ void run(const Blk &B) const { mg_xp_b<TK, TP>(n, x, p, z, red, st, LoopCtl{}, B); }
+  __device__ void runs(int b0, int nr) const
+  {
+    const TK a = TK(st->alpha), bt = TK(st->beta);
+    const bool conv = st->conv != 0;
+    sum_runs<1, VB>(
+        b0, nr, g.gx, red,
+        [&](const Blk &B, double(&)[1]) { mg_xp_b<TK, TP>(n, x, p, z, a, bt, conv, B); },
+        FinXPmg{st, LoopCtl{}});
+  }
+};
+// (64 registers a thread; 48 for the sweep that reads two vectors and writes none)
+struct VecThreads
+{
+  static constexpr int v = VB, ctas = 4;
+};
+template <typename TP> struct BatchThreads<InitL<double, TP>> : VecThreads
+{
+};
+template <typename TP> struct BatchThreads<Init2L<double, TP>> : VecThreads
+{
+};
+template <typename TP> struct BatchThreads<RL<double, TP>> : VecThreads
+{
+};
+template <typename TP> struct BatchThreads<XpL<double, TP>> : VecThreads
+{
+};
+template <typename TP> struct BatchThreads<RzL<double, TP>>
+{
+  static constexpr int v = VB, ctas = 5;
 };
 /// the transfers write each node from its own reads only, so a batched
 /// launch may give a block several node rows: g.gy blocks take the ry rows
@@ -138,7 +197,7 @@ template <typename T> struct RestrictL
     Blk b = B;
 #pragma unroll 2
     for(b.y = B.y; b.y < ry; b.y += B.gy)
-      restrict_b<T>(df, dc, sh, rf, bc, fixc, gate, first, b);
+      restrict_b<T, 2>(df, dc, sh, rf, bc, fixc, gate, first, b);
   }
 };
 /// g.gy blocks along y, each ry node rows from its first, kProlongRows at a
@@ -161,8 +220,16 @@ template <typename T> struct ProlongL
     const int i = B.x * blockDim.x + threadIdx.x;
     const int j1 = min(df.sy, int((B.y + 1) * ry));
     for(int j = int(B.y * ry); j < j1; j += kProlongRows)
-      prolong_rows_b<T>(df, dc, sh, xc, xf, fixf, i, j, B.z);
+      prolong_rows_b<T, 2>(df, dc, sh, xc, xf, fixf, i, j, B.z);
   }
+};
+template <typename T> struct BatchThreads<RestrictL<T>>
+{
+  static constexpr int v = kTB, ctas = 8;
+};
+template <typename T> struct BatchThreads<ProlongL<T>>
+{
+  static constexpr int v = kTB, ctas = 8;
 };
 /// Rows per work item of a batched launch whose rows are independent: one
 /// while the launch's rows (`rows`, over every problem) fill the GPU's
@@ -254,11 +321,11 @@ template <bool REG> struct InvertL
 
 template <> struct BatchThreads<InvertL<true>>
 {
-  static constexpr int v = kInvThreads;
+  static constexpr int v = kInvThreads, ctas = 1;
 };
 template <> struct BatchThreads<InvertL<false>>
 {
-  static constexpr int v = 1024;
+  static constexpr int v = 1024, ctas = 1;
 };
 
 /// number of problems whose solve has not stopped

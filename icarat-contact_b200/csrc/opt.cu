@@ -1378,43 +1378,47 @@ __global__ void __launch_bounds__(VB)
         }
       });
 }
-/// one bisection step on a tile in the column form (k_oc_update's arithmetic):
-/// the candidates of the tile and its halo into shared memory, the volume, and
-/// in a problem's last block its bisection logic
-__device__ __forceinline__ void oc_step_cols_b(const OcBatch::Rec &r, int b, double *buf)
+/// one bisection step on tiles b0 .. b0 + n - 1 in the column form (k_oc_update's
+/// arithmetic): the candidates of a tile and its halo into shared memory, the
+/// volume, and in a problem's last block its bisection logic
+__device__ __forceinline__ void oc_step_cols_b(const OcBatch::Rec &r, int b0, int n, double *buf)
 {
-  if(r.st->done)
-    return;
   const Dims &d = r.d;
   const ConeCols &C = r.cols;
   const double c = 1.0 / oc_power(r.st->lam, r.P.eta), tb = r.st->tanhTb;
-  const int x0 = int(unsigned(b) % r.ntx) * kOcTW, y0 = int(unsigned(b) / r.ntx) * kOcTH;
   const int W = kOcTW + 2 * C.hx, cells = oc_up_cells(C);
-  double aav[4], volv[4];
-  oc_tile_weights(d, x0 + int(threadIdx.x & 31), y0 + 4 * int(threadIdx.x >> 5), r.aa, r.vol, aav,
-                  volv);
-  constexpr int U = 4;
-  for(int q0 = threadIdx.x; q0 < cells; q0 += VB * U)
-  {
-    double h[U], lo[U], hi[U];
+  sum_runs<1, VB>(
+      b0, n, r.gx, r.red,
+      [&](const Blk &B, double(&v)[1]) {
+        const int x0 = int(B.x % r.ntx) * kOcTW, y0 = int(B.x / r.ntx) * kOcTH;
+        double aav[4], volv[4];
+        oc_tile_weights(d, x0 + int(threadIdx.x & 31), y0 + 4 * int(threadIdx.x >> 5), r.aa, r.vol,
+                        aav, volv);
+        if(int(B.x) != b0)
+          __syncthreads(); // the tile before is summed
+        constexpr int U = 4;
+        for(int q0 = threadIdx.x; q0 < cells; q0 += VB * U)
+        {
+          double h[U], lo[U], hi[U];
 #pragma unroll
-    for(int u = 0; u < U; u++)
-    {
-      const int q = q0 + u * VB, ty = q / W, i = x0 - C.hx + q - ty * W, j = y0 - C.hz + ty;
-      const bool in = q < cells && unsigned(i) < unsigned(d.nx) && unsigned(j) < unsigned(d.ny);
-      const long long e = i + (long long)j * d.nx;
-      h[u] = in ? __ldg(r.prep + e) : 0.0;
-      lo[u] = in ? __ldg(r.prep + d.nel + e) : 0.0;
-      hi[u] = in ? __ldg(r.prep + 2 * d.nel + e) : 0.0;
-    }
+          for(int u = 0; u < U; u++)
+          {
+            const int q = q0 + u * VB, ty = q / W, i = x0 - C.hx + q - ty * W, j = y0 - C.hz + ty;
+            const bool in = q < cells && unsigned(i) < unsigned(d.nx) && unsigned(j) < unsigned(d.ny);
+            const long long e = i + (long long)j * d.nx;
+            h[u] = in ? __ldg(r.prep + e) : 0.0;
+            lo[u] = in ? __ldg(r.prep + d.nel + e) : 0.0;
+            hi[u] = in ? __ldg(r.prep + 2 * d.nel + e) : 0.0;
+          }
 #pragma unroll
-    for(int u = 0; u < U; u++)
-      if(q0 + u * VB < cells)
-        buf[q0 + u * VB] = oc_bounded(h[u] * c, lo[u], hi[u]);
-  }
-  __syncthreads();
-  double v[1] = {oc_tile_volume(buf, W, C, aav, volv, r.P, tb)};
-  block_reduce_at<1>(v, r.red, FinOc{r.st, LoopCtl{}}, b, int(r.gx));
+          for(int u = 0; u < U; u++)
+            if(q0 + u * VB < cells)
+              buf[q0 + u * VB] = oc_bounded(h[u] * c, lo[u], hi[u]);
+        }
+        __syncthreads();
+        v[0] = oc_tile_volume(buf, W, C, aav, volv, r.P, tb);
+      },
+      FinOc{r.st, LoopCtl{}});
 }
 
 __global__ void k_oc_init_batch(const OcBatch::Rec *__restrict__ R, int n)
@@ -1438,19 +1442,27 @@ __global__ void __launch_bounds__(VB, 4)
     k_oc_step_batch(const OcBatch::Rec *__restrict__ R, const int2 *__restrict__ map, BatchQueue q)
 {
   extern __shared__ __align__(16) unsigned char oc_batch_dyn[];
-  batch_queue(
+  batch_runs(
       R, map, q, [](const OcBatch::Rec &r) { return int(r.gx); },
       [](const OcBatch::Rec &r) { return r.st->done != 0; },
-      [](const OcBatch::Rec &r, int b, bool) {
-        const Blk B{unsigned(b), 0, 0, r.gx, 1, 1};
+      [](const OcBatch::Rec &r, int b0, int n) {
         if(r.cols.ncol)
-          oc_step_cols_b(r, b, reinterpret_cast<double *>(oc_batch_dyn));
-        else if(r.tiled)
-          oc_step_tile_b(r.d, r.hx, r.hy, r.ntx, r.off, r.w, r.nnb, r.aa, r.vol, r.xc, r.P, r.red,
-                         r.st, LoopCtl{}, B, oc_batch_dyn);
-        else
-          oc_step_b(r.d, r.off, r.w, r.nnb, r.aa, r.x, r.df, r.dg, r.xmin, r.xmax, r.vol, r.xc,
-                    r.P, r.red, r.st, LoopCtl{}, B);
+        {
+          oc_step_cols_b(r, b0, n, reinterpret_cast<double *>(oc_batch_dyn));
+          return;
+        }
+        for(int b = b0; b < b0 + n; b++)
+        {
+          const Blk B{unsigned(b), 0, 0, r.gx, 1, 1};
+          if(b > b0)
+            __syncthreads();
+          if(r.tiled)
+            oc_step_tile_b(r.d, r.hx, r.hy, r.ntx, r.off, r.w, r.nnb, r.aa, r.vol, r.xc, r.P, r.red,
+                           r.st, LoopCtl{}, B, oc_batch_dyn);
+          else
+            oc_step_b(r.d, r.off, r.w, r.nnb, r.aa, r.x, r.df, r.dg, r.xmin, r.xmax, r.vol, r.xc,
+                      r.P, r.red, r.st, LoopCtl{}, B);
+        }
       });
 }
 __global__ void __launch_bounds__(256)

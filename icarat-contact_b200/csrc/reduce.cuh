@@ -15,12 +15,12 @@ namespace icb
 /// semantics at GPU scope, which orders this thread's partial stores before
 /// the ticket (release) and, for the last block, the other blocks' partials
 /// before its reads (acquire) -- without a full sequentially consistent fence
-__device__ __forceinline__ unsigned ticket_acq_rel(unsigned *counter)
+__device__ __forceinline__ unsigned ticket_acq_rel(unsigned *counter, unsigned take = 1)
 {
   unsigned t;
-  asm volatile("atom.acq_rel.gpu.add.u32 %0, [%1], 1;"
+  asm volatile("atom.acq_rel.gpu.add.u32 %0, [%1], %2;"
                : "=r"(t)
-               : "l"(counter)
+               : "l"(counter), "r"(take)
                : "memory");
   return t;
 }
@@ -31,6 +31,48 @@ __device__ __forceinline__ double warp_sum_d(double v)
   for(int o = 16; o > 0; o >>= 1)
     v += __shfl_down_sync(0xffffffffu, v, o);
   return v;
+}
+
+/// the last block's part of a grid-wide sum: the nb blocks' partials in a fixed
+/// order (thread t takes t, t + blockDim, ...; then the warps in order), the
+/// total handed to fin, the counter ready for the next launch
+template <int NV, class Fin>
+__device__ __forceinline__ void partials_finish(double (&sw)[32][NV], const RedScratch &red,
+                                                const Fin &fin, int nb)
+{
+  const int tid = threadIdx.x + blockDim.x * (threadIdx.y + blockDim.y * threadIdx.z);
+  const int nth = blockDim.x * blockDim.y * blockDim.z;
+  const int nw = (nth + 31) >> 5;
+  double s[NV];
+#pragma unroll
+  for(int k = 0; k < NV; k++)
+    s[k] = 0.0;
+  for(int b = tid; b < nb; b += nth)
+#pragma unroll
+    for(int k = 0; k < NV; k++)
+      s[k] += __ldcg(red.partials + (long long)b * NV + k);
+#pragma unroll
+  for(int k = 0; k < NV; k++)
+    s[k] = warp_sum_d(s[k]);
+  __syncthreads();
+  if((tid & 31) == 0)
+#pragma unroll
+    for(int k = 0; k < NV; k++)
+      sw[tid >> 5][k] = s[k];
+  __syncthreads();
+  if(tid == 0)
+  {
+    double tot[NV];
+#pragma unroll
+    for(int k = 0; k < NV; k++)
+    {
+      tot[k] = 0.0;
+      for(int w = 0; w < nw; w++)
+        tot[k] += sw[w][k];
+    }
+    *red.counter = 0u;
+    fin(tot);
+  }
 }
 
 /// the reduction of block `bid` of `nb` blocks: a batched launch that runs
@@ -70,36 +112,7 @@ __device__ __forceinline__ void block_reduce_at(double (&v)[NV], const RedScratc
   if(!last)
     return;
   __threadfence();
-  double s[NV];
-#pragma unroll
-  for(int k = 0; k < NV; k++)
-    s[k] = 0.0;
-  for(int b = tid; b < nb; b += nth)
-#pragma unroll
-    for(int k = 0; k < NV; k++)
-      s[k] += __ldcg(red.partials + (long long)b * NV + k);
-#pragma unroll
-  for(int k = 0; k < NV; k++)
-    s[k] = warp_sum_d(s[k]);
-  __syncthreads();
-  if((tid & 31) == 0)
-#pragma unroll
-    for(int k = 0; k < NV; k++)
-      sw[tid >> 5][k] = s[k];
-  __syncthreads();
-  if(tid == 0)
-  {
-    double tot[NV];
-#pragma unroll
-    for(int k = 0; k < NV; k++)
-    {
-      tot[k] = 0.0;
-      for(int w = 0; w < nw; w++)
-        tot[k] += sw[w][k];
-    }
-    *red.counter = 0u;
-    fin(tot);
-  }
+  partials_finish<NV>(sw, red, fin, nb);
 }
 
 /// The finish of a sum whose partials sit at slots fixed by the work, not by
@@ -126,9 +139,22 @@ __device__ __forceinline__ void slots_reduce_finish(const RedScratch &red, long 
   if(!last)
     return;
   __threadfence();
+  // one block is left to sum them: its loads eight to a group, or the sum is
+  // a chain of their latencies (640 x 320 elements, 7,704 slots on 128
+  // threads)
+  constexpr int G = 8;
   double s = 0.0;
-  for(long long k = tid; k < nslots; k += nth)
-    s += __ldcg(red.partials + k);
+  for(long long k = tid; k < nslots; k += (long long)G * nth)
+  {
+    double v[G];
+#pragma unroll
+    for(int g = 0; g < G; g++)
+      v[g] = k + (long long)g * nth < nslots ? __ldcg(red.partials + k + (long long)g * nth) : 0.0;
+#pragma unroll
+    for(int g = 0; g < G; g++)
+      if(k + (long long)g * nth < nslots)
+        s += v[g];
+  }
   s = warp_sum_d(s);
   if((tid & 31) == 0)
     sw[tid >> 5] = s;
