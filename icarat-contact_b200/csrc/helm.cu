@@ -95,18 +95,6 @@ __global__ void k_helm_diag(KMat<double, 8> K, Dims d, double *__restrict__ dinv
   dinv[n] = s != 0.0 ? 1.0 / s : 1.0;
 }
 
-/// 1-D assembled mass and stiffness stencils of one axis: off-diagonals h/6
-/// and -1/h, diagonal h/3 and 1/h per element beside the node
-struct HelmAxis
-{
-  double mo, mh, so, sh;
-};
-struct HelmTensor
-{
-  HelmAxis a[3];
-  double re2;
-};
-
 /// The 3D Helmholtz operator as a tensor-product stencil.  On the box grid
 /// the assembled M + re^2 K_grad is Mx.My.Mz + re^2 (Sx.My.Mz + Mx.Sy.Mz +
 /// Mx.My.Sz) with the 1-D assembled mass / stiffness matrices of each axis
@@ -305,7 +293,31 @@ int HelmFilter::apply(const double *in, double *out, bool sens, double tol, cuda
   else
     k_helm_rhs<2><<<nbn, 256, 0, s>>>(d, in, wr, rhs.p);
   count_launch();
+  const double wo = sens ? 1.0 : 1.0 / ne;
+  auto finish = [&](int status) {
+    if(d.dim == 3)
+      k_helm_out<3><<<nbe, 256, 0, s>>>(d, phi.p, wo, out);
+    else
+      k_helm_out<2><<<nbe, 256, 0, s>>>(d, phi.p, wo, out);
+    ICB_CUDA(cudaGetLastError());
+    count_launch();
+    return status;
+  };
+  HelmTensor T{};
+  T.re2 = std::pow(radius / (2.0 * std::sqrt(3.0)), 2);
+  for(int k = 0; k < 3; k++)
+  {
+    const double hk = k < d.dim ? h[k] : 1.0;
+    T.a[k] = HelmAxis{hk / 6.0, hk / 3.0, -1.0 / hk, 1.0 / hk};
+  }
   JacobiPcg<double> &P = *pcg;
+  // a 3D grid that fits on the chip: all iterations as one kernel (pcgtile.cu)
+  if(P.tiles.ctas())
+    return finish(P.solveTiles(
+        [&] {
+          launch_pcg_tiles(P.tiles, P.d, T, dinv.p, phi.p, P.r.p, P.p.p, P.q.p, P.st.p, s);
+        },
+        dinv.p, rhs.p, phi.p, tol, 10000, s, info));
   const Dims dd = d;
   const KMat<double, 8> KK = K;
   double *pp = P.p.p, *qp = P.q.p, *dp = P.dots.p;
@@ -314,13 +326,6 @@ int HelmFilter::apply(const double *in, double *out, bool sens, double tol, cuda
   const int nb = vblocks(d.nnode);
   // 3D: the tensor-product stencil kernel, z split so that the CTAs fill
   // the GPU about four times over within the reduction scratch
-  HelmTensor T{};
-  T.re2 = std::pow(radius / (2.0 * std::sqrt(3.0)), 2);
-  for(int k = 0; k < 3; k++)
-  {
-    const double hk = k < d.dim ? h[k] : 1.0;
-    T.a[k] = HelmAxis{hk / 6.0, hk / 3.0, -1.0 / hk, 1.0 / hk};
-  }
   const int tx = (d.sx + HTX - 1) / HTX, ty = (d.sy + HTY - 1) / HTY;
   const long long tiles = (long long)tx * ty;
   // planes per CTA: fewest rounds x (planes + 2) for the CTAs resident at once
@@ -362,15 +367,7 @@ int HelmFilter::apply(const double *in, double *out, bool sens, double tol, cuda
       k_helm_apply<2, true><<<nb, VB, 0, cs>>>(KK, dd, pp, qp, *rp, dp, sp);
     count_launch();
   };
-  int st = P.solveOp(op, this, nullptr, nullptr, dinv.p, rhs.p, phi.p, tol, 10000, s, info);
-  double wo = sens ? 1.0 : 1.0 / ne;
-  if(d.dim == 3)
-    k_helm_out<3><<<nbe, 256, 0, s>>>(d, phi.p, wo, out);
-  else
-    k_helm_out<2><<<nbe, 256, 0, s>>>(d, phi.p, wo, out);
-  ICB_CUDA(cudaGetLastError());
-  count_launch();
-  return st;
+  return finish(P.solveOp(op, this, nullptr, nullptr, dinv.p, rhs.p, phi.p, tol, 10000, s, info));
 }
 
 } // namespace icb

@@ -323,15 +323,9 @@ int JacobiPcg<T>::solve(const T *K, const T *E, const uint8_t *fix, const T *inv
   {
     // a small problem's iterations as one kernel (pcgtile.cu)
     if(tiles.ctas())
-    {
-      const SolveTimer timer(s);
-      k_pcg_init<T><<<vec_blocks(n), VB, 0, s>>>(n, b, x, r.p, p.p, invdiag, red, st.p, tol, maxit);
-      ICB_CUDA(cudaGetLastError());
-      count_launch();
-      launch_pcg_tiles(tiles, d, K, E, invdiag, x, r.p, p.p, q.p, st.p, s);
-      ICB_CUDA(cudaMemcpyAsync(hst, st.p, sizeof(KState), cudaMemcpyDeviceToHost, s));
-      return report(timer, info);
-    }
+      return solveTiles(
+          [&] { launch_pcg_tiles(tiles, d, K, E, invdiag, x, r.p, p.p, q.p, st.p, s); }, invdiag,
+          b, x, tol, maxit, s, info);
   }
   const Dims dd = d;
   RedScratch *rp = &red;
@@ -342,6 +336,19 @@ int JacobiPcg<T>::solve(const T *K, const T *E, const uint8_t *fix, const T *inv
     launch_matvec<T>(dd, K, E, pp, qp, fix, cs, rp, dp, sp);
   };
   return solveOp(op, K, E, fix, invdiag, b, x, tol, maxit, s, info);
+}
+
+template <typename T>
+int JacobiPcg<T>::solveTiles(const std::function<void()> &iterate, const T *invdiag, const T *b,
+                             T *x, double tol, int maxit, cudaStream_t s, icb_solve_info *info)
+{
+  const SolveTimer timer(s);
+  k_pcg_init<T><<<vec_blocks(n), VB, 0, s>>>(n, b, x, r.p, p.p, invdiag, red, st.p, tol, maxit);
+  ICB_CUDA(cudaGetLastError());
+  count_launch();
+  iterate();
+  ICB_CUDA(cudaMemcpyAsync(hst, st.p, sizeof(KState), cudaMemcpyDeviceToHost, s));
+  return report(timer, info);
 }
 
 template <typename T>

@@ -29,7 +29,7 @@ template <typename T> struct JacobiPcg
   KState *hst = nullptr; ///< pinned mirror
   WhileGraph loop; ///< host form: 16 iterations per launch
   GraphKey graphKey; ///< what `loop` bakes in besides this object's own buffers
-  PcgTiles tiles;    ///< the one-kernel form of solve(), when the grid is small enough
+  PcgTiles tiles;    ///< the one-kernel form's cut, when the grid is small enough
 
   JacobiPcg(const Dims &dims, cudaStream_t s);
   ~JacobiPcg();
@@ -43,6 +43,10 @@ template <typename T> struct JacobiPcg
   int solveOp(const std::function<void(cudaStream_t)> &op, const void *opKey0,
               const void *opKey1, const void *opKey2, const T *invdiag, const T *b, T *x,
               double tol, int maxit, cudaStream_t s, icb_solve_info *info);
+  /// the same with all iterations as one kernel, which iterate() launches on
+  /// this object's r, p, q and st (pcgtile.cu)
+  int solveTiles(const std::function<void()> &iterate, const T *invdiag, const T *b, T *x,
+                 double tol, int maxit, cudaStream_t s, icb_solve_info *info);
   /// wait for the solve and hand out what it left in hst
   int report(const SolveTimer &timer, icb_solve_info *info);
 };

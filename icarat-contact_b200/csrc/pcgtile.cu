@@ -20,6 +20,12 @@
 // against one: 120 x 40 (9,920 unknowns) 14.9 and 4.7 us, 60 x 20 x 20 (79,380) 17.9
 // and 7.7, 540 x 540 (585,360) 33.0 and 10.1, 48 x 46 x 45 (318,000) 26.5 and 16.4.
 //
+// The 3D Helmholtz filter's solves (12 iterations or so) take the same form with a
+// scalar a node and its separable stencil: a filter call at R = 2.2, host arrays in
+// and out, takes 201 us instead of 363 on 40 x 20 x 20 elements, 518 instead of 699
+// on 80 x 40 x 40 and 1,113 instead of 1,301 on 128 x 64 x 64, about the largest grid
+// whose vectors fit; an MMA run on 80 x 40 x 40 17.2 -> 15.0 ms.
+//
 // The launch is cooperative (every CTA is resident), and every poll is bounded:
 // a CTA whose poll runs out marks the solve ICB_ERR_TIMEOUT and returns, and so
 // do the others when theirs run out.
@@ -40,7 +46,9 @@ namespace
 /// below the node and one for the four above
 template <int DIM> constexpr int kThreads = DIM == 3 ? 384 : 256;
 template <int DIM> constexpr int kNodeThreads = DIM == 3 ? 192 : 256;
-constexpr int kTileSmem = 200 << 10;
+/// of the scalar form: one a node, as many as an exchange takes
+constexpr int kScalarThreads = 512;
+constexpr int kTileSmem = 200 << 10, kScalarSmem = 226 << 10;
 
 template <int DIM> struct ElemK;
 template <> struct ElemK<2>
@@ -160,14 +168,68 @@ __device__ __forceinline__ void node_product3(const ElemK<3> &K, const double *p
   }
 }
 
-template <int DIM>
-__global__ void __launch_bounds__(kThreads<DIM>)
-    k_pcg_tiles(const __grid_constant__ ElemK<DIM> K, const Dims d, const PcgTiles T,
+/// the Helmholtz operator at padded entry c0 of the box: the separable sums of
+/// k_helm_apply3 in its order (the same bits).  `at`: an own node's sown entry,
+/// whose flags say where the grid ends beside it
+constexpr int kAtBits = 16;       ///< of a sown entry: the padded entry
+constexpr int kAtLow = 1 << 16;   ///< no node at -1 on axis a: kAtLow << 2 a
+constexpr int kAtHigh = 2 << 16;  ///< none at +1: kAtHigh << 2 a
+constexpr int kAtFace = 1 << 22;  ///< a neighbour CTA reads the node
+__device__ __forceinline__ double node_helm(const HelmTensor &C, const double *p, const Box<3> &B,
+                                            int at)
+{
+  const int c0 = at & ((1 << kAtBits) - 1);
+  double md[3], sd[3];
+#pragma unroll
+  for(int a = 0; a < 3; a++)
+  {
+    const bool lo = !(at & (kAtLow << 2 * a)), hi = !(at & (kAtHigh << 2 * a));
+    md[a] = (lo ? C.a[a].mh : 0.0) + (hi ? C.a[a].mh : 0.0);
+    sd[a] = (lo ? C.a[a].sh : 0.0) + (hi ? C.a[a].sh : 0.0);
+  }
+  const HelmAxis &ax = C.a[0], &ay = C.a[1], &az = C.a[2];
+  double G[3], H[3];
+#pragma unroll
+  for(int k = 0; k < 3; k++)
+  {
+    double mx[3], sx[3];
+#pragma unroll
+    for(int r = 0; r < 3; r++)
+    {
+      const double *q = p + c0 + (r - 1) * B.W + (k - 1) * B.WH;
+      const double c = q[0], e = q[-1] + q[1];
+      mx[r] = fma(md[0], c, ax.mo * e);
+      sx[r] = fma(sd[0], c, ax.so * e);
+    }
+    G[k] = fma(md[1], mx[1], ay.mo * (mx[0] + mx[2]));
+    H[k] = G[k] + C.re2 * (fma(md[1], sx[1], ay.mo * (sx[0] + sx[2])) +
+                           fma(sd[1], mx[1], ay.so * (mx[0] + mx[2])));
+  }
+  return fma(md[2], H[1], az.mo * (H[0] + H[2])) + C.re2 * fma(sd[2], G[1], az.so * (G[0] + G[2]));
+}
+
+/// what the kernel is given as its operator and threads: NC = DIM the elastic
+/// one, NC = 1 the 3D Helmholtz filter's
+template <int DIM, int NC> struct TileOp
+{
+  using K = ElemK<DIM>;
+  static constexpr int NT = kThreads<DIM>, kSmem = kTileSmem;
+};
+template <> struct TileOp<3, 1>
+{
+  using K = HelmTensor;
+  static constexpr int NT = kScalarThreads, kSmem = kScalarSmem;
+};
+
+template <int DIM, int NC>
+__global__ void __launch_bounds__(TileOp<DIM, NC>::NT)
+    k_pcg_tiles(const __grid_constant__ typename TileOp<DIM, NC>::K K, const Dims d, const PcgTiles T,
                 const double *__restrict__ E, const double *__restrict__ dinv,
                 double *__restrict__ x, double *__restrict__ r, double *p0, double *z, double *slots,
                 KState *st)
 {
-  constexpr int NT = kThreads<DIM>;
+  constexpr int NT = TileOp<DIM, NC>::NT;
+  constexpr bool kElastic = NC == DIM;
   extern __shared__ __align__(16) double pcg_dyn[];
   __shared__ double sw[NT / 32][2], sres[3];
   __shared__ int nring;
@@ -187,10 +249,10 @@ __global__ void __launch_bounds__(kThreads<DIM>)
   B.WH = DIM == 3 ? B.W * (T.by + 2) : 0;
   B.pad = B.W * (T.by + 2) * (DIM == 3 ? T.bz + 2 : 1);
   const int cap = T.bx * T.by * T.bz;
-  double *sp = pcg_dyn, *sE = sp + DIM * B.pad, *sx = sE + B.pad, *sr = sx + DIM * cap,
-         *sd = sr + DIM * cap, *sq = sd + DIM * cap, *sz = sq + DIM * cap;
+  double *sp = pcg_dyn, *sE = sp + NC * B.pad, *sx = sE + (kElastic ? B.pad : 0),
+         *sr = sx + NC * cap, *sd = sr + NC * cap, *sq = sd + NC * cap, *sz = sq + NC * cap;
   // (padded entry, node) of the box's own nodes and of the ring's
-  int2 *sown = reinterpret_cast<int2 *>(sq + (DIM == 3 ? 2 : 1) * DIM * cap), *sring = sown + cap;
+  int2 *sown = reinterpret_cast<int2 *>(sq + (NC == 3 ? 2 : 1) * NC * cap), *sring = sown + cap;
   if(tid == 0)
     nring = 0;
   __syncthreads();
@@ -201,14 +263,15 @@ __global__ void __launch_bounds__(kThreads<DIM>)
     const int k = DIM == 3 ? row / (T.by + 2) - 1 : 0;
     const int j = row - (DIM == 3 ? (k + 1) * (T.by + 2) : 0) - 1;
     const int gx = B.x0 + i, gy = B.y0 + j, gz = B.z0 + k;
-    const bool elem = unsigned(gx) < unsigned(d.nx) && unsigned(gy) < unsigned(d.ny) &&
+    [[maybe_unused]] const bool elem = unsigned(gx) < unsigned(d.nx) && unsigned(gy) < unsigned(d.ny) &&
                       (DIM == 2 || unsigned(gz) < unsigned(d.nz));
-    sE[t] = elem ? E[gx + (long long)d.nx * (gy + (long long)d.ny * gz)] : 0.0;
+    if constexpr(kElastic)
+      sE[t] = elem ? E[gx + (long long)d.nx * (gy + (long long)d.ny * gz)] : 0.0;
     const bool node = unsigned(gx) < unsigned(d.sx) && unsigned(gy) < unsigned(d.sy) &&
                       unsigned(gz) < unsigned(d.sz);
     const int g = gx + d.sx * (gy + d.sy * gz);
 #pragma unroll
-    for(int c = 0; c < DIM; c++)
+    for(int c = 0; c < NC; c++)
       sp[c * B.pad + t] = node ? __ldcg(p0 + c * d.ld + g) : 0.0;
     if(node && !(unsigned(i) < unsigned(B.nx) && unsigned(j) < unsigned(B.ny) &&
                  unsigned(k) < unsigned(B.nz)))
@@ -218,9 +281,23 @@ __global__ void __launch_bounds__(kThreads<DIM>)
   {
     const int row = n / B.nx, i = n - row * B.nx, k = row / B.ny, j = row - k * B.ny;
     const int g = B.x0 + i + d.sx * (B.y0 + j + d.sy * (B.z0 + k));
-    sown[n] = make_int2(B.at(i, j, k), g);
+    int at = B.at(i, j, k);
+    if constexpr(!kElastic)
+    {
+      const int l[3] = {i, j, k}, lo[3] = {B.x0, B.y0, B.z0}, nb[3] = {B.nx, B.ny, B.nz},
+                last[3] = {d.sx - 1, d.sy - 1, d.sz - 1};
 #pragma unroll
-    for(int c = 0; c < DIM; c++)
+      for(int a = 0; a < 3; a++)
+      {
+        const int ga = lo[a] + l[a];
+        at |= ga == 0 ? kAtLow << 2 * a : 0;
+        at |= ga == last[a] ? kAtHigh << 2 * a : 0;
+        at |= (l[a] == 0 && ga > 0) || (l[a] == nb[a] - 1 && ga < last[a]) ? kAtFace : 0;
+      }
+    }
+    sown[n] = make_int2(at, g);
+#pragma unroll
+    for(int c = 0; c < NC; c++)
     {
       sx[c * cap + n] = 0.0;
       sr[c * cap + n] = r[c * d.ld + g];
@@ -244,7 +321,7 @@ __global__ void __launch_bounds__(kThreads<DIM>)
     double *zcur = it & 1 ? p0 : z, *zold = it & 1 ? z : p0;
     // q = K p and p.q on the box (constrained rows of q are 0)
     double v[1] = {0.0};
-    if constexpr(DIM == 3)
+    if constexpr(NC == 3)
     {
       double q[3];
       constexpr int NN = kNodeThreads<3>;
@@ -268,14 +345,16 @@ __global__ void __launch_bounds__(kThreads<DIM>)
     }
     for(int n = tid; n < B.own; n += NT)
     {
-      const int c0 = sown[n].x;
-      double q[DIM];
-      if constexpr(DIM == 2)
+      const int at = sown[n].x, c0 = kElastic ? at : at & ((1 << kAtBits) - 1);
+      double q[NC];
+      if constexpr(!kElastic)
+        q[0] = node_helm(K, sp, B, at);
+      else if constexpr(DIM == 2)
         node_product2(K, sp, sE, B, c0, q);
 #pragma unroll
-      for(int c = 0; c < DIM; c++)
+      for(int c = 0; c < NC; c++)
       {
-        if constexpr(DIM == 3)
+        if constexpr(NC == 3)
           q[c] = sz[c * cap + n] + sq[c * cap + n];
         if(sd[c * cap + n] == 0.0)
           q[c] = 0.0;
@@ -303,13 +382,17 @@ __global__ void __launch_bounds__(kThreads<DIM>)
     {
       const int g = sown[n].y;
 #pragma unroll
-      for(int c = 0; c < DIM; c++)
+      for(int c = 0; c < NC; c++)
       {
         const double ri = sr[c * cap + n] - alpha * sq[c * cap + n];
         sr[c * cap + n] = ri;
         const double zi = sd[c * cap + n] * ri;
-        slot_put(zcur + c * d.ld + g, zi);
-        slot_store(zold + c * d.ld + g, kExEmpty);
+        // an elastic box is small: nearly all its nodes are on its faces
+        if(kElastic || (sown[n].x & kAtFace))
+        {
+          slot_put(zcur + c * d.ld + g, zi);
+          slot_store(zold + c * d.ld + g, kExEmpty);
+        }
         w[0] += ri * ri;
         w[1] += ri * zi;
       }
@@ -335,9 +418,9 @@ __global__ void __launch_bounds__(kThreads<DIM>)
     // x += alpha p; p = z + beta p on the box, then on the ring
     for(int n = tid; n < B.own; n += NT)
     {
-      const int c0 = sown[n].x;
+      const int c0 = kElastic ? sown[n].x : sown[n].x & ((1 << kAtBits) - 1);
 #pragma unroll
-      for(int c = 0; c < DIM; c++)
+      for(int c = 0; c < NC; c++)
       {
         const double pi = sp[c * B.pad + c0];
         sx[c * cap + n] += alpha * pi;
@@ -356,16 +439,16 @@ __global__ void __launch_bounds__(kThreads<DIM>)
     for(int t = tid; t < nring; t += NT)
     {
       const int2 e = sring[t];
-      unsigned long long b[DIM];
+      unsigned long long b[NC];
       bool more = true;
 #pragma unroll
-      for(int c = 0; c < DIM; c++)
+      for(int c = 0; c < NC; c++)
         b[c] = kExEmpty;
       for(unsigned n = 0; n < kExPolls && more; n++)
       {
         more = false;
 #pragma unroll
-        for(int c = 0; c < DIM; c++)
+        for(int c = 0; c < NC; c++)
           if(b[c] == kExEmpty)
           {
             b[c] = slot_read(zcur + c * d.ld + e.y);
@@ -374,7 +457,7 @@ __global__ void __launch_bounds__(kThreads<DIM>)
       }
       late |= more;
 #pragma unroll
-      for(int c = 0; c < DIM; c++)
+      for(int c = 0; c < NC; c++)
         sp[c * B.pad + e.x] =
             __longlong_as_double((long long)b[c]) + beta * sp[c * B.pad + e.x];
     }
@@ -388,7 +471,7 @@ __global__ void __launch_bounds__(kThreads<DIM>)
   {
     const int g = sown[n].y;
 #pragma unroll
-    for(int c = 0; c < DIM; c++)
+    for(int c = 0; c < NC; c++)
     {
       x[c * d.ld + g] = sx[c * cap + n];
       r[c * d.ld + g] = sr[c * cap + n];
@@ -421,16 +504,23 @@ PcgTiles pcg_tiles(const Dims &d)
 {
   PcgTiles best;
   long long bestCost = LLONG_MAX;
+  // dim 1: a scalar on the nodes of a grid (the Helmholtz filter's; 3D only, and
+  // a box takes what shared memory holds)
+  const bool scalar = d.dim == 1, solid = scalar ? d.sz > 1 : d.dim == 3;
+  if(scalar && !solid)
+    return best;
   const int G = num_sms(), nc = d.dim;
   // nodes a CTA takes at most: six (3D) or eight (2D) a thread; its shared memory
   // ends near there, and 3D is still 1.6 times the three kernels' speed
-  const long long most = d.dim == 3 ? 6 * kNodeThreads<3> : 8 * kNodeThreads<2>;
+  const long long most = scalar       ? LLONG_MAX
+                         : d.dim == 3 ? 6 * kNodeThreads<3>
+                                      : 8 * kNodeThreads<2>;
   if(G > kExCtas || d.nnode >= (1LL << 30))
     return best;
   for(int px = 1; px <= std::min(G, d.sx); px++)
     for(int py = 1; px * py <= G && py <= d.sy; py++)
     {
-      const int pzMost = d.dim == 3 ? std::min(G / (px * py), d.sz) : 1;
+      const int pzMost = solid ? std::min(G / (px * py), d.sz) : 1;
       for(int pz = 1; pz <= pzMost; pz++)
       {
         PcgTiles t;
@@ -442,13 +532,13 @@ PcgTiles pcg_tiles(const Dims &d)
         if(own > most)
           continue;
         const long long pad =
-            (long long)(t.bx + 2) * (t.by + 2) * (d.dim == 3 ? t.bz + 2 : 1);
-        const long long bytes = 8 * (pad * (nc + 1) + (d.dim == 3 ? 5 : 4) * nc * own) + 8 * pad;
-        if(bytes > kTileSmem)
+            (long long)(t.bx + 2) * (t.by + 2) * (solid ? t.bz + 2 : 1);
+        const long long bytes = 8 * (pad * (scalar ? 1 : nc + 1) + (d.dim == 3 ? 5 : 4) * nc * own) + 8 * pad;
+        if(bytes > (scalar ? kScalarSmem : kTileSmem))
           continue;
         // cycles of an iteration that depend on the cut: the element work, the
         // ring, and the polls of two exchanges (measured slopes)
-        const long long cost = own * (d.dim == 3 ? 20 : 4) + (pad - own) * 3 + t.ctas() * 12;
+        const long long cost = own * (d.dim == 3 ? 20 : scalar ? 3 : 4) + (pad - own) * 3 + t.ctas() * 12;
         if(cost < bestCost)
         {
           bestCost = cost;
@@ -460,24 +550,23 @@ PcgTiles pcg_tiles(const Dims &d)
   return best;
 }
 
-template <int DIM>
-static void run_tiles(const PcgTiles &t, const Dims &d, const ElemK<DIM> &K, const double *E,
-                      const double *invdiag, double *x, double *r, double *p, double *z,
-                      KState *st, cudaStream_t s)
+template <int DIM, int NC>
+static void run_tiles(const PcgTiles &t, const Dims &d, typename TileOp<DIM, NC>::K K,
+                      const double *E, const double *invdiag, double *x, double *r, double *p,
+                      double *z, KState *st, cudaStream_t s)
 {
-  const size_t nsoa = size_t(DIM) * size_t(d.ld);
+  const size_t nsoa = size_t(NC) * size_t(d.ld);
   // the shared-memory opt-in is a per-device attribute shared by every host
   // thread: always its largest value
-  ICB_CUDA(cudaFuncSetAttribute(k_pcg_tiles<DIM>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                kTileSmem));
+  ICB_CUDA(cudaFuncSetAttribute(k_pcg_tiles<DIM, NC>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                TileOp<DIM, NC>::kSmem));
   double *slots = z + nsoa; // a multiple of 64 doubles past z: line-aligned
   ICB_CUDA(cudaMemsetAsync(z, 0xff, sizeof(double) * (nsoa + pcg_tile_slots(t)), s)); // kExEmpty
   Dims dd = d;
   PcgTiles tt = t;
-  ElemK<DIM> kk = K;
-  void *args[] = {&kk, &dd, &tt, &E, &invdiag, &x, &r, &p, &z, &slots, &st};
-  ICB_CUDA(cudaLaunchCooperativeKernel((const void *)k_pcg_tiles<DIM>, dim3(t.ctas()),
-                                       dim3(kThreads<DIM>), args, size_t(t.smem), s));
+  void *args[] = {&K, &dd, &tt, &E, &invdiag, &x, &r, &p, &z, &slots, &st};
+  ICB_CUDA(cudaLaunchCooperativeKernel((const void *)k_pcg_tiles<DIM, NC>, dim3(t.ctas()),
+                                       dim3(TileOp<DIM, NC>::NT), args, size_t(t.smem), s));
   count_launch();
 }
 
@@ -489,7 +578,7 @@ void launch_pcg_tiles(const PcgTiles &t, const Dims &d, const double *K, const d
   {
     ElemK<2> k;
     std::copy(K, K + 64, k.k);
-    run_tiles<2>(t, d, k, E, invdiag, x, r, p, z, st, s);
+    run_tiles<2, 2>(t, d, k, E, invdiag, x, r, p, z, st, s);
   }
   else
   {
@@ -497,7 +586,14 @@ void launch_pcg_tiles(const PcgTiles &t, const Dims &d, const double *K, const d
     for(int i = 0, m = 0; i < 24; i++)
       for(int j = i; j < 24; j++)
         k.k[m++] = K[i * 24 + j];
-    run_tiles<3>(t, d, k, E, invdiag, x, r, p, z, st, s);
+    run_tiles<3, 3>(t, d, k, E, invdiag, x, r, p, z, st, s);
   }
+}
+
+void launch_pcg_tiles(const PcgTiles &t, const Dims &d, const HelmTensor &C,
+                      const double *invdiag, double *x, double *r, double *p, double *z,
+                      KState *st, cudaStream_t s)
+{
+  run_tiles<3, 1>(t, d, C, nullptr, invdiag, x, r, p, z, st, s);
 }
 } // namespace icb
