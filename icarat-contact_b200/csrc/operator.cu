@@ -299,11 +299,10 @@ __device__ __forceinline__ void row_get(const double (&p)[4], double (&v)[3])
   v[0] = a.x, v[1] = a.y, v[2] = p[2];
 }
 
-/// dynamic shared memory of k_matvec_h8m: the carry, and for FP64 with two CTAs
-/// an SM the bottom plane's modes (12 values per thread each)
-template <typename T, int TYK, int MINB> constexpr int h8m_smem_bytes()
+/// dynamic shared memory of k_matvec_h8m: the carry, 12 values per thread
+template <typename T, int TYK> constexpr int h8m_smem_bytes()
 {
-  return int(sizeof(T)) * 12 * TYK * TX * (sizeof(T) == 8 && MINB > 1 ? 2 : 1);
+  return int(sizeof(T)) * 12 * TYK * TX;
 }
 /// whether a grid's vectors can be addressed by 32-bit byte offsets per component
 template <typename T> inline bool h8m_offsets_fit(const Dims &d)
@@ -338,16 +337,12 @@ __global__ void __launch_bounds__(TX *TYK, MINB)
 {
   if(gate && (gate->stop || (gateConv && gate->conv)))
     return;
-  // FP64 with two CTAs an SM (the fused dot): the registers end at 128, so the
-  // bottom plane's modes live in shared memory too and the loads wait until the
-  // element product's registers are free
-  constexpr bool kTight = sizeof(T) == 8 && MINB > 1;
   using V = typename Vec16<T>::V;
   constexpr int PER = Vec16<T>::PER, NT = TX * TYK;
   extern __shared__ __align__(16) unsigned char h8m_dyn[];
   const int lx = threadIdx.x, ly = threadIdx.y;
   // component c's modes: vectors (c PER + 0 .. PER - 1) NT + thread
-  V *sC = reinterpret_cast<V *>(h8m_dyn) + ly * TX + lx, *sH = sC + 3 * PER * NT;
+  V *sC = reinterpret_cast<V *>(h8m_dyn) + ly * TX + lx;
   // the row below's corner sums: three values a thread
   __shared__ __align__(16) T sB[2][TYK][TX][4];
   const int X0 = blockIdx.x * (TX - 1), Y0 = blockIdx.y * (TYK - 1);
@@ -391,8 +386,6 @@ __global__ void __launch_bounds__(TX *TYK, MINB)
       plane_modes(v[c], bh[c]);
       const T zero[4] = {T(0), T(0), T(0), T(0)};
       Vec16<T>::put(sC + c * PER * NT, NT, zero);
-      if(kTight)
-        Vec16<T>::put(sH + c * PER * NT, NT, bh[c]);
     }
   }
   if(Z0 > 0)
@@ -413,50 +406,37 @@ __global__ void __launch_bounds__(TX *TYK, MINB)
       plane_modes(nxt[c], th[c]);
     const T Ee = Enxt;
     // next layer's inputs
-    auto load_next = [&]() {
-      if(ek + 2 <= d.nz)
-        o0 += sxy;
-      load_plane(nxt);
-      if(ek >= 0)
-        eo += exy;
-      Enxt = load_E(ek + 1);
-    };
-    if(!kTight)
-      load_next();
+    if(ek + 2 <= d.nz)
+      o0 += sxy;
+    load_plane(nxt);
+    if(ek >= 0)
+      eo += exy;
+    Enxt = load_E(ek + 1);
     const bool out = ek >= Z0;
     const bool own = out && ownCol;
     unsigned f = 0;
     EpiIn<T> in;
-    auto load_in = [&]() {
-      if(own)
-      {
-        f = __ldg(fix + node / unsigned(sizeof(T)));
+    if(own)
+    {
+      f = __ldg(fix + node / unsigned(sizeof(T)));
 #pragma unroll
-        for(int c = 0; c < 3; c++)
-        {
-          if(DOT || MODE >= OP_JACOBI)
-            in.us[c] = __ldg(at_byte(u + c * ld, node));
-          if(MODE != OP_APPLY)
-            in.b[c] = __ldg(at_byte(ep.b + c * ld, node));
-          if(MODE >= OP_JACOBI)
-            in.dinv[c] = __ldg(at_byte(ep.dinv + c * ld, node));
-          if(MODE == OP_CHEB)
-            in.d[c] = ep.c1 != T(0) && !ep.prev0 ? *at_byte(y + c * ld, node) : T(0); // the previous iterate
-        }
+      for(int c = 0; c < 3; c++)
+      {
+        if(DOT || MODE >= OP_JACOBI)
+          in.us[c] = __ldg(at_byte(u + c * ld, node));
+        if(MODE != OP_APPLY)
+          in.b[c] = __ldg(at_byte(ep.b + c * ld, node));
+        if(MODE >= OP_JACOBI)
+          in.dinv[c] = __ldg(at_byte(ep.dinv + c * ld, node));
+        if(MODE == OP_CHEB)
+          in.d[c] = ep.c1 != T(0) && !ep.prev0 ? *at_byte(y + c * ld, node) : T(0); // the previous iterate
       }
-    };
-    if(!kTight)
-      load_in();
+    }
     // element modes: z butterfly of the two planes' x-y modes
     T uh[24], yh[24];
 #pragma unroll
     for(int c = 0; c < 3; c++)
     {
-      if(kTight)
-      {
-        Vec16<T>::get(sH + c * PER * NT, NT, bh[c]);
-        Vec16<T>::put(sH + c * PER * NT, NT, th[c]);
-      }
 #pragma unroll
       for(int s = 0; s < 4; s++)
       {
@@ -466,8 +446,6 @@ __global__ void __launch_bounds__(TX *TYK, MINB)
     }
     yh[0] = yh[1] = yh[2] = T(0); // rigid translations
     modal_blocks_apply<0, 0>(K, uh, yh);
-    if(kTight)
-      load_next();
     // inverse z butterfly: bottom face completes plane ek, top face is carried
     T acc[3][4];
 #pragma unroll
@@ -484,14 +462,11 @@ __global__ void __launch_bounds__(TX *TYK, MINB)
       Vec16<T>::put(sC + c * PER * NT, NT, carry);
       plane_corners(hb, acc[c]);
     }
-    if(!kTight)
 #pragma unroll
-      for(int c = 0; c < 3; c++)
+    for(int c = 0; c < 3; c++)
 #pragma unroll
-        for(int q = 0; q < 4; q++)
-          bh[c][q] = th[c][q];
-    if(kTight)
-      load_in();
+      for(int q = 0; q < 4; q++)
+        bh[c][q] = th[c][q];
     if(out)
     {
       T A[3], S[3];
@@ -1535,13 +1510,11 @@ static void launch_op_mode(const Dims &d, const T *K, const T *E, const T *u, T 
   Epi<T> ep{x.b, x.dinv, T(x.omega), T(x.c1), T(x.c2), x.prev0};
   if(d.dim == 3)
   {
-    // element rows per tile: 8; 12 for the FP64 product and residual without a
-    // dot, whose registers (168) still fit 384 threads without spills: 12 warps
-    // an SM and a smaller halo (y = K u at 384x128x128 183 us, with 8 rows 198,
-    // with 8 rows and the fused dot's form 211; the Chebyshev step spills at 12
-    // rows, 288 against 285 us).  12 rows for FP32 measured 89.6 against 88.2 us.
-    // The dot keeps 8 rows: its sum is cut by tiles, and a mixed solve follows
-    // every bit of it
+    // element rows per tile: 8; 12 for the FP64 product (with and without the
+    // dot) and residual in corner-mode form, whose registers (168) still fit 384
+    // threads without spills: 12 warps an SM and a smaller halo (y = K u at
+    // 384x128x128 183 us, with 8 rows 198; the Chebyshev step spills at 12 rows, 288
+    // against 285 us).  12 rows for FP32 measured 89.6 against 88.2 us.
     constexpr int TYK0 = TY3;
     constexpr int TYK1 = sizeof(T) == 8 && MODE <= OP_RESIDUAL ? TY3 + 4 : TY3;
     const int bx = (d.sx + TX - 2) / (TX - 1);
@@ -1580,15 +1553,13 @@ static void launch_op_mode(const Dims &d, const T *K, const T *E, const T *u, T 
     }
     if(g_hex8_modal && h8m_offsets_fit<T>(d) && modal_form_cached(K, kmod))
     {
-      // 3 (FP32) CTAs of 256 threads per SM; FP64 two with the fused dot and one
-      // without, whose registers let the next plane's loads go out a whole layer
-      // ahead and keep the bottom plane's modes (only the carry in shared memory)
-      constexpr int MB = sizeof(T) == 8 ? 2 : 3, MBnodot = sizeof(T) == 8 ? 1 : 3;
-      if(x.dotRed)
-        run(k_matvec_h8m<T, TYK0, true, MODE, MB>, kmod, h8m_smem_bytes<T, TYK0, MB>(), TYK0);
-      else
-        run(k_matvec_h8m<T, TYK1, false, MODE, MBnodot>, kmod,
-            h8m_smem_bytes<T, TYK1, MBnodot>(), TYK1);
+      // 3 (FP32) CTAs of 256 threads per SM; FP64 one, whose registers let the next
+      // plane's loads go out a whole layer ahead and keep the bottom plane's modes.
+      // (The fused dot at two CTAs of 8 rows under 128 registers, modes in shared
+      // memory and the loads after the product, took 211 us at 384x128x128, DOTUS now.)
+      constexpr int MB = sizeof(T) == 8 ? 1 : 3;
+      run(x.dotRed ? k_matvec_h8m<T, TYK1, true, MODE, MB> : k_matvec_h8m<T, TYK1, false, MODE, MB>,
+          kmod, h8m_smem_bytes<T, TYK1>(), TYK1);
     }
     else if constexpr(std::is_same<T, double>::value)
     {
