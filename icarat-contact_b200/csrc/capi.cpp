@@ -613,6 +613,11 @@ int icb_set_option(const char *name, long long value)
     need(value >= 0 && value <= 0x7fffffffLL, "tc_spin_limit must be in [0, 2^31)");
     set_tc_spin_limit(unsigned(value));
   }
+  else if(n == "exchange_spin_limit")
+  {
+    need(value >= 0 && value <= 0x7fffffffLL, "exchange_spin_limit must be in [0, 2^31)");
+    set_exchange_spin_limit(unsigned(value));
+  }
   else
     need(false, "unknown option");
   ICB_API_END
@@ -649,6 +654,8 @@ long long icb_get_option(const char *name)
     return (long long)tc_timeouts();
   if(n == "tc_spin_limit")
     return (long long)tc_spin_limit();
+  if(n == "exchange_spin_limit")
+    return (long long)exchange_spin_limit();
   return -1;
 }
 

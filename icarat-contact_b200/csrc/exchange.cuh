@@ -17,7 +17,9 @@ namespace icb
 /// with 32 bytes each and 1.6 us with a line each (1.1 us for 20 CTAs).
 constexpr int kExSlot = 16;
 constexpr int kExCtas = 256;           ///< CTAs of an exchange at most
-constexpr unsigned kExPolls = 1u << 22; ///< polls before a CTA gives up: about two seconds
+/// polls of a wait before a CTA gives up (about two seconds on a GPU that runs
+/// nothing else), unless the option exchange_spin_limit says otherwise
+constexpr unsigned kExPolls = 1u << 22;
 constexpr unsigned long long kExEmpty = ~0ull;
 
 #ifdef __CUDACC__
@@ -43,10 +45,11 @@ __device__ __forceinline__ unsigned long long slot_read(const double *s)
 /// - 1 of slot set `set`.  `clear` (may be NULL): the set to empty.  With it,
 /// a fence follows the CTA's own stores to the slots: whoever sees a later value
 /// of this CTA and fences too sees all its stores before this exchange.  False
-/// when a poll ran out (the same in all threads of the CTA).
+/// when a slot was still empty after `polls` polls (the same in all threads of
+/// the CTA).
 template <int NT, int NV>
 __device__ __forceinline__ bool exchange(double (&v)[NV], int first, double *set, double *clear,
-                                         double (*sw)[2], double *sres)
+                                         unsigned polls, double (*sw)[2], double *sres)
 {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int G = gridDim.x, cta = blockIdx.x;
@@ -89,7 +92,7 @@ __device__ __forceinline__ bool exchange(double (&v)[NV], int first, double *set
       for(int k = 0; k < NV; k++)
         b[q][k] = lane + 32 * q < G ? kExEmpty : 0ull;
     bool more = true;
-    for(unsigned n = 0; n < kExPolls && more; n++)
+    for(unsigned n = 0; n < polls && more; n++)
     {
       more = false;
 #pragma unroll

@@ -282,6 +282,10 @@ unsigned tc_timeouts();
 /// and returns (process-wide; default 2^22)
 unsigned tc_spin_limit();
 void set_tc_spin_limit(unsigned polls);
+/// polls of a wait between the CTAs of a cooperative kernel (exchange.cuh) before
+/// a CTA gives up (process-wide; default 2^22)
+unsigned exchange_spin_limit();
+void set_exchange_spin_limit(unsigned polls);
 /// whether FP32 Hex8 operator launches use the tensor-core kernel
 bool tc_operator_enabled();
 void set_tc_operator(bool on);

@@ -608,7 +608,8 @@ __global__ void __launch_bounds__(VB)
     k_oc_update(Dims d, ConeCols C, const double *__restrict__ aa, double *x,
                 const double *__restrict__ df, const double *__restrict__ dg,
                 const double *__restrict__ xmin, const double *__restrict__ xmax,
-                const double *__restrict__ vol, OcParams P, double g, double *slots, OcState *st)
+                const double *__restrict__ vol, OcParams P, double g, double *slots, const unsigned polls,
+                OcState *st)
 {
   extern __shared__ __align__(16) double oc_up_dyn[];
   __shared__ double sw[VB / 32][2], sres[3];
@@ -672,7 +673,7 @@ __global__ void __launch_bounds__(VB)
     // it is emptied now, this CTA's value of it + 1 comes after the fence, and
     // everyone reads that value, and fences, before it polls set it + 2
     if(!exchange<VB, 1>(v, 0, slots + (it % kOcUpSets) * kExSlot * G,
-                        slots + ((it + 2) % kOcUpSets) * kExSlot * G, sw, sres))
+                        slots + ((it + 2) % kOcUpSets) * kExSlot * G, polls, sw, sres))
     {
       dead = true;
       break;
@@ -703,11 +704,16 @@ __global__ void __launch_bounds__(VB)
           x[e] = oc_candidate(x[e], df[e], dg[e], S.lastLam, P.eta, P.move, xmin[e], xmax[e]);
         }
     }
-  if(threadIdx.x == 0 && (dead || blockIdx.x == 0))
+  // done is 0 until now: -1 once a CTA's wait ran out, which stays
+  if(threadIdx.x == 0 && dead)
+    atomicExch(&st->done, -1);
+  else if(threadIdx.x == 0 && blockIdx.x == 0)
   {
-    S.done = dead ? -1 : 1;
-    if(dead || st->done != -1)
-      *st = S;
+    st->counter = S.counter;
+    st->lam = S.lam;
+    st->lastLam = S.lastLam;
+    st->vol = S.vol;
+    atomicCAS(&st->done, 0, 1);
   }
 }
 
@@ -1275,7 +1281,8 @@ void OcUpdater::launch(const ConeFilter *cone, double *x, const double *df, cons
     const double *aa = cone->aa.p;
     OcParams Pu = P;
     OcState *sp = st.p;
-    void *args[] = {&dd, &cc, &aa, &x, &df, &dg, &xmin, &xmax, &vol, &Pu, &g, &slots, &sp};
+    unsigned polls = exchange_spin_limit();
+    void *args[] = {&dd, &cc, &aa, &x, &df, &dg, &xmin, &xmax, &vol, &Pu, &g, &slots, &polls, &sp};
     ICB_CUDA(cudaLaunchCooperativeKernel((const void *)k_oc_update, dim3(unsigned(ctas)), dim3(VB),
                                          args, size_t(upSmem), s));
     count_launch();

@@ -26,12 +26,14 @@
 // on 80 x 40 x 40 and 1,113 instead of 1,301 on 128 x 64 x 64, about the largest grid
 // whose vectors fit; an MMA run on 80 x 40 x 40 17.2 -> 15.0 ms.
 //
-// The launch is cooperative (every CTA is resident), and every poll is bounded:
-// a CTA whose poll runs out marks the solve ICB_ERR_TIMEOUT and returns, and so
-// do the others when theirs run out.
+// The launch is cooperative (every CTA is resident), and every wait is bounded (an
+// iteration's polls of the ring together): a CTA whose wait runs out marks the
+// solve ICB_ERR_TIMEOUT and returns, and so do the others when theirs run out.
+// The mark stays, whatever status CTA 0 ends with.
 #include "pcgtile.hpp"
 
 #include <algorithm>
+#include <atomic>
 #include <cfloat>
 #include <climits>
 
@@ -226,7 +228,7 @@ __global__ void __launch_bounds__(TileOp<DIM, NC>::NT)
     k_pcg_tiles(const __grid_constant__ typename TileOp<DIM, NC>::K K, const Dims d, const PcgTiles T,
                 const double *__restrict__ E, const double *__restrict__ dinv,
                 double *__restrict__ x, double *__restrict__ r, double *p0, double *z, double *slots,
-                KState *st)
+                const unsigned polls, KState *st)
 {
   constexpr int NT = TileOp<DIM, NC>::NT;
   constexpr bool kElastic = NC == DIM;
@@ -362,7 +364,7 @@ __global__ void __launch_bounds__(TileOp<DIM, NC>::NT)
         v[0] += sp[c * B.pad + c0] * q[c];
       }
     }
-    bool ok = exchange<NT, 1>(v, 0, set, nullptr, sw, sres);
+    bool ok = exchange<NT, 1>(v, 0, set, nullptr, polls, sw, sres);
     pq = v[0];
     if(!ok)
     {
@@ -397,7 +399,7 @@ __global__ void __launch_bounds__(TileOp<DIM, NC>::NT)
         w[1] += ri * zi;
       }
     }
-    ok = exchange<NT, 2>(w, 1, set, clear, sw, sres);
+    ok = exchange<NT, 2>(w, 1, set, clear, polls, sw, sres);
     if(!ok)
     {
       status = ICB_ERR_TIMEOUT;
@@ -436,7 +438,8 @@ __global__ void __launch_bounds__(TileOp<DIM, NC>::NT)
       break;
     }
     bool late = false;
-    for(int t = tid; t < nring; t += NT)
+    unsigned left = polls;
+    for(int t = tid; t < nring && !late; t += NT)
     {
       const int2 e = sring[t];
       unsigned long long b[NC];
@@ -444,7 +447,7 @@ __global__ void __launch_bounds__(TileOp<DIM, NC>::NT)
 #pragma unroll
       for(int c = 0; c < NC; c++)
         b[c] = kExEmpty;
-      for(unsigned n = 0; n < kExPolls && more; n++)
+      for(; left > 0 && more; left--)
       {
         more = false;
 #pragma unroll
@@ -455,7 +458,7 @@ __global__ void __launch_bounds__(TileOp<DIM, NC>::NT)
             more |= b[c] == kExEmpty;
           }
       }
-      late |= more;
+      late = more;
 #pragma unroll
       for(int c = 0; c < NC; c++)
         sp[c * B.pad + e.x] =
@@ -479,7 +482,7 @@ __global__ void __launch_bounds__(TileOp<DIM, NC>::NT)
   }
   if(tid == 0 && status == ICB_ERR_TIMEOUT)
   {
-    st->status = ICB_ERR_TIMEOUT;
+    atomicExch(&st->status, ICB_ERR_TIMEOUT);
     st->stop = 1;
   }
   else if(cta == 0 && tid == 0)
@@ -492,13 +495,17 @@ __global__ void __launch_bounds__(TileOp<DIM, NC>::NT)
     st->iter = iter;
     st->matvecs = matvecs;
     st->conv = conv;
-    // a CTA that timed out has set its own status
-    if(st->status != ICB_ERR_TIMEOUT)
-      st->status = status;
+    // ICB_OK until now, unless another CTA's wait ran out; one that runs out
+    // later stores over this
+    atomicCAS(&st->status, ICB_OK, status);
     st->stop = 1;
   }
 }
 } // namespace
+
+static std::atomic<unsigned> g_exchange_spin{kExPolls};
+unsigned exchange_spin_limit() { return g_exchange_spin.load(); }
+void set_exchange_spin_limit(unsigned polls) { g_exchange_spin = polls; }
 
 PcgTiles pcg_tiles(const Dims &d)
 {
@@ -564,7 +571,8 @@ static void run_tiles(const PcgTiles &t, const Dims &d, typename TileOp<DIM, NC>
   ICB_CUDA(cudaMemsetAsync(z, 0xff, sizeof(double) * (nsoa + pcg_tile_slots(t)), s)); // kExEmpty
   Dims dd = d;
   PcgTiles tt = t;
-  void *args[] = {&K, &dd, &tt, &E, &invdiag, &x, &r, &p, &z, &slots, &st};
+  unsigned polls = exchange_spin_limit();
+  void *args[] = {&K, &dd, &tt, &E, &invdiag, &x, &r, &p, &z, &slots, &polls, &st};
   ICB_CUDA(cudaLaunchCooperativeKernel((const void *)k_pcg_tiles<DIM, NC>, dim3(t.ctas()),
                                        dim3(TileOp<DIM, NC>::NT), args, size_t(t.smem), s));
   count_launch();
