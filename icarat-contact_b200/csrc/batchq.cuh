@@ -130,11 +130,14 @@ __device__ __forceinline__ void batch_queue(const Rec *__restrict__ D, const int
 /// barrier, one fence and one ticket, where a block at a time takes those after
 /// its few entries a thread -- a chain of latencies that bounded these kernels
 /// (32 designs of 6.1M DOFs, a block at a time and in runs: residual update 96
-/// and 66 us, r.z 49 and 35, x and p 76 and 50).
-template <int NV, int T, class Acc, class Fin>
+/// and 66 us, r.z 49 and 35, x and p 76 and 50).  HALVES: the warps' sums are added by
+/// halves and the blocks' by the first warp, as the one-kernel OC update does
+/// (oc_exchange).
+template <int NV, int T, bool HALVES = false, class Acc, class Fin>
 __device__ __forceinline__ void sum_runs(int b0, int n, unsigned gx, const RedScratch &red,
                                          const Acc &acc, const Fin &fin)
 {
+  static_assert(!HALVES || NV == 1, "one value a block");
   __shared__ double part[kMaxChunk][T / 32][NV], sw[32][NV];
   __shared__ int last;
   const int tid = threadIdx.x;
@@ -155,8 +158,11 @@ __device__ __forceinline__ void sum_runs(int b0, int n, unsigned gx, const RedSc
   if(tid < n * NV)
   {
     double s = 0.0;
-    for(int w = 0; w < T / 32; w++)
-      s += part[tid / NV][w][tid % NV];
+    if constexpr(HALVES)
+      s = sum_by_halves<T / 32>([&](int w) { return part[tid / NV][w][tid % NV]; });
+    else
+      for(int w = 0; w < T / 32; w++)
+        s += part[tid / NV][w][tid % NV];
     red.partials[(long long)b0 * NV + tid] = s;
     __threadfence();
   }
@@ -167,7 +173,10 @@ __device__ __forceinline__ void sum_runs(int b0, int n, unsigned gx, const RedSc
   if(!last)
     return;
   __threadfence();
-  partials_finish<NV>(sw, red, fin, int(gx));
+  if constexpr(HALVES)
+    partials_finish_warp<T / 32>(red, fin, int(gx));
+  else
+    partials_finish<NV>(sw, red, fin, int(gx));
 }
 
 /// CTAs of a persistent batched launch (the kernel's residency on every SM,

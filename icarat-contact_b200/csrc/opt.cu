@@ -540,8 +540,12 @@ __global__ void k_oc_final(long long n, double *__restrict__ x, const double *__
 /// The whole OC update of a 2D design as one cooperative kernel: a CTA takes
 /// every gridDim-th tile of 32 x 32 elements for all steps of the bisection.  A
 /// step was two launches inside a WHILE graph; here it is the tiles' work and one
-/// exchange between the CTAs.  An update (37 steps) takes 245 us less on 640 x 320
-/// elements and 105 us less on 120 x 40.
+/// exchange of their volumes between the CTAs.  An update (37 steps) takes 245 us
+/// less on 640 x 320 elements and 105 us less on 120 x 40.
+///
+/// Every tile's volume has a slot of its own, and every CTA adds them in the order of
+/// the batched step's sum (sum_runs): a batch and a run alone take the same turns
+/// even where the volume is within rounding of g.
 ///
 /// What a step needs of an element is staged once: h = (-df/dg)^eta x, so that the
 /// candidate at lambda is lambda^-eta h between its bounds, and the bounds.  A
@@ -589,6 +593,69 @@ __device__ __forceinline__ double oc_tile_volume(const double *buf, int W, const
   }
   return v;
 }
+/// The volume of all tiles, part[k][w] being warp w's share of tile blockIdx.x + k
+/// gridDim.x, summed in the order of the batched step (sum_runs with HALVES).  ok:
+/// false when a tile's volume did not come within `polls` polls (the same in all
+/// threads of the CTA).  set: a slot per tile; clear: the set to empty.  One warp
+/// polls: with a thread per tile in all eight a step took 0.9 us longer.
+__device__ __forceinline__ double oc_exchange(const double (*part)[VB / 32], int nt, int tiles,
+                                              double *set, double *clear, unsigned polls,
+                                              double *sres, bool &ok)
+{
+  const int lane = threadIdx.x & 31;
+  __syncthreads();
+  if(threadIdx.x < 32)
+  {
+    if(lane < nt)
+    {
+      const double s = sum_by_halves<VB / 32>([&](int w) { return part[lane][w]; });
+      const long long at = (long long)(blockIdx.x + lane * gridDim.x) * kExSlot;
+      slot_put(set + at, s);
+      slot_store(clear + at, kExEmpty);
+    }
+    fence_gpu();
+    constexpr int PER = VB / 32; // tiles of a lane in a round
+    double t[PER];
+#pragma unroll
+    for(int q = 0; q < PER; q++)
+      t[q] = 0.0;
+    bool late = false;
+    for(int t0 = 0; t0 < tiles; t0 += VB)
+    {
+      unsigned long long b[PER];
+#pragma unroll
+      for(int q = 0; q < PER; q++)
+        b[q] = t0 + lane + 32 * q < tiles ? kExEmpty : 0ull;
+      bool more = true;
+      for(unsigned n = 0; n < polls && more; n++)
+      {
+        more = false;
+#pragma unroll
+        for(int q = 0; q < PER; q++)
+          if(b[q] == kExEmpty)
+          {
+            b[q] = slot_read(set + (long long)(t0 + lane + 32 * q) * kExSlot);
+            more |= b[q] == kExEmpty;
+          }
+        more = __any_sync(0xffffffffu, more);
+      }
+      late |= more;
+#pragma unroll
+      for(int q = 0; q < PER; q++)
+        if(t0 + lane + 32 * q < tiles)
+          t[q] += __longlong_as_double((long long)b[q]);
+    }
+    const double s = warp_sum_d(sum_by_halves<PER>([&](int q) { return t[q]; }));
+    if(lane == 0)
+    {
+      sres[0] = s;
+      sres[1] = late ? 1.0 : 0.0;
+    }
+  }
+  __syncthreads();
+  ok = sres[1] == 0.0;
+  return sres[0];
+}
 /// weight sums and volumes of the thread's four elements (volume 0 outside)
 __device__ __forceinline__ void oc_tile_weights(const Dims &d, int i, int j0,
                                                 const double *__restrict__ aa,
@@ -612,7 +679,7 @@ __global__ void __launch_bounds__(VB)
                 OcState *st)
 {
   extern __shared__ __align__(16) double oc_up_dyn[];
-  __shared__ double sw[VB / 32][2], sres[3];
+  __shared__ double part[kOcUpTiles][VB / 32], sres[2];
   const int G = gridDim.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int ntx = (d.nx + kOcTW - 1) / kOcTW, tiles = ntx * ((d.ny + kOcTH - 1) / kOcTH);
   const int W = kOcTW + 2 * C.hx, cells = oc_up_cells(C);
@@ -654,7 +721,6 @@ __global__ void __launch_bounds__(VB)
   for(int it = 0; !S.done; it++)
   {
     const double c = 1.0 / oc_power(S.lam, P.eta);
-    double v[1] = {0.0};
     for(int k = 0; k < nt; k++)
     {
       const int t = blockIdx.x + k * G, x0 = t % ntx * kOcTW, y0 = t / ntx * kOcTH;
@@ -667,24 +733,31 @@ __global__ void __launch_bounds__(VB)
       for(int q = threadIdx.x; q < cells; q += VB)
         buf[q] = oc_bounded(h[q] * c, lo[q], hi[q]);
       __syncthreads();
-      v[0] += oc_tile_volume(buf, W, C, aav, volv, P, S.tanhTb);
+      const double s = warp_sum_d(oc_tile_volume(buf, W, C, aav, volv, P, S.tanhTb));
+      if(lane == 0)
+        part[k][warp] = s;
     }
     // set it + 2 was last polled at it - 2, by everyone before it arrived at it - 1:
-    // it is emptied now, this CTA's value of it + 1 comes after the fence, and
-    // everyone reads that value, and fences, before it polls set it + 2
-    if(!exchange<VB, 1>(v, 0, slots + (it % kOcUpSets) * kExSlot * G,
-                        slots + ((it + 2) % kOcUpSets) * kExSlot * G, polls, sw, sres))
+    // a tile's slot is emptied now, its value of it + 1 comes after the fence, and
+    // the lane that polls the slot reads that value, and fences, before it polls set
+    // it + 2
+    const long long setSize = (long long)tiles * kExSlot;
+    bool ok;
+    const double sum =
+        oc_exchange(part, nt, tiles, slots + (it % kOcUpSets) * setSize,
+                    slots + ((it + 2) % kOcUpSets) * setSize, polls, sres, ok);
+    if(!ok)
     {
       dead = true;
       break;
     }
     S.lastLam = S.lam;
-    if(v[0] - S.g > 0.0)
+    if(sum - S.g > 0.0)
       S.l0 = S.lam;
     else
       S.l1 = S.lam;
     S.counter++;
-    S.vol = v[0];
+    S.vol = sum;
     if(!((S.l1 - S.l0) / (S.l1 + S.l0) > S.lambdaeps && S.maxiter > S.counter))
       S.done = 1;
     else
@@ -1200,22 +1273,35 @@ OcTiling oc_tiling(const Dims &d, const ConeFilter *cone)
   t.blocks = int(t.ntx) * ((d.ny + kOcTH - 1) / kOcTH);
   return t;
 }
-/// CTAs of the one-kernel update on a grid: no more than there are tiles or SMs;
-/// 0 for 3D grids and those with too many tiles a CTA
-int oc_update_ctas(const Dims &d)
+/// tiles of the one-kernel update on a 2D grid; 0 for 3D grids and those with too many
+/// tiles a CTA
+int oc_update_tiles(const Dims &d)
 {
   if(d.dim != 2)
     return 0;
   const long long tiles =
       (long long)((d.nx + kOcTW - 1) / kOcTW) * ((d.ny + kOcTH - 1) / kOcTH);
-  const int G = std::min(num_sms(), kExCtas);
-  return tiles <= (long long)kOcUpTiles * G ? int(std::min<long long>(tiles, G)) : 0;
+  return tiles <= (long long)kOcUpTiles * std::min(num_sms(), kExCtas) ? int(tiles) : 0;
 }
-/// its shared memory: two buffers of candidates and three values a cell of its tiles
-int oc_update_smem(const Dims &d, const ConeCols &C, int ctas)
+/// the one-kernel update's CTAs (no more than tiles or SMs) and shared memory: two
+/// buffers of candidates and three values a cell of its tiles.  ctas 0: the update
+/// runs as a graph (3D, too many tiles, a stencil too large).  Batched updates
+/// take the column form where a run alone is this kernel, and only there, so that
+/// both form every volume by the same operations
+struct OcOneKernel
 {
-  const int tiles = ((d.nx + kOcTW - 1) / kOcTW) * ((d.ny + kOcTH - 1) / kOcTH);
-  return int(sizeof(double)) * oc_up_cells(C) * (2 + 3 * ((tiles + ctas - 1) / ctas));
+  int ctas = 0, smem = 0;
+};
+OcOneKernel oc_one_kernel(const Dims &d, const ConeFilter *cone)
+{
+  OcOneKernel r;
+  const int tiles = cone && cone->cols.ncol ? oc_update_tiles(d) : 0;
+  if(!tiles)
+    return r;
+  const int ctas = std::min(tiles, std::min(num_sms(), kExCtas));
+  r.smem = int(sizeof(double)) * oc_up_cells(cone->cols) * (2 + 3 * ((tiles + ctas - 1) / ctas));
+  r.ctas = r.smem <= kOcUpSmem ? ctas : 0;
+  return r;
 }
 } // namespace
 
@@ -1233,8 +1319,8 @@ OcUpdater::OcUpdater(const Dims &dims, cudaStream_t s) : d(dims)
   ICB_CUDA(cudaMemsetAsync(counter.p, 0, sizeof(unsigned), s));
   red = RedScratch{partials.p, counter.p, nb};
   // the candidates; or the one-kernel form's slots
-  const int ctas = oc_update_ctas(d);
-  cand.alloc(std::max<long long>(std::max<long long>(d.nel, 1), kOcUpSets * kExSlot * ctas));
+  cand.alloc(std::max<long long>(std::max<long long>(d.nel, 1),
+                                 (long long)kOcUpSets * kExSlot * oc_update_tiles(d)));
   ICB_CUDA(cudaMallocHost(&hst, sizeof(OcState)));
 }
 OcUpdater::~OcUpdater()
@@ -1266,15 +1352,14 @@ void OcUpdater::launch(const ConeFilter *cone, double *x, const double *df, cons
                        double g, const double *xmin, const double *xmax, const double *vol,
                        const OcParams &P, cudaStream_t s)
 {
-  const int ctas = cone && cone->cols.ncol ? oc_update_ctas(d) : 0;
-  const int upSmem = ctas ? oc_update_smem(d, cone->cols, ctas) : 0;
-  oneKernel = ctas && upSmem <= kOcUpSmem;
+  const OcOneKernel one = oc_one_kernel(d, cone);
+  oneKernel = one.ctas > 0;
   if(oneKernel)
   {
     ICB_CUDA(cudaFuncSetAttribute(k_oc_update, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   kOcUpSmem));
     double *slots = cand.p;
-    ICB_CUDA(cudaMemsetAsync(slots, 0xff, sizeof(double) * kOcUpSets * kExSlot * ctas, s));
+    ICB_CUDA(cudaMemsetAsync(slots, 0xff, sizeof(double) * kOcUpSets * kExSlot * size_t(oc_update_tiles(d)), s));
     ICB_CUDA(cudaMemsetAsync(st.p, 0, sizeof(OcState), s));
     Dims dd = d;
     ConeCols cc = cone->cols;
@@ -1283,8 +1368,8 @@ void OcUpdater::launch(const ConeFilter *cone, double *x, const double *df, cons
     OcState *sp = st.p;
     unsigned polls = exchange_spin_limit();
     void *args[] = {&dd, &cc, &aa, &x, &df, &dg, &xmin, &xmax, &vol, &Pu, &g, &slots, &polls, &sp};
-    ICB_CUDA(cudaLaunchCooperativeKernel((const void *)k_oc_update, dim3(unsigned(ctas)), dim3(VB),
-                                         args, size_t(upSmem), s));
+    ICB_CUDA(cudaLaunchCooperativeKernel((const void *)k_oc_update, dim3(unsigned(one.ctas)), dim3(VB),
+                                         args, size_t(one.smem), s));
     count_launch();
     ICB_CUDA(cudaMemcpyAsync(hst, st.p, sizeof(OcState), cudaMemcpyDeviceToHost, s));
     return;
@@ -1394,7 +1479,7 @@ __device__ __forceinline__ void oc_step_cols_b(const OcBatch::Rec &r, int b0, in
   const ConeCols &C = r.cols;
   const double c = 1.0 / oc_power(r.st->lam, r.P.eta), tb = r.st->tanhTb;
   const int W = kOcTW + 2 * C.hx, cells = oc_up_cells(C);
-  sum_runs<1, VB>(
+  sum_runs<1, VB, true>(
       b0, n, r.gx, r.red,
       [&](const Blk &B, double(&v)[1]) {
         const int x0 = int(B.x % r.ntx) * kOcTW, y0 = int(B.x / r.ntx) * kOcTH;
@@ -1523,7 +1608,7 @@ void OcBatch::build(const std::vector<OcBatchItem> &items, cudaStream_t s)
   std::vector<int2> ms, mc, mp, mf;
   smemStep = 0;
   size_t np = 0;
-  auto columns = [](const OcBatchItem &it) { return it.cone && it.cone->cols.ncol; };
+  auto columns = [](const OcBatchItem &it) { return oc_one_kernel(it.oc->d, it.cone).ctas > 0; };
   for(const OcBatchItem &it : items)
     np += columns(it) ? 3 * size_t(it.oc->d.nel) : 0;
   prep.alloc(std::max<size_t>(np, 1));
@@ -1542,7 +1627,7 @@ void OcBatch::build(const std::vector<OcBatchItem> &items, cudaStream_t s)
     r.ntx = tl.ntx;
     r.cols = ConeCols{};
     r.prep = nullptr;
-    if(tl.tiled && columns(it))
+    if(columns(it))
     {
       r.cols = it.cone->cols;
       r.prep = prep.p + np;

@@ -33,6 +33,22 @@ __device__ __forceinline__ double warp_sum_d(double v)
   return v;
 }
 
+/// w(0) .. w(NW - 1) added by halves: three additions deep for eight values instead of
+/// eight
+template <int NW, class W> __device__ __forceinline__ double sum_by_halves(const W &w)
+{
+  double v[NW];
+#pragma unroll
+  for(int q = 0; q < NW; q++)
+    v[q] = w(q);
+#pragma unroll
+  for(int o = NW / 2; o > 0; o >>= 1)
+#pragma unroll
+    for(int q = 0; q < o; q++)
+      v[q] += v[q + o];
+  return v[0];
+}
+
 /// the last block's part of a grid-wide sum: the nb blocks' partials in a fixed
 /// order (thread t takes t, t + blockDim, ...; then the warps in order), the
 /// total handed to fin, the counter ready for the next launch
@@ -72,6 +88,37 @@ __device__ __forceinline__ void partials_finish(double (&sw)[32][NV], const RedS
     }
     *red.counter = 0u;
     fin(tot);
+  }
+}
+
+/// the same by the first warp alone, one value a block: lane l takes block l + 32 q
+/// of every 32 N into sum q, adds the N sums by halves, then the lanes' are added
+template <int N, class Fin>
+__device__ __forceinline__ void partials_finish_warp(const RedScratch &red, const Fin &fin, int nb)
+{
+  const int lane = threadIdx.x;
+  if(lane >= 32)
+    return;
+  double t[N];
+#pragma unroll
+  for(int q = 0; q < N; q++)
+    t[q] = 0.0;
+  for(int t0 = 0; t0 < nb; t0 += 32 * N)
+  {
+    double v[N];
+#pragma unroll
+    for(int q = 0; q < N; q++)
+      v[q] = t0 + lane + 32 * q < nb ? __ldcg(red.partials + t0 + lane + 32 * q) : 0.0;
+#pragma unroll
+    for(int q = 0; q < N; q++)
+      if(t0 + lane + 32 * q < nb)
+        t[q] += v[q];
+  }
+  double s[1] = {warp_sum_d(sum_by_halves<N>([&](int q) { return t[q]; }))};
+  if(lane == 0)
+  {
+    *red.counter = 0u;
+    fin(s);
   }
 }
 
