@@ -312,10 +312,10 @@ int HelmFilter::apply(const double *in, double *out, bool sens, double tol, cuda
   }
   JacobiPcg<double> &P = *pcg;
   // a 3D grid that fits on the chip: all iterations as one kernel (pcgtile.cu)
-  if(P.tiles.ctas())
+  if(P.tiles.boxes())
     return finish(P.solveTiles(
-        [&] {
-          launch_pcg_tiles(P.tiles, P.d, T, dinv.p, phi.p, P.r.p, P.p.p, P.q.p, P.st.p, s);
+        [&](int jobs) {
+          launch_pcg_tiles(P.tiles, P.d, T, dinv.p, phi.p, P.r.p, P.p.p, P.q.p, P.st.p, jobs, s);
         },
         dinv.p, rhs.p, phi.p, tol, 10000, s, info));
   const Dims dd = d;

@@ -11,6 +11,7 @@
 #include <cfloat>
 #include <cmath>
 
+#include <atomic>
 #include <functional>
 
 #include "krylov.hpp"
@@ -283,6 +284,24 @@ struct SolveTimer
   }
 };
 
+/// a one-kernel solve from its launch to its end, counted on the current device
+struct TileJob
+{
+  std::atomic<int> &count;
+  int jobs; ///< with this one
+  TileJob() : count(of_device()), jobs(++count) {}
+  TileJob(const TileJob &) = delete;
+  TileJob &operator=(const TileJob &) = delete;
+  ~TileJob() { --count; }
+  static std::atomic<int> &of_device()
+  {
+    static std::atomic<int> counts[64];
+    int dev = 0;
+    ICB_CUDA(cudaGetDevice(&dev));
+    return counts[dev & 63];
+  }
+};
+
 template <typename T> JacobiPcg<T>::JacobiPcg(const Dims &dims, cudaStream_t s) : d(dims)
 {
   n = (long long)d.dim * d.ld;
@@ -322,10 +341,12 @@ int JacobiPcg<T>::solve(const T *K, const T *E, const uint8_t *fix, const T *inv
   if constexpr(sizeof(T) == 8)
   {
     // a small problem's iterations as one kernel (pcgtile.cu)
-    if(tiles.ctas())
+    if(tiles.boxes())
       return solveTiles(
-          [&] { launch_pcg_tiles(tiles, d, K, E, invdiag, x, r.p, p.p, q.p, st.p, s); }, invdiag,
-          b, x, tol, maxit, s, info);
+          [&](int jobs) {
+            launch_pcg_tiles(tiles, d, K, E, invdiag, x, r.p, p.p, q.p, st.p, jobs, s);
+          },
+          invdiag, b, x, tol, maxit, s, info);
   }
   const Dims dd = d;
   RedScratch *rp = &red;
@@ -339,14 +360,15 @@ int JacobiPcg<T>::solve(const T *K, const T *E, const uint8_t *fix, const T *inv
 }
 
 template <typename T>
-int JacobiPcg<T>::solveTiles(const std::function<void()> &iterate, const T *invdiag, const T *b,
+int JacobiPcg<T>::solveTiles(const std::function<void(int)> &iterate, const T *invdiag, const T *b,
                              T *x, double tol, int maxit, cudaStream_t s, icb_solve_info *info)
 {
+  const TileJob job;
   const SolveTimer timer(s);
   k_pcg_init<T><<<vec_blocks(n), VB, 0, s>>>(n, b, x, r.p, p.p, invdiag, red, st.p, tol, maxit);
   ICB_CUDA(cudaGetLastError());
   count_launch();
-  iterate();
+  iterate(job.jobs);
   ICB_CUDA(cudaMemcpyAsync(hst, st.p, sizeof(KState), cudaMemcpyDeviceToHost, s));
   return report(timer, info);
 }

@@ -43,9 +43,9 @@ template <typename T> struct JacobiPcg
   int solveOp(const std::function<void(cudaStream_t)> &op, const void *opKey0,
               const void *opKey1, const void *opKey2, const T *invdiag, const T *b, T *x,
               double tol, int maxit, cudaStream_t s, icb_solve_info *info);
-  /// the same with all iterations as one kernel, which iterate() launches on
-  /// this object's r, p, q and st (pcgtile.cu)
-  int solveTiles(const std::function<void()> &iterate, const T *invdiag, const T *b, T *x,
+  /// the same with all iterations as one kernel, which iterate(jobs) launches on
+  /// this object's r, p, q and st (pcgtile.cu); jobs: solves of this form in flight
+  int solveTiles(const std::function<void(int)> &iterate, const T *invdiag, const T *b, T *x,
                  double tol, int maxit, cudaStream_t s, icb_solve_info *info);
   /// wait for the solve and hand out what it left in hst
   int report(const SolveTimer &timer, icb_solve_info *info);

@@ -26,6 +26,11 @@
 // on 80 x 40 x 40 and 1,113 instead of 1,301 on 128 x 64 x 64, about the largest grid
 // whose vectors fit; an MMA run on 80 x 40 x 40 17.2 -> 15.0 ms.
 //
+// Solves that run at the same time (host threads, the batch runner's workers, the
+// server's slots) share the SMs: each then gives a CTA several boxes of its cut.  A
+// box's arithmetic and its place in the sums are the same wherever it runs, so a
+// solve's iterates do not depend on what else is in flight.
+//
 // The launch is cooperative (every CTA is resident), and every wait is bounded (an
 // iteration's polls of the ring together): a CTA whose wait runs out marks the
 // solve ICB_ERR_TIMEOUT and returns, and so do the others when theirs run out.
@@ -37,7 +42,6 @@
 #include <cfloat>
 #include <climits>
 
-#include "exchange.cuh"
 #include "hex8modal.cuh"
 
 namespace icb
@@ -51,6 +55,8 @@ template <int DIM> constexpr int kNodeThreads = DIM == 3 ? 192 : 256;
 /// of the scalar form: one a node, as many as an exchange takes
 constexpr int kScalarThreads = 512;
 constexpr int kTileSmem = 200 << 10, kScalarSmem = 226 << 10;
+/// boxes of a CTA at most, and their shared memory (their sums take some more)
+constexpr int kTileShare = 8, kShareSmem = 222 << 10;
 
 template <int DIM> struct ElemK;
 template <> struct ElemK<2>
@@ -223,90 +229,132 @@ template <> struct TileOp<3, 1>
   static constexpr int NT = kScalarThreads, kSmem = kScalarSmem;
 };
 
-template <int DIM, int NC>
+/// body(k, t, w) for the threads t of box k, in its warp w: the CTA's own threads when
+/// it has one box, else a warp at a time, `wbox` of each of the nb boxes
+template <bool MANY, int NT, class F>
+__device__ __forceinline__ void each_thread(int nb, int wbox, const F &body)
+{
+  const int tid = threadIdx.x, warp = tid >> 5;
+  if(!MANY)
+  {
+    body(0, tid, warp);
+    return;
+  }
+  for(int t = warp; t < nb * wbox; t += NT / 32)
+  {
+    const int k = t / wbox, w = t - k * wbox;
+    body(k, 32 * w + (tid & 31), w);
+  }
+}
+
+/// One box a CTA; MANY: the boxes blockIdx.x + gridDim.x k (tile_share).  A box is in
+/// shared memory with the direction and the moduli on the padded box, x, r, D^-1 and
+/// products of its own nodes and their (padded entry, node); the (entry, node) of all
+/// boxes' rings follow as one list.  With many boxes a warp takes 32 of a box's threads
+/// at a time: each adds the nodes that thread would add, so the boxes' sums, and with
+/// them all iterates, are bitwise those of one box a CTA.
+template <int DIM, int NC, bool MANY>
 __global__ void __launch_bounds__(TileOp<DIM, NC>::NT)
     k_pcg_tiles(const __grid_constant__ typename TileOp<DIM, NC>::K K, const Dims d, const PcgTiles T,
                 const double *__restrict__ E, const double *__restrict__ dinv,
                 double *__restrict__ x, double *__restrict__ r, double *p0, double *z, double *slots,
                 const unsigned polls, KState *st)
 {
-  constexpr int NT = TileOp<DIM, NC>::NT;
+  constexpr int NT = TileOp<DIM, NC>::NT, NB = MANY ? kTileShare : 1;
   constexpr bool kElastic = NC == DIM;
   extern __shared__ __align__(16) double pcg_dyn[];
-  __shared__ double sw[NT / 32][2], sres[3];
-  __shared__ int nring;
-  const int G = gridDim.x, cta = blockIdx.x, tid = threadIdx.x;
+  __shared__ double sw[NB][NT / 32][2], sres[3];
+  __shared__ int nring, nown[NB];
+  const int cta = blockIdx.x, tid = threadIdx.x, warp = tid >> 5;
+  const int G = gridDim.x, boxes = T.px * T.py * T.pz;
+  const int nb = MANY ? (boxes - cta + G - 1) / G : 1;
   // every CTA reads the state before any writes it (the last thing a solve does)
   if(st->stop)
     return;
   const double thr = st->thr;
   const int maxit = st->maxit;
   double rz = st->rz, rr = st->rr;
+  const int cap = T.bx * T.by * T.bz;
   Box<DIM> B;
-  const int cx = cta % T.px, cy = cta / T.px % T.py, cz = cta / (T.px * T.py);
-  B.x0 = cx * T.bx, B.y0 = cy * T.by, B.z0 = cz * T.bz;
-  B.nx = min(T.bx, d.sx - B.x0), B.ny = min(T.by, d.sy - B.y0), B.nz = min(T.bz, d.sz - B.z0);
-  B.own = B.nx * B.ny * B.nz;
   B.W = T.bx + 2;
   B.WH = DIM == 3 ? B.W * (T.by + 2) : 0;
   B.pad = B.W * (T.by + 2) * (DIM == 3 ? T.bz + 2 : 1);
-  const int cap = T.bx * T.by * T.bz;
+  // of box k: k stride further
+  const int stride = MANY ? T.smem / 8 - (B.pad - cap) : 0;
   double *sp = pcg_dyn, *sE = sp + NC * B.pad, *sx = sE + (kElastic ? B.pad : 0),
          *sr = sx + NC * cap, *sd = sr + NC * cap, *sq = sd + NC * cap, *sz = sq + NC * cap;
-  // (padded entry, node) of the box's own nodes and of the ring's
-  int2 *sown = reinterpret_cast<int2 *>(sq + (NC == 3 ? 2 : 1) * NC * cap), *sring = sown + cap;
+  int2 *sown = reinterpret_cast<int2 *>(sq + (NC == 3 ? 2 : 1) * NC * cap);
+  int2 *sring = MANY ? reinterpret_cast<int2 *>(pcg_dyn + nb * stride) : sown + cap;
+  const int wbox = (min(cap, NT) + 31) / 32; // warps of a box with nodes
   if(tid == 0)
     nring = 0;
+  if(MANY)
+    for(int t = tid; t < NB * (NT / 32) * 2; t += NT)
+      (&sw[0][0][0])[t] = 0.0; // the warps of a box without nodes
   __syncthreads();
-  // the box and its ring: moduli and direction, 0 outside the grid
-  for(int t = tid; t < B.pad; t += NT)
+  for(int k = 0; k < nb; k++)
   {
-    const int row = t / B.W, i = t - row * B.W - 1;
-    const int k = DIM == 3 ? row / (T.by + 2) - 1 : 0;
-    const int j = row - (DIM == 3 ? (k + 1) * (T.by + 2) : 0) - 1;
-    const int gx = B.x0 + i, gy = B.y0 + j, gz = B.z0 + k;
-    [[maybe_unused]] const bool elem = unsigned(gx) < unsigned(d.nx) && unsigned(gy) < unsigned(d.ny) &&
-                      (DIM == 2 || unsigned(gz) < unsigned(d.nz));
-    if constexpr(kElastic)
-      sE[t] = elem ? E[gx + (long long)d.nx * (gy + (long long)d.ny * gz)] : 0.0;
-    const bool node = unsigned(gx) < unsigned(d.sx) && unsigned(gy) < unsigned(d.sy) &&
-                      unsigned(gz) < unsigned(d.sz);
-    const int g = gx + d.sx * (gy + d.sy * gz);
-#pragma unroll
-    for(int c = 0; c < NC; c++)
-      sp[c * B.pad + t] = node ? __ldcg(p0 + c * d.ld + g) : 0.0;
-    if(node && !(unsigned(i) < unsigned(B.nx) && unsigned(j) < unsigned(B.ny) &&
-                 unsigned(k) < unsigned(B.nz)))
-      sring[atomicAdd(&nring, 1)] = make_int2(t, g); // any order: the entries are independent
-  }
-  for(int n = tid; n < B.own; n += NT)
-  {
-    const int row = n / B.nx, i = n - row * B.nx, k = row / B.ny, j = row - k * B.ny;
-    const int g = B.x0 + i + d.sx * (B.y0 + j + d.sy * (B.z0 + k));
-    int at = B.at(i, j, k);
-    if constexpr(!kElastic)
+    const int box = cta + G * k, o = k * stride;
+    const int cx = box % T.px, cy = box / T.px % T.py, cz = box / (T.px * T.py);
+    B.x0 = cx * T.bx, B.y0 = cy * T.by, B.z0 = cz * T.bz;
+    B.nx = min(T.bx, d.sx - B.x0), B.ny = min(T.by, d.sy - B.y0), B.nz = min(T.bz, d.sz - B.z0);
+    B.own = B.nx * B.ny * B.nz;
+    if(tid == 0)
+      nown[k] = B.own;
+    // the box and its ring: moduli and direction, 0 outside the grid
+    for(int t = tid; t < B.pad; t += NT)
     {
-      const int l[3] = {i, j, k}, lo[3] = {B.x0, B.y0, B.z0}, nb[3] = {B.nx, B.ny, B.nz},
-                last[3] = {d.sx - 1, d.sy - 1, d.sz - 1};
+      const int row = t / B.W, i = t - row * B.W - 1;
+      const int kz = DIM == 3 ? row / (T.by + 2) - 1 : 0;
+      const int j = row - (DIM == 3 ? (kz + 1) * (T.by + 2) : 0) - 1;
+      const int gx = B.x0 + i, gy = B.y0 + j, gz = B.z0 + kz;
+      [[maybe_unused]] const bool elem = unsigned(gx) < unsigned(d.nx) &&
+                                         unsigned(gy) < unsigned(d.ny) &&
+                                         (DIM == 2 || unsigned(gz) < unsigned(d.nz));
+      if constexpr(kElastic)
+        sE[o + t] = elem ? E[gx + (long long)d.nx * (gy + (long long)d.ny * gz)] : 0.0;
+      const bool node = unsigned(gx) < unsigned(d.sx) && unsigned(gy) < unsigned(d.sy) &&
+                        unsigned(gz) < unsigned(d.sz);
+      const int g = gx + d.sx * (gy + d.sy * gz);
 #pragma unroll
-      for(int a = 0; a < 3; a++)
+      for(int c = 0; c < NC; c++)
+        sp[o + c * B.pad + t] = node ? __ldcg(p0 + c * d.ld + g) : 0.0;
+      if(node && !(unsigned(i) < unsigned(B.nx) && unsigned(j) < unsigned(B.ny) &&
+                   unsigned(kz) < unsigned(B.nz)))
+        // any order: the entries are independent
+        sring[atomicAdd(&nring, 1)] = make_int2(o + t, g);
+    }
+    for(int n = tid; n < B.own; n += NT)
+    {
+      const int row = n / B.nx, i = n - row * B.nx, kz = row / B.ny, j = row - kz * B.ny;
+      const int g = B.x0 + i + d.sx * (B.y0 + j + d.sy * (B.z0 + kz));
+      int at = B.at(i, j, kz);
+      if constexpr(!kElastic)
       {
-        const int ga = lo[a] + l[a];
-        at |= ga == 0 ? kAtLow << 2 * a : 0;
-        at |= ga == last[a] ? kAtHigh << 2 * a : 0;
-        at |= (l[a] == 0 && ga > 0) || (l[a] == nb[a] - 1 && ga < last[a]) ? kAtFace : 0;
+        const int l[3] = {i, j, kz}, lo[3] = {B.x0, B.y0, B.z0}, nn[3] = {B.nx, B.ny, B.nz},
+                  last[3] = {d.sx - 1, d.sy - 1, d.sz - 1};
+#pragma unroll
+        for(int a = 0; a < 3; a++)
+        {
+          const int ga = lo[a] + l[a];
+          at |= ga == 0 ? kAtLow << 2 * a : 0;
+          at |= ga == last[a] ? kAtHigh << 2 * a : 0;
+          at |= (l[a] == 0 && ga > 0) || (l[a] == nn[a] - 1 && ga < last[a]) ? kAtFace : 0;
+        }
+      }
+      sown[o + n] = make_int2(at, g);
+#pragma unroll
+      for(int c = 0; c < NC; c++)
+      {
+        sx[o + c * cap + n] = 0.0;
+        sr[o + c * cap + n] = r[c * d.ld + g];
+        sd[o + c * cap + n] = dinv[c * d.ld + g];
       }
     }
-    sown[n] = make_int2(at, g);
-#pragma unroll
-    for(int c = 0; c < NC; c++)
-    {
-      sx[c * cap + n] = 0.0;
-      sr[c * cap + n] = r[c * d.ld + g];
-      sd[c * cap + n] = dinv[c * d.ld + g];
-    }
   }
   __syncthreads();
+  // nodes of box k
+  auto own = [&](int k) { return MANY ? nown[k] : B.own; };
   // the state of the loop, the same in every thread of every CTA
   int iter = 0, matvecs = 0, status = ICB_OK, conv = 0;
   double alpha = 0.0, beta = 0.0, pq = 0.0;
@@ -319,52 +367,82 @@ __global__ void __launch_bounds__(TileOp<DIM, NC>::NT)
     // The next value this CTA puts (first exchange of it + 1) is read by all
     // before their own fence (second exchange of it + 1), and only after that
     // fence do they read the emptied z (end of it + 1) or slots (it + 2) again.
-    double *set = slots + (it % 3) * kExSlot * G, *clear = slots + ((it + 2) % 3) * kExSlot * G;
+    double *set = slots + (it % 3) * kExSlot * boxes;
+    double *clear = slots + ((it + 2) % 3) * kExSlot * boxes;
     double *zcur = it & 1 ? p0 : z, *zold = it & 1 ? z : p0;
     // q = K p and p.q on the box (constrained rows of q are 0)
-    double v[1] = {0.0};
     if constexpr(NC == 3)
     {
+      // threads for the elements below the nodes and others for those above
       double q[3];
-      constexpr int NN = kNodeThreads<3>;
-      if(tid >= NN)
-        for(int n = tid - NN; n < B.own; n += NN)
-        {
-          node_product3<1>(K, sp, sE, B, sown[n].x, q);
+      auto below = [&](int o, int n) {
+        node_product3<1>(K, sp + o, sE + o, B, sown[o + n].x, q);
 #pragma unroll
-          for(int c = 0; c < 3; c++)
-            sq[c * cap + n] = q[c];
+        for(int c = 0; c < 3; c++)
+          sq[o + c * cap + n] = q[c];
+      };
+      auto above = [&](int o, int n) {
+        node_product3<0>(K, sp + o, sE + o, B, sown[o + n].x, q);
+#pragma unroll
+        for(int c = 0; c < 3; c++)
+          sz[o + c * cap + n] = q[c];
+      };
+      constexpr int NN = kNodeThreads<3>;
+      if constexpr(MANY)
+      {
+        const int wn = (cap + 31) / 32;
+        for(int t = warp; t < nb * 2 * wn; t += NT / 32)
+        {
+          const int k = t / (2 * wn), w = t - k * 2 * wn;
+          const int n = 32 * (w < wn ? w : w - wn) + (tid & 31);
+          if(n < own(k))
+          {
+            if(w < wn)
+              above(k * stride, n);
+            else
+              below(k * stride, n);
+          }
         }
+      }
+      else if(tid >= NN)
+        for(int n = tid - NN; n < B.own; n += NN)
+          below(0, n);
       else
         for(int n = tid; n < B.own; n += NN)
-        {
-          node_product3<0>(K, sp, sE, B, sown[n].x, q);
-#pragma unroll
-          for(int c = 0; c < 3; c++)
-            sz[c * cap + n] = q[c];
-        }
+          above(0, n);
       __syncthreads();
     }
-    for(int n = tid; n < B.own; n += NT)
-    {
-      const int at = sown[n].x, c0 = kElastic ? at : at & ((1 << kAtBits) - 1);
-      double q[NC];
-      if constexpr(!kElastic)
-        q[0] = node_helm(K, sp, B, at);
-      else if constexpr(DIM == 2)
-        node_product2(K, sp, sE, B, c0, q);
-#pragma unroll
-      for(int c = 0; c < NC; c++)
+    double v[1] = {0.0};
+    each_thread<MANY, NT>(nb, wbox, [&](int k, int t, int w) {
+      const int o = k * stride, nk = own(k);
+      if(MANY)
+        v[0] = 0.0;
+#pragma unroll 1
+      for(int n = t; n < nk; n += NT)
       {
-        if constexpr(NC == 3)
-          q[c] = sz[c * cap + n] + sq[c * cap + n];
-        if(sd[c * cap + n] == 0.0)
-          q[c] = 0.0;
-        sq[c * cap + n] = q[c];
-        v[0] += sp[c * B.pad + c0] * q[c];
+        const int at = sown[o + n].x, c0 = kElastic ? at : at & ((1 << kAtBits) - 1);
+        double q[NC];
+        if constexpr(!kElastic)
+          q[0] = node_helm(K, sp + o, B, at);
+        else if constexpr(DIM == 2)
+          node_product2(K, sp + o, sE + o, B, c0, q);
+#pragma unroll
+        for(int c = 0; c < NC; c++)
+        {
+          const int e = o + c * cap + n;
+          if constexpr(NC == 3)
+            q[c] = sz[e] + sq[e];
+          if(sd[e] == 0.0)
+            q[c] = 0.0;
+          sq[e] = q[c];
+          v[0] += sp[o + c * B.pad + c0] * q[c];
+        }
       }
-    }
-    bool ok = exchange<NT, 1>(v, 0, set, nullptr, polls, sw, sres);
+      if(MANY)
+        exchange_part<1>(v, sw[k][w]);
+    });
+    bool ok = MANY ? exchange_parts<NT, 1>(v, nb, boxes, 0, set, nullptr, polls, sw, sres)
+                   : exchange<NT, 1>(v, 0, set, nullptr, polls, sw[0], sres);
     pq = v[0];
     if(!ok)
     {
@@ -379,34 +457,44 @@ __global__ void __launch_bounds__(TileOp<DIM, NC>::NT)
       break;
     }
     // r -= alpha q; z = D^-1 r for the neighbours; r.r and r.z
-    double w[2] = {0.0, 0.0};
-    for(int n = tid; n < B.own; n += NT)
-    {
-      const int g = sown[n].y;
-#pragma unroll
-      for(int c = 0; c < NC; c++)
+    double w2[2] = {0.0, 0.0};
+    each_thread<MANY, NT>(nb, wbox, [&](int k, int t, int w) {
+      const int o = k * stride, nk = own(k);
+      if(MANY)
+        w2[0] = w2[1] = 0.0;
+#pragma unroll 1
+      for(int n = t; n < nk; n += NT)
       {
-        const double ri = sr[c * cap + n] - alpha * sq[c * cap + n];
-        sr[c * cap + n] = ri;
-        const double zi = sd[c * cap + n] * ri;
-        // an elastic box is small: nearly all its nodes are on its faces
-        if(kElastic || (sown[n].x & kAtFace))
+        const int2 to = sown[o + n];
+#pragma unroll
+        for(int c = 0; c < NC; c++)
         {
-          slot_put(zcur + c * d.ld + g, zi);
-          slot_store(zold + c * d.ld + g, kExEmpty);
+          const int e = o + c * cap + n;
+          const double ri = sr[e] - alpha * sq[e];
+          sr[e] = ri;
+          const double zi = sd[e] * ri;
+          // an elastic box is small: nearly all its nodes are on its faces
+          if(kElastic || (to.x & kAtFace))
+          {
+            slot_put(zcur + c * d.ld + to.y, zi);
+            slot_store(zold + c * d.ld + to.y, kExEmpty);
+          }
+          w2[0] += ri * ri;
+          w2[1] += ri * zi;
         }
-        w[0] += ri * ri;
-        w[1] += ri * zi;
       }
-    }
-    ok = exchange<NT, 2>(w, 1, set, clear, polls, sw, sres);
+      if(MANY)
+        exchange_part<2>(w2, sw[k][w]);
+    });
+    ok = MANY ? exchange_parts<NT, 2>(w2, nb, boxes, 1, set, clear, polls, sw, sres)
+              : exchange<NT, 2>(w2, 1, set, clear, polls, sw[0], sres);
     if(!ok)
     {
       status = ICB_ERR_TIMEOUT;
       break;
     }
-    rr = w[0];
-    if(!isfinite(rr) || !isfinite(w[1]))
+    rr = w2[0];
+    if(!isfinite(rr) || !isfinite(w2[1]))
     {
       status = ICB_ERR_NAN;
       break;
@@ -414,21 +502,26 @@ __global__ void __launch_bounds__(TileOp<DIM, NC>::NT)
     conv = rr < thr;
     if(!conv)
     {
-      beta = w[1] / rz;
-      rz = w[1];
+      beta = w2[1] / rz;
+      rz = w2[1];
     }
     // x += alpha p; p = z + beta p on the box, then on the ring
-    for(int n = tid; n < B.own; n += NT)
-    {
-      const int c0 = kElastic ? sown[n].x : sown[n].x & ((1 << kAtBits) - 1);
-#pragma unroll
-      for(int c = 0; c < NC; c++)
+    each_thread<MANY, NT>(nb, wbox, [&](int k, int t, int) {
+      const int o = k * stride, nk = own(k);
+#pragma unroll 1
+      for(int n = t; n < nk; n += NT)
       {
-        const double pi = sp[c * B.pad + c0];
-        sx[c * cap + n] += alpha * pi;
-        sp[c * B.pad + c0] = sd[c * cap + n] * sr[c * cap + n] + beta * pi;
+        const int at = sown[o + n].x, c0 = kElastic ? at : at & ((1 << kAtBits) - 1);
+#pragma unroll
+        for(int c = 0; c < NC; c++)
+        {
+          const int e = o + c * cap + n, a = o + c * B.pad + c0;
+          const double pi = sp[a];
+          sx[e] += alpha * pi;
+          sp[a] = fma(beta, pi, sd[e] * sr[e]);
+        }
       }
-    }
+    });
     if(conv)
       break;
     iter++;
@@ -461,8 +554,7 @@ __global__ void __launch_bounds__(TileOp<DIM, NC>::NT)
       late = more;
 #pragma unroll
       for(int c = 0; c < NC; c++)
-        sp[c * B.pad + e.x] =
-            __longlong_as_double((long long)b[c]) + beta * sp[c * B.pad + e.x];
+        sp[c * B.pad + e.x] = fma(beta, sp[c * B.pad + e.x], __longlong_as_double((long long)b[c]));
     }
     if(__syncthreads_or(late))
     {
@@ -470,16 +562,19 @@ __global__ void __launch_bounds__(TileOp<DIM, NC>::NT)
       break;
     }
   }
-  for(int n = tid; n < B.own; n += NT)
-  {
-    const int g = sown[n].y;
-#pragma unroll
-    for(int c = 0; c < NC; c++)
+  each_thread<MANY, NT>(nb, wbox, [&](int k, int t, int) {
+    const int o = k * stride, nk = own(k);
+    for(int n = t; n < nk; n += NT)
     {
-      x[c * d.ld + g] = sx[c * cap + n];
-      r[c * d.ld + g] = sr[c * cap + n];
+      const int g = sown[o + n].y;
+#pragma unroll
+      for(int c = 0; c < NC; c++)
+      {
+        x[c * d.ld + g] = sx[o + c * cap + n];
+        r[c * d.ld + g] = sr[o + c * cap + n];
+      }
     }
-  }
+  });
   if(tid == 0 && status == ICB_ERR_TIMEOUT)
   {
     atomicExch(&st->status, ICB_ERR_TIMEOUT);
@@ -545,7 +640,7 @@ PcgTiles pcg_tiles(const Dims &d)
           continue;
         // cycles of an iteration that depend on the cut: the element work, the
         // ring, and the polls of two exchanges (measured slopes)
-        const long long cost = own * (d.dim == 3 ? 20 : scalar ? 3 : 4) + (pad - own) * 3 + t.ctas() * 12;
+        const long long cost = own * (d.dim == 3 ? 20 : scalar ? 3 : 4) + (pad - own) * 3 + t.boxes() * 12;
         if(cost < bestCost)
         {
           bestCost = cost;
@@ -557,36 +652,66 @@ PcgTiles pcg_tiles(const Dims &d)
   return best;
 }
 
-template <int DIM, int NC>
-static void run_tiles(const PcgTiles &t, const Dims &d, typename TileOp<DIM, NC>::K K,
-                      const double *E, const double *invdiag, double *x, double *r, double *p,
-                      double *z, KState *st, cudaStream_t s)
+/// boxes of a CTA when `jobs` solves are on the device: each then takes its part of the
+/// SMs.  The cut for one solve fills the chip, so that a second one would wait for it.
+/// Microseconds an iteration and solve, with 1, 2, 4 and 8 threads solving: one box a
+/// CTA always, this rule, and three kernels an iteration
+///   40x15x15   7.2 7.0 6.9 6.9    7.0  5.2  3.4  3.9   16.5  9.4  5.4  3.4
+///   60x20x20   7.8 7.6 7.5 7.5    7.8  6.6  5.4  5.6   18.1 11.0  6.3  4.5
+///   50x30x30  10.4 10.1 10.0 10.0 10.3  8.8  8.7  8.3  21.9 13.0  8.1  6.8
+///   40x40x40  12.5 12.2 12.2 12.2 12.5 10.5 10.5 10.0  24.2 14.7 10.5 10.3
+///   300x100    5.8 5.6 5.6 5.6    5.8  5.2  3.8  4.0   16.6  9.0  5.3  3.5
+///   120x40     5.0 2.6 1.7 1.7    4.8  2.5  1.8  1.7   15.9  8.4  4.3  2.4
+/// Boxes of more than half of kShareSmem (3D grids of more than 70k nodes or so, 2D ones
+/// of more than 150k) stay alone on an SM: 48x46x45 16.4 with any number, three kernels
+/// 27.3, 17.0, 12.6 and 13.0; 540x540 10.2, three kernels 32.2, 18.8, 15.1, 16.6.
+static int tile_share(const PcgTiles &t, int jobs)
+{
+  const long long m = ((long long)t.boxes() * jobs + num_sms() - 1) / num_sms();
+  return int(std::max(1LL, std::min<long long>({m, kTileShare, kShareSmem / t.smem})));
+}
+
+template <int DIM, int NC, bool MANY>
+static void run_tiles_as(const PcgTiles &t, int share, const Dims &d,
+                         typename TileOp<DIM, NC>::K K, const double *E, const double *invdiag,
+                         double *x, double *r, double *p, double *z, KState *st, cudaStream_t s)
 {
   const size_t nsoa = size_t(NC) * size_t(d.ld);
   // the shared-memory opt-in is a per-device attribute shared by every host
   // thread: always its largest value
-  ICB_CUDA(cudaFuncSetAttribute(k_pcg_tiles<DIM, NC>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                TileOp<DIM, NC>::kSmem));
+  ICB_CUDA(cudaFuncSetAttribute(k_pcg_tiles<DIM, NC, MANY>,
+                                cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                MANY ? kShareSmem : TileOp<DIM, NC>::kSmem));
   double *slots = z + nsoa; // a multiple of 64 doubles past z: line-aligned
   ICB_CUDA(cudaMemsetAsync(z, 0xff, sizeof(double) * (nsoa + pcg_tile_slots(t)), s)); // kExEmpty
   Dims dd = d;
   PcgTiles tt = t;
   unsigned polls = exchange_spin_limit();
   void *args[] = {&K, &dd, &tt, &E, &invdiag, &x, &r, &p, &z, &slots, &polls, &st};
-  ICB_CUDA(cudaLaunchCooperativeKernel((const void *)k_pcg_tiles<DIM, NC>, dim3(t.ctas()),
-                                       dim3(TileOp<DIM, NC>::NT), args, size_t(t.smem), s));
+  ICB_CUDA(cudaLaunchCooperativeKernel((const void *)k_pcg_tiles<DIM, NC, MANY>,
+                                       dim3(unsigned((t.boxes() + share - 1) / share)),
+                                       dim3(TileOp<DIM, NC>::NT), args, size_t(t.smem) * share, s));
   count_launch();
+}
+template <int DIM, int NC>
+static void run_tiles(const PcgTiles &t, const Dims &d, const typename TileOp<DIM, NC>::K &K,
+                      const double *E, const double *invdiag, double *x, double *r, double *p,
+                      double *z, KState *st, int jobs, cudaStream_t s)
+{
+  const int share = tile_share(t, jobs);
+  (share > 1 ? run_tiles_as<DIM, NC, true> : run_tiles_as<DIM, NC, false>)(
+      t, share, d, K, E, invdiag, x, r, p, z, st, s);
 }
 
 void launch_pcg_tiles(const PcgTiles &t, const Dims &d, const double *K, const double *E,
                       const double *invdiag, double *x, double *r, double *p, double *z,
-                      KState *st, cudaStream_t s)
+                      KState *st, int jobs, cudaStream_t s)
 {
   if(d.dim == 2)
   {
     ElemK<2> k;
     std::copy(K, K + 64, k.k);
-    run_tiles<2, 2>(t, d, k, E, invdiag, x, r, p, z, st, s);
+    run_tiles<2, 2>(t, d, k, E, invdiag, x, r, p, z, st, jobs, s);
   }
   else
   {
@@ -594,14 +719,14 @@ void launch_pcg_tiles(const PcgTiles &t, const Dims &d, const double *K, const d
     for(int i = 0, m = 0; i < 24; i++)
       for(int j = i; j < 24; j++)
         k.k[m++] = K[i * 24 + j];
-    run_tiles<3, 3>(t, d, k, E, invdiag, x, r, p, z, st, s);
+    run_tiles<3, 3>(t, d, k, E, invdiag, x, r, p, z, st, jobs, s);
   }
 }
 
 void launch_pcg_tiles(const PcgTiles &t, const Dims &d, const HelmTensor &C,
                       const double *invdiag, double *x, double *r, double *p, double *z,
-                      KState *st, cudaStream_t s)
+                      KState *st, int jobs, cudaStream_t s)
 {
-  run_tiles<3, 1>(t, d, C, nullptr, invdiag, x, r, p, z, st, s);
+  run_tiles<3, 1>(t, d, C, nullptr, invdiag, x, r, p, z, st, jobs, s);
 }
 } // namespace icb
