@@ -1366,14 +1366,14 @@ static int resident_ctas(const void *kern, int threads, int smem)
 /// z planes per CTA of the Hex8 kernels: `tiles` x-y tiles, `resident` CTAs
 /// in flight.  A CTA marches zchunk + 1 element layers (the layer below its
 /// chunk is recomputed), and the launch takes ceil(CTAs / resident) rounds,
-/// so the split minimises rounds x (zchunk + 1).
-static int h8_zchunk(const Dims &d, long long tiles, int resident)
+/// so the split minimises rounds x (zchunk + 1); *layers: that minimum.
+static int h8_zchunk(const Dims &d, long long tiles, int resident, long long *layers = nullptr)
 {
   int best = d.sz;
   long long bestCost = -1;
-  for(int bz = 1; bz <= d.sz; bz++)
+  for(int bz = 1, zc = 0; zc != 1; bz = (d.sz + zc - 2) / std::max(zc - 1, 1))
   {
-    const int zc = (d.sz + bz - 1) / bz;
+    zc = (d.sz + bz - 1) / bz; // the next bz is the first with a smaller one
     const long long n = tiles * ((d.sz + zc - 1) / zc);
     const long long cost = (n + resident - 1) / resident * (zc + 1);
     if(bestCost < 0 || cost < bestCost)
@@ -1382,6 +1382,8 @@ static int h8_zchunk(const Dims &d, long long tiles, int resident)
       best = zc;
     }
   }
+  if(layers)
+    *layers = bestCost;
   return best;
 }
 
@@ -1510,13 +1512,8 @@ static void launch_op_mode(const Dims &d, const T *K, const T *E, const T *u, T 
   Epi<T> ep{x.b, x.dinv, T(x.omega), T(x.c1), T(x.c2), x.prev0};
   if(d.dim == 3)
   {
-    // element rows per tile: 8; 12 for the FP64 product (with and without the
-    // dot) and residual in corner-mode form, whose registers (168) still fit 384
-    // threads without spills: 12 warps an SM and a smaller halo (y = K u at
-    // 384x128x128 183 us, with 8 rows 198; the Chebyshev step spills at 12 rows, 288
-    // against 285 us).  12 rows for FP32 measured 89.6 against 88.2 us.
+    // element rows per tile: 8, or 12 (below)
     constexpr int TYK0 = TY3;
-    constexpr int TYK1 = sizeof(T) == 8 && MODE <= OP_RESIDUAL ? TY3 + 4 : TY3;
     const int bx = (d.sx + TX - 2) / (TX - 1);
     auto run = [&](auto kern, const auto &kp, int smem, int rows) {
       const int by = (d.sy + rows - 2) / (rows - 1);
@@ -1556,10 +1553,38 @@ static void launch_op_mode(const Dims &d, const T *K, const T *E, const T *u, T 
       // 3 (FP32) CTAs of 256 threads per SM; FP64 one, whose registers let the next
       // plane's loads go out a whole layer ahead and keep the bottom plane's modes.
       // (The fused dot at two CTAs of 8 rows under 128 registers, modes in shared
-      // memory and the loads after the product, took 211 us at 384x128x128, DOTUS now.)
+      // memory and the loads after the product: 241 us at 384x128x128, now 214.)
       constexpr int MB = sizeof(T) == 8 ? 1 : 3;
-      run(x.dotRed ? k_matvec_h8m<T, TYK1, true, MODE, MB> : k_matvec_h8m<T, TYK1, false, MODE, MB>,
-          kmod, h8m_smem_bytes<T, TYK1>(), TYK1);
+      auto kern8 = x.dotRed ? k_matvec_h8m<T, TYK0, true, MODE, MB>
+                            : k_matvec_h8m<T, TYK0, false, MODE, MB>;
+      if constexpr(sizeof(T) == 8 && MODE <= OP_RESIDUAL)
+      {
+        // The FP64 product (with and without the dot) and residual fit 384 threads
+        // without spills (168 registers): tiles of 12 rows have a smaller halo, and a
+        // layer of them takes 1.5 times one of 8 rows (1.39 to 1.59 over the sizes
+        // below), so the fewer of 3 x layers and 2 x layers.  Product with the dot, 8
+        // and 12 rows: 240x80x80 55.5 and 63.0 us, 256x100x64 60.2 and 64.2, 60x60x60
+        // 13.0 and 14.0; 384x128x128 217 and 214, 300x100x75 97.4 and 84.4, 128x64x64
+        // 29.9 and 27.1 (without it 198 and 183 at 384x128x128).  The Chebyshev step
+        // spills at 12 rows (288 against 285 us); FP32 took 89.6 us with 12 and 88.2
+        // with 8.
+        constexpr int TYK1 = TY3 + 4;
+        auto kern12 = x.dotRed ? k_matvec_h8m<T, TYK1, true, MODE, MB>
+                               : k_matvec_h8m<T, TYK1, false, MODE, MB>;
+        auto layers = [&](auto kern, int smem, int rows) {
+          long long n = 0;
+          h8_zchunk(d, (long long)bx * ((d.sy + rows - 2) / (rows - 1)),
+                    resident_ctas((const void *)kern, TX * rows, smem), &n);
+          return n;
+        };
+        if(2 * layers(kern8, h8m_smem_bytes<T, TYK0>(), TYK0) <
+           3 * layers(kern12, h8m_smem_bytes<T, TYK1>(), TYK1))
+          run(kern8, kmod, h8m_smem_bytes<T, TYK0>(), TYK0);
+        else
+          run(kern12, kmod, h8m_smem_bytes<T, TYK1>(), TYK1);
+      }
+      else
+        run(kern8, kmod, h8m_smem_bytes<T, TYK0>(), TYK0);
     }
     else if constexpr(std::is_same<T, double>::value)
     {
