@@ -14,6 +14,7 @@ unsigned long long kernel_switches()
 {
   return (tc_operator_enabled() ? 1ull : 0ull) | (hex8_modal_enabled() ? 2ull : 0ull) |
          (device_loops_enabled() ? 4ull : 0ull) | (hex8_pair_enabled() ? 8ull : 0ull) |
+         (hex8_far_enabled() ? 16ull : 0ull) |
          ((unsigned long long)tc_spin_limit() << 8);
 }
 

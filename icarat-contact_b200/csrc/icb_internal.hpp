@@ -295,6 +295,10 @@ void set_hex8_modal(bool on);
 /// whether FP32 corner-mode Hex8 launches run two element rows per thread
 bool hex8_pair_enabled();
 void set_hex8_pair(bool on);
+/// whether corner-mode Hex8 launches count their offsets per z chunk on every grid, not
+/// only where they exceed 32 bits
+bool hex8_far_enabled();
+void set_hex8_far(bool on);
 
 /// K: HOST pointer to the unit element matrix ((d*ne)^2 entries); it is
 /// passed by value, so the kernel's FMAs take it from the constant bank.

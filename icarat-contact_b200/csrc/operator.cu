@@ -30,6 +30,7 @@
 
 #include <algorithm>
 #include <atomic>
+#include <climits>
 #include <cmath>
 #include <mutex>
 #include <unordered_map>
@@ -304,10 +305,20 @@ template <typename T, int TYK> constexpr int h8m_smem_bytes()
 {
   return int(sizeof(T)) * 12 * TYK * TX;
 }
+static std::atomic<bool> g_hex8_far{false}; // the FAR form on every grid
 /// whether a grid's vectors can be addressed by 32-bit byte offsets per component
 template <typename T> inline bool h8m_offsets_fit(const Dims &d)
 {
-  return (unsigned long long)d.nnode * sizeof(T) < (1ull << 32);
+  return !g_hex8_far && d.nnode * (long long)sizeof(T) < (1LL << 32);
+}
+/// most node planes of a CTA's z chunk in the FAR form of k_matvec_h8m, for grids whose
+/// vectors cannot: it addresses the planes it reads (one more below and above) by 32-bit
+/// byte offsets from its first one.  Below 1 on grids of planes of more than 2^30 bytes a
+/// component, which the dense kernel takes
+template <typename T> inline int h8m_most_planes(const Dims &d)
+{
+  const unsigned long long plane = (unsigned long long)d.sx * d.sy * sizeof(T);
+  return int(std::min<unsigned long long>((1ull << 32) / plane, 1u << 30)) - 3;
 }
 /// base[off bytes]: a base all threads share and a 32-bit offset (one register
 /// serves every component and vector at the same node)
@@ -328,12 +339,16 @@ template <typename T> __device__ __forceinline__ T *at_byte(T *base, unsigned of
 /// small: one 32-bit byte offset per node row serves all components (instead of
 /// twelve 64-bit addresses), and columns and planes outside the grid read the
 /// nearest inside with a zero modulus instead of selecting zeros.
-template <typename T, int TYK, bool DOT, int MODE, int MINB>
+/// FAR: grids whose offsets exceed 32 bits count them from the chunk's first plane
+/// (820x820x810 elements, FP64: 15.0 ms, the dense product 28.9); the others from the
+/// arrays' (the same pointer arithmetic took an FP32 Chebyshev step from 222 to 238 us
+/// at 384x128x128).
+template <typename T, int TYK, bool DOT, int MODE, int MINB, bool FAR = false>
 __global__ void __launch_bounds__(TX *TYK, MINB)
     k_matvec_h8m(const KModal<T> K, const Dims d, const int zchunk,
                  const T *__restrict__ E, const T *__restrict__ u, T *__restrict__ y,
                  const uint8_t *__restrict__ fix, RedScratch red, double *dotOut,
-                 const KState *gate, const int gateConv, const Epi<T> ep)
+                 const KState *gate, const int gateConv, Epi<T> ep)
 {
   if(gate && (gate->stop || (gateConv && gate->conv)))
     return;
@@ -353,11 +368,25 @@ __global__ void __launch_bounds__(TX *TYK, MINB)
   const unsigned sxy = unsigned(d.sx) * unsigned(d.sy) * unsigned(sizeof(T));
   const unsigned exy = unsigned(d.nx) * unsigned(d.ny) * unsigned(sizeof(T));
   const long long ld = d.ld;
+  const int Zb = FAR ? max(Z0 - 1, 0) : 0;
+  if constexpr(FAR)
+  {
+    // from here on all arrays begin at the chunk's first plane
+    const long long below = (long long)Zb * d.sx * d.sy;
+    u += below;
+    y += below;
+    fix += below;
+    E += (long long)Zb * d.nx * d.ny;
+    if(MODE != OP_APPLY)
+      ep.b += below;
+    if(MODE >= OP_JACOBI)
+      ep.dinv += below;
+  }
   // byte offsets of the column's low corners in the two node rows, of the next
   // plane to load (planes outside the grid: the nearest)
   const int cx = min(max(ei, 0), d.nx - 1), cy = min(max(ej, 0), d.ny - 1);
   unsigned o0 = (unsigned(cx) + unsigned(cy) * unsigned(d.sx)) * unsigned(sizeof(T)) +
-                unsigned(max(Z0 - 1, 0)) * sxy;
+                unsigned(max(Z0 - 1, 0) - Zb) * sxy;
   const unsigned rowb = unsigned(d.sx) * unsigned(sizeof(T));
   auto load_plane = [&](T(&v)[3][4]) {
     const unsigned o1 = o0 + rowb;
@@ -372,7 +401,7 @@ __global__ void __launch_bounds__(TX *TYK, MINB)
     }
   };
   unsigned eo = (unsigned(cx) + unsigned(cy) * unsigned(d.nx)) * unsigned(sizeof(T)) +
-                unsigned(max(Z0 - 1, 0)) * exy;
+                unsigned(max(Z0 - 1, 0) - Zb) * exy;
   auto load_E = [&](int k) { return col && k >= 0 && k < d.nz ? __ldg(at_byte(E, eo)) : T(0); };
 
   // the bottom plane's x-y modes; the top-face result carried up (sC)
@@ -396,7 +425,7 @@ __global__ void __launch_bounds__(TX *TYK, MINB)
   const int ni = ei + 1, nj = ej + 1;
   const bool ownCol = lx < TX - 1 && ly < TYK - 1 && ni < d.sx && nj < d.sy;
   unsigned node = (unsigned(ni) + unsigned(nj) * unsigned(d.sx)) * unsigned(sizeof(T)) +
-                  (unsigned(Z0) - 1u) * sxy; // wraps below plane 0, where it is not used
+                  (unsigned(Z0 - Zb) - 1u) * sxy; // wraps below plane 0, where it is not used
   double dot = 0.0;
   for(int ek = Z0 - 1; ek <= Z1; ++ek)
   {
@@ -1367,13 +1396,17 @@ static int resident_ctas(const void *kern, int threads, int smem)
 /// in flight.  A CTA marches zchunk + 1 element layers (the layer below its
 /// chunk is recomputed), and the launch takes ceil(CTAs / resident) rounds,
 /// so the split minimises rounds x (zchunk + 1); *layers: that minimum.
-static int h8_zchunk(const Dims &d, long long tiles, int resident, long long *layers = nullptr)
+/// Chunks have at most `most` planes.
+static int h8_zchunk(const Dims &d, long long tiles, int resident, int most = INT_MAX,
+                     long long *layers = nullptr)
 {
   int best = d.sz;
   long long bestCost = -1;
   for(int bz = 1, zc = 0; zc != 1; bz = (d.sz + zc - 2) / std::max(zc - 1, 1))
   {
     zc = (d.sz + bz - 1) / bz; // the next bz is the first with a smaller one
+    if(zc > most)
+      continue;
     const long long n = tiles * ((d.sz + zc - 1) / zc);
     const long long cost = (n + resident - 1) / resident * (zc + 1);
     if(bestCost < 0 || cost < bestCost)
@@ -1409,10 +1442,13 @@ int matvec_blocks(const Dims &d)
     {
       const long long tiles = bx * ((d.sy + rows - 1) / rows);
       for(int k = 1; k <= 8; k++)
-      {
-        const int zc = h8_zchunk(d, tiles, k * num_sms());
-        most = std::max(most, tiles * ((d.sz + zc - 1) / zc));
-      }
+        for(int planes : {INT_MAX, h8m_most_planes<double>(d), h8m_most_planes<float>(d)})
+        {
+          if(planes < 1)
+            continue; // the dense kernel's, without a limit
+          const int zc = h8_zchunk(d, tiles, k * num_sms(), planes);
+          most = std::max(most, tiles * ((d.sz + zc - 1) / zc));
+        }
     }
     return int(most);
   }
@@ -1515,10 +1551,10 @@ static void launch_op_mode(const Dims &d, const T *K, const T *E, const T *u, T 
     // element rows per tile: 8, or 12 (below)
     constexpr int TYK0 = TY3;
     const int bx = (d.sx + TX - 2) / (TX - 1);
-    auto run = [&](auto kern, const auto &kp, int smem, int rows) {
+    auto run = [&](auto kern, const auto &kp, int smem, int rows, int planes) {
       const int by = (d.sy + rows - 2) / (rows - 1);
-      const int zchunk =
-          h8_zchunk(d, (long long)bx * by, resident_ctas((const void *)kern, TX * rows, smem));
+      const int zchunk = h8_zchunk(d, (long long)bx * by,
+                                   resident_ctas((const void *)kern, TX * rows, smem), planes);
       const int bz = (d.sz + zchunk - 1) / zchunk;
       if(x.dotRed)
         ICB_REQUIRE((long long)bx * by * bz <= red.maxBlocks, "reduction scratch too small");
@@ -1548,7 +1584,9 @@ static void launch_op_mode(const Dims &d, const T *K, const T *E, const T *u, T 
         return;
       }
     }
-    if(g_hex8_modal && h8m_offsets_fit<T>(d) && modal_form_cached(K, kmod))
+    const bool far = !h8m_offsets_fit<T>(d);
+    const int planes = far ? h8m_most_planes<T>(d) : INT_MAX;
+    if(g_hex8_modal && planes >= 1 && modal_form_cached(K, kmod))
     {
       // 3 (FP32) CTAs of 256 threads per SM; FP64 one, whose registers let the next
       // plane's loads go out a whole layer ahead and keep the bottom plane's modes.
@@ -1557,7 +1595,11 @@ static void launch_op_mode(const Dims &d, const T *K, const T *E, const T *u, T 
       constexpr int MB = sizeof(T) == 8 ? 1 : 3;
       auto kern8 = x.dotRed ? k_matvec_h8m<T, TYK0, true, MODE, MB>
                             : k_matvec_h8m<T, TYK0, false, MODE, MB>;
-      if constexpr(sizeof(T) == 8 && MODE <= OP_RESIDUAL)
+      if(far)
+        run(x.dotRed ? k_matvec_h8m<T, TYK0, true, MODE, MB, true>
+                     : k_matvec_h8m<T, TYK0, false, MODE, MB, true>,
+            kmod, h8m_smem_bytes<T, TYK0>(), TYK0, planes);
+      else if constexpr(sizeof(T) == 8 && MODE <= OP_RESIDUAL)
       {
         // The FP64 product (with and without the dot) and residual fit 384 threads
         // without spills (168 registers): tiles of 12 rows have a smaller halo, and a
@@ -1574,17 +1616,17 @@ static void launch_op_mode(const Dims &d, const T *K, const T *E, const T *u, T 
         auto layers = [&](auto kern, int smem, int rows) {
           long long n = 0;
           h8_zchunk(d, (long long)bx * ((d.sy + rows - 2) / (rows - 1)),
-                    resident_ctas((const void *)kern, TX * rows, smem), &n);
+                    resident_ctas((const void *)kern, TX * rows, smem), planes, &n);
           return n;
         };
         if(2 * layers(kern8, h8m_smem_bytes<T, TYK0>(), TYK0) <
            3 * layers(kern12, h8m_smem_bytes<T, TYK1>(), TYK1))
-          run(kern8, kmod, h8m_smem_bytes<T, TYK0>(), TYK0);
+          run(kern8, kmod, h8m_smem_bytes<T, TYK0>(), TYK0, planes);
         else
-          run(kern12, kmod, h8m_smem_bytes<T, TYK1>(), TYK1);
+          run(kern12, kmod, h8m_smem_bytes<T, TYK1>(), TYK1, planes);
       }
       else
-        run(kern8, kmod, h8m_smem_bytes<T, TYK0>(), TYK0);
+        run(kern8, kmod, h8m_smem_bytes<T, TYK0>(), TYK0, planes);
     }
     else if constexpr(std::is_same<T, double>::value)
     {
@@ -1593,18 +1635,18 @@ static void launch_op_mode(const Dims &d, const T *K, const T *E, const T *u, T 
         for(int c = r; c < 24; c++)
           ks.k[symIdx(r, c)] = K[r * 24 + c];
       if(x.dotRed)
-        run(k_matvec_h8<T, KSym24, TYK0, true, MODE>, ks, 0, TYK0);
+        run(k_matvec_h8<T, KSym24, TYK0, true, MODE>, ks, 0, TYK0, INT_MAX);
       else
-        run(k_matvec_h8<T, KSym24, TYK0, false, MODE>, ks, 0, TYK0);
+        run(k_matvec_h8<T, KSym24, TYK0, false, MODE>, ks, 0, TYK0, INT_MAX);
     }
     else
     {
       KMat<T, 24> km;
       std::copy(K, K + 576, km.k);
       if(x.dotRed)
-        run(k_matvec_h8<T, KMat<T, 24>, TYK0, true, MODE>, km, 0, TYK0);
+        run(k_matvec_h8<T, KMat<T, 24>, TYK0, true, MODE>, km, 0, TYK0, INT_MAX);
       else
-        run(k_matvec_h8<T, KMat<T, 24>, TYK0, false, MODE>, km, 0, TYK0);
+        run(k_matvec_h8<T, KMat<T, 24>, TYK0, false, MODE>, km, 0, TYK0, INT_MAX);
     }
   }
   else
@@ -1726,6 +1768,8 @@ bool hex8_modal_enabled() { return g_hex8_modal; }
 void set_hex8_modal(bool on) { g_hex8_modal = on; }
 bool hex8_pair_enabled() { return g_hex8_pair; }
 void set_hex8_pair(bool on) { g_hex8_pair = on; }
+bool hex8_far_enabled() { return g_hex8_far; }
+void set_hex8_far(bool on) { g_hex8_far = on; }
 
 template <typename T>
 void launch_op(const Dims &d, const T *K, const T *E, const T *u, T *y, const uint8_t *fix,

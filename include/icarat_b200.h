@@ -447,7 +447,9 @@ long long icb_launch_count(void);
  * microseconds and count, by the share of the batch still iterating when
  * each started: more than a half, more than an eighth, at most an eighth).
  * Further switches: "hex8_pair" (FP32 Hex8 operator with two element rows per
- * thread), "tc_spin_limit" (polls of a tensor-core wait before it gives up),
+ * thread), "hex8_far" (the corner-mode operator takes every grid as it takes
+ * those whose vectors exceed 2^32 bytes a component), "tc_spin_limit" (polls
+ * of a tensor-core wait before it gives up),
  * "exchange_spin_limit" (polls of a wait between the blocks of a one-kernel
  * solve, filter or OC update before it ends with ICB_ERR_TIMEOUT),
  * "batch_fused" (icb_run_batch advances qualifying 2D OC batches together),
