@@ -11,6 +11,7 @@
 
 #include "graphloop.hpp"
 #include "mg.hpp"
+#include "mgtail.cuh"
 #include "problem.hpp"
 
 using namespace icb;
@@ -601,6 +602,13 @@ int icb_set_option(const char *name, long long value)
     set_device_loops(value != 0);
   else if(n == "hex8_pair")
     set_hex8_pair(value != 0);
+  else if(n == "mg_tail")
+    set_mg_tail(value != 0);
+  else if(n == "mg_restrict_planes")
+  {
+    need(value >= 0 && value <= 64, "mg_restrict_planes must be in [0, 64]");
+    set_mg_restrict_planes(int(value));
+  }
   else if(n == "hex8_far")
     set_hex8_far(value != 0);
   else if(n == "batch_fused")
@@ -638,6 +646,10 @@ long long icb_get_option(const char *name)
     return device_loops_enabled() ? 1 : 0;
   if(n == "hex8_pair")
     return hex8_pair_enabled() ? 1 : 0;
+  if(n == "mg_tail")
+    return mg_tail_enabled() ? 1 : 0;
+  if(n == "mg_restrict_planes")
+    return mg_restrict_planes();
   if(n == "hex8_far")
     return hex8_far_enabled() ? 1 : 0;
   if(n == "batch_fused")

@@ -3,6 +3,8 @@
 #include <atomic>
 
 #include "graphloop.hpp"
+#include "mg.hpp"
+#include "mgtail.cuh"
 
 namespace icb
 {
@@ -14,7 +16,8 @@ unsigned long long kernel_switches()
 {
   return (tc_operator_enabled() ? 1ull : 0ull) | (hex8_modal_enabled() ? 2ull : 0ull) |
          (device_loops_enabled() ? 4ull : 0ull) | (hex8_pair_enabled() ? 8ull : 0ull) |
-         (hex8_far_enabled() ? 16ull : 0ull) |
+         (hex8_far_enabled() ? 16ull : 0ull) | (mg_tail_enabled() ? 32ull : 0ull) |
+         ((unsigned long long)mg_restrict_planes() << 40) |
          ((unsigned long long)tc_spin_limit() << 8);
 }
 

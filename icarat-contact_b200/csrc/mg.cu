@@ -36,10 +36,16 @@
 // The whole V-cycle is a fixed kernel sequence, so one PCG iteration with
 // its V-cycle is captured as the body of a CUDA graph's conditional WHILE
 // node, which the device repeats until the stop flag is set.
+#include <atomic>
+
 #include "mg_impl.cuh"
 
 namespace icb
 {
+static std::atomic<int> g_restrict_planes{0};
+int mg_restrict_planes() { return g_restrict_planes; }
+void set_mg_restrict_planes(int n) { g_restrict_planes = n; }
+
 // ============================================================== Mixed ======
 /// r32 = float(s * r64): the outer residual, scaled to unit norm, as the
 /// right-hand side of the FP32 inner solve

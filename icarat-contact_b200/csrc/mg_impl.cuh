@@ -357,6 +357,8 @@ __global__ void __launch_bounds__(kTB)
 constexpr int kRestrictPlanes = 4;
 inline int restrict_planes(const dim3 &g)
 {
+  if(const int forced = mg_restrict_planes())
+    return forced;
   return (long long)g.x * g.y * ((g.z + kRestrictPlanes - 1) / kRestrictPlanes) >= 4 * num_sms()
              ? kRestrictPlanes
              : 1;
@@ -1400,8 +1402,9 @@ template <typename TK, typename TP> struct MgPcg
   /// CUDA-core corner-mode operator, which the process-wide switches may exclude
   bool useTail() const
   {
-    return tail0 >= 0 && (lv[0].d.dim == 2 ||
-                          (hex8_modal_enabled() && !(sizeof(TP) == 4 && tc_operator_enabled())));
+    return tail0 >= 0 && mg_tail_enabled() &&
+           (lv[0].d.dim == 2 ||
+            (hex8_modal_enabled() && !(sizeof(TP) == 4 && tc_operator_enabled())));
   }
   TailArgs<TP> tailArgs(const KState *gate) const
   {

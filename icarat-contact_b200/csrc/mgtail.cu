@@ -26,6 +26,7 @@
 #include "mgtail.cuh"
 
 #include <algorithm>
+#include <atomic>
 
 #include "hex8modal.cuh"
 #include "reduce.cuh"
@@ -552,6 +553,10 @@ template <typename Kern> void tail_optin(Kern kern)
   ICB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kTailSmem));
 }
 } // namespace
+
+static std::atomic<bool> g_mg_tail{true};
+bool mg_tail_enabled() { return g_mg_tail; }
+void set_mg_tail(bool on) { g_mg_tail = on; }
 
 template <typename T> bool tail_plan(TailArgs<T> &A)
 {

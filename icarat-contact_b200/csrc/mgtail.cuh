@@ -50,6 +50,9 @@ template <typename T> struct TailArgs
   const int *entry; ///< per coarsest unknown its entry in the padded vectors
   const KState *gate;
 };
+/// whether coarse levels run as one launch (option mg_tail, default on)
+bool mg_tail_enabled();
+void set_mg_tail(bool on);
 /// entries of TailK
 constexpr int tail_k(int dim) { return dim == 2 ? 64 : 45; }
 /// lay the levels out in shared memory; false when they do not fit

@@ -452,6 +452,9 @@ long long icb_launch_count(void);
  * of a tensor-core wait before it gives up),
  * "exchange_spin_limit" (polls of a wait between the blocks of a one-kernel
  * solve, filter or OC update before it ends with ICB_ERR_TIMEOUT),
+ * "mg_tail" (1, the default: a V-cycle's coarse levels as one launch; 0: each
+ * level's own), "mg_restrict_planes" (coarse planes a thread of the 3D
+ * restriction takes; 0, the default: by the grid's size),
  * "batch_fused" (icb_run_batch advances qualifying 2D OC batches together),
  * "batch_handoff" (a fused batch's solves hand the designs still iterating to
  * their own solve loops once at most this many are left; 0, the default: an
