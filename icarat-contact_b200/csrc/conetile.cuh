@@ -17,6 +17,7 @@ namespace icb
 {
 constexpr int kConeMaxHz = 4;        ///< largest half height of a column (unrolled loops)
 constexpr int kConeSmem = 100 << 10; ///< most shared memory of a tile (two CTAs per SM)
+constexpr int kConeMaxHalo = 256;     ///< no tile's halo is wider (keeps its size in an int)
 
 /// the stencil as columns, on the device
 struct ConeCols

@@ -1196,11 +1196,12 @@ ConeFilter::ConeFilter(const Dims &dims, const double *h, double radius, cudaStr
       cols.hy = std::max(cols.hy, dj);
       cols.hz = std::max(cols.hz, hk);
     }
+  const bool narrow = cols.hx <= kConeMaxHalo && cols.hy <= kConeMaxHalo;
   const bool fits =
       d.dim == 3 ? (d.ny + 7) / 8 <= 65535 && (d.nz + 3) / 4 <= 65535 &&
                        ConeTile<8>::cells(cols) * int(sizeof(double)) <= kConeSmem
                  : cols.hx <= kOcHalo;
-  if(cols.hz <= kConeMaxHz && fits)
+  if(cols.hz <= kConeMaxHz && narrow && fits)
   {
     cols.ncol = int(cc.size());
     nb4.insert(nb4.end(), cc.begin(), cc.end());
