@@ -149,33 +149,33 @@ __device__ __forceinline__ void restrict_b(Dims df, Dims dc, int3 sh, const T *_
     }
   }
   else
-  for(int dk = -kr; dk <= kr; dk++)
-  {
-    const int k = (K << sh.z) + dk;
-    if(k < 0 || k >= df.sz)
-      continue;
-    T sk[3] = {T(0), T(0), T(0)};
-    for(int dj = -sh.y; dj <= sh.y; dj++)
+    for(int dk = -kr; dk <= kr; dk++)
     {
-      const int j = (J << sh.y) + dj;
-      if(j < 0 || j >= df.sy)
+      const int k = (K << sh.z) + dk;
+      if(k < 0 || k >= df.sz)
         continue;
-      const long long row = (long long)j * df.sx + (long long)k * fsxy;
-      const int i = I << sh.x;
-      const bool lo = sh.x && i - 1 >= 0, mid = i < df.sx, hi = sh.x && i + 1 < df.sx;
+      T sk[3] = {T(0), T(0), T(0)};
+      for(int dj = -sh.y; dj <= sh.y; dj++)
+      {
+        const int j = (J << sh.y) + dj;
+        if(j < 0 || j >= df.sy)
+          continue;
+        const long long row = (long long)j * df.sx + (long long)k * fsxy;
+        const int i = I << sh.x;
+        const bool lo = sh.x && i - 1 >= 0, mid = i < df.sx, hi = sh.x && i + 1 < df.sx;
+#pragma unroll
+        for(int c = 0; c < 3; c++)
+          if(c < DIM)
+          {
+            const T *r = rf + c * df.ld + row;
+            const T v = (mid ? r[i] : T(0)) + h * ((lo ? r[i - 1] : T(0)) + (hi ? r[i + 1] : T(0)));
+            sk[c] = dj ? fma(h, v, sk[c]) : sk[c] + v;
+          }
+      }
 #pragma unroll
       for(int c = 0; c < 3; c++)
-        if(c < DIM)
-        {
-          const T *r = rf + c * df.ld + row;
-          const T v = (mid ? r[i] : T(0)) + h * ((lo ? r[i - 1] : T(0)) + (hi ? r[i + 1] : T(0)));
-          sk[c] = dj ? fma(h, v, sk[c]) : sk[c] + v;
-        }
+        s[c] = dk ? fma(h, sk[c], s[c]) : s[c] + sk[c];
     }
-#pragma unroll
-    for(int c = 0; c < 3; c++)
-      s[c] = dk ? fma(h, sk[c], s[c]) : s[c] + sk[c];
-  }
 #pragma unroll
   for(int c = 0; c < 3; c++)
     if(c < DIM)
@@ -1126,10 +1126,14 @@ template <typename TK, typename TP> struct MgPcg
   DevBuf<unsigned> counter;
   RedScratch red;
   KState *hst = nullptr;
-  /// the levels tail0 .. coarsest as one launch (mgtail.cu): its arguments
-  /// without the gate; tail0 < 0: none
-  int tail0 = -1;
-  TailArgs<TP> tail{};
+  /// the levels `from` .. coarsest as one launch (mgtail.cu): its arguments without the
+  /// gate; from < 0: none
+  struct Tail
+  {
+    int from = -1;
+    TailArgs<TP> args{};
+  };
+  Tail tail, batchTail; ///< of the solve alone, and in a batch
   TailK<TP> tailK{};
   DevBuf<int> tailEntry;
   WhileGraph loop; ///< one FCG iteration, repeated on the device until stop
@@ -1312,7 +1316,7 @@ template <typename TK, typename TP> struct MgPcg
   /// the levels' element matrices are powers of two times one another
   void buildTail(const std::vector<long long> &soa, cudaStream_t s)
   {
-    tail0 = -1;
+    tail.from = batchTail.from = -1;
     const int dim = lv[0].d.dim, KN = tail_k(dim), depth = int(lv.size());
     if(nu > kTailSmooth || depth < 2)
       return;
@@ -1337,7 +1341,7 @@ template <typename TK, typename TP> struct MgPcg
     for(int l = l0; l >= std::max(0, depth - kTailLevels); l--)
     {
       TailK<TP> k{};
-      if(lv[l].d.nnode > tail_nodes<TP>(dim) || !matrix(l, k))
+      if(!tail_level<TP>(lv[l].d, true) || !matrix(l, k))
         break;
       int e = 0;
       const double q = double(k.v[0]) / double(tailK.v[0]);
@@ -1350,65 +1354,72 @@ template <typename TK, typename TP> struct MgPcg
       l0 = l;
     }
     // the longest tail that fits one CTA's shared memory
-    for(; l0 <= depth - 2; l0++)
-    {
-      TailArgs<TP> A{};
-      A.dim = dim;
-      A.nlev = depth - l0;
-      A.nu = nu;
-      A.nc = nc;
-      for(int k = 0; k < nu; k++)
+    auto plan = [&](Tail &t, bool batch) {
+      for(int from = l0; from <= depth - 2; from++)
       {
-        A.c1[k] = TP(cc1[k]);
-        A.c2[k] = TP(cc2[k]);
-      }
-      for(int l = l0; l < depth; l++)
-      {
-        Level<TP> &L = lv[l];
-        TailLevel<TP> &t = A.lv[l - l0];
-        t.nx = L.d.nx, t.ny = L.d.ny, t.nz = L.d.nz;
-        t.sx = L.d.sx, t.sy = L.d.sy, t.sz = L.d.sz;
-        t.shx = L.sh.x, t.shy = L.sh.y, t.shz = dim == 3 ? L.sh.z : 0;
-        t.es = es[l];
-        t.ld = L.d.ld;
-        t.E = L.E;
-        t.dinv = L.dinv.p;
-      }
-      A.b = l0 ? lv[l0].b.p : rin();
-      A.out = l0 ? lv[l0].x.p : z.p;
-      A.Ainv = cA.p;
-      if(lv[l0].d.nnode <= tail_nodes<TP>(dim) && tail_plan(A))
-      {
-        std::vector<int> entry(std::max(nc, 1), 0);
-        const Dims &dc = lv.back().d;
-        for(int q = 0; q < nc; q++)
+        TailArgs<TP> A{};
+        A.dim = dim;
+        A.nlev = depth - from;
+        A.nu = nu;
+        A.nc = nc;
+        for(int k = 0; k < nu; k++)
         {
-          const long long c = soa[q] / dc.ld, nd = soa[q] % dc.ld;
-          entry[q] = tail_entry(A.lv[depth - 1 - l0], dim, int(c), int(nd % dc.sx),
-                                int(nd / dc.sx % dc.sy), int(nd / ((long long)dc.sx * dc.sy)));
+          A.c1[k] = TP(cc1[k]);
+          A.c2[k] = TP(cc2[k]);
         }
-        tailEntry.alloc(entry.size());
-        ICB_CUDA(cudaMemcpyAsync(tailEntry.p, entry.data(), sizeof(int) * entry.size(),
-                                 cudaMemcpyHostToDevice, s));
-        ICB_CUDA(cudaStreamSynchronize(s));
+        for(int l = from; l < depth; l++)
+        {
+          Level<TP> &L = lv[l];
+          TailLevel<TP> &v = A.lv[l - from];
+          v.nx = L.d.nx, v.ny = L.d.ny, v.nz = L.d.nz;
+          v.sx = L.d.sx, v.sy = L.d.sy, v.sz = L.d.sz;
+          v.shx = L.sh.x, v.shy = L.sh.y, v.shz = dim == 3 ? L.sh.z : 0;
+          v.es = es[l];
+          v.ld = L.d.ld;
+          v.E = L.E;
+          v.dinv = L.dinv.p;
+        }
+        A.b = from ? lv[from].b.p : rin();
+        A.out = from ? lv[from].x.p : z.p;
+        A.Ainv = cA.p;
         A.entry = tailEntry.p;
-        tail = A;
-        tail0 = l0;
-        return;
+        if(tail_level<TP>(lv[from].d, batch) && tail_plan(A))
+        {
+          t.from = from;
+          t.args = A;
+          return;
+        }
       }
+    };
+    tailEntry.alloc(std::max(nc, 1));
+    plan(tail, false);
+    plan(batchTail, true);
+    if(batchTail.from < 0) // neither: every tail alone is one in a batch
+      return;
+    std::vector<int> entry(std::max(nc, 1), 0);
+    const Dims &dc = lv.back().d;
+    const TailLevel<TP> &last = batchTail.args.lv[depth - 1 - batchTail.from];
+    for(int q = 0; q < nc; q++)
+    {
+      const long long c = soa[q] / dc.ld, nd = soa[q] % dc.ld;
+      entry[q] = tail_entry(last, dim, int(c), int(nd % dc.sx), int(nd / dc.sx % dc.sy),
+                            int(nd / ((long long)dc.sx * dc.sy)));
     }
+    ICB_CUDA(cudaMemcpyAsync(tailEntry.p, entry.data(), sizeof(int) * entry.size(),
+                             cudaMemcpyHostToDevice, s));
+    ICB_CUDA(cudaStreamSynchronize(s));
   }
   /// whether the tail stands for its levels' own launches: it runs the
   /// CUDA-core corner-mode operator, which the process-wide switches may exclude
-  bool useTail() const
+  bool useTail(const Tail &t) const
   {
-    return tail0 >= 0 && mg_tail_enabled() &&
+    return t.from >= 0 && mg_tail_enabled() &&
            (lv[0].d.dim == 2 ||
             (hex8_modal_enabled() && !(sizeof(TP) == 4 && tc_operator_enabled())));
   }
-  TailArgs<TP> tailArgs(const KState *gate) const
+  TailArgs<TP> tailArgs(const Tail &t, const KState *gate) const
   {
-    TailArgs<TP> A = tail;
+    TailArgs<TP> A = t.args;
     A.gate = gate;
     return A;
   }
@@ -1457,9 +1468,9 @@ template <typename TK, typename TP> struct MgPcg
   }
 
   /// level l's first smoothing step, when it runs as launches of its own
-  FirstStep<TP> firstStep(size_t l)
+  FirstStep<TP> firstStep(size_t l, const Tail &t)
   {
-    if(l + 1 >= lv.size() || (int(l) == tail0 && useTail()))
+    if(l + 1 >= lv.size() || (int(l) == t.from && useTail(t)))
       return FirstStep<TP>{TP(0), nullptr, nullptr};
     return FirstStep<TP>{TP(cc2[0]), lv[l].dinv.p, lv[l].t.p};
   }
@@ -1468,9 +1479,9 @@ template <typename TK, typename TP> struct MgPcg
   void level(size_t l, const TP *b, TP *out, cudaStream_t s, const KState *gate)
   {
     Level<TP> &L = lv[l];
-    if(int(l) == tail0 && useTail())
+    if(int(l) == tail.from && useTail(tail))
     {
-      launch_mg_tail(tailArgs(gate), tailK, s);
+      launch_mg_tail(tailArgs(tail, gate), tailK, s);
       return;
     }
     if(l + 1 == lv.size())
@@ -1511,11 +1522,11 @@ template <typename TK, typename TP> struct MgPcg
     {
       const int planes = restrict_planes(gr);
       gr.z = (gr.z + planes - 1) / planes;
-      k_restrict3<TP><<<gr, kTB, 0, s>>>(L.d, Cn.d, planes, L.r.p, Cn.b.p, Cn.fix, gate, firstStep(l + 1));
+      k_restrict3<TP><<<gr, kTB, 0, s>>>(L.d, Cn.d, planes, L.r.p, Cn.b.p, Cn.fix, gate, firstStep(l + 1, tail));
     }
     else
       (L.d.dim == 2 ? k_restrict<TP, 2> : k_restrict<TP, 3>)<<<gr, kTB, 0, s>>>(
-          L.d, Cn.d, Cn.sh, L.r.p, Cn.b.p, Cn.fix, gate, firstStep(l + 1));
+          L.d, Cn.d, Cn.sh, L.r.p, Cn.b.p, Cn.fix, gate, firstStep(l + 1, tail));
     count_launch();
     level(l + 1, Cn.b.p, Cn.x.p, s, gate);
     dim3 gp = grid3(L.d);
@@ -1553,7 +1564,7 @@ template <typename TK, typename TP> struct MgPcg
     a.gate = st.p;
     launch_op<TK>(d, Kk, Ek, p.p, q.p, lv[0].fix, s, a);
     k_mg_r<TK, TP><<<nb, VB, 0, s>>>(n, r.p, same() ? nullptr : rP.p, q.p, z.p, dots.p, red, st.p,
-                                      firstStep(0));
+                                      firstStep(0, tail));
     level(0, rin(), z.p, s, st.p);
     k_mg_rz<TK, TP><<<nb, VB, 0, s>>>(n, r.p, z.p, red, st.p);
     k_mg_xp<TK, TP><<<nb, VB, 0, s>>>(n, x, p.p, z.p, red, st.p, L);
@@ -1564,7 +1575,7 @@ template <typename TK, typename TP> struct MgPcg
   {
     int nb = vblocks(n);
     k_mg_init<TK, TP><<<nb, VB, 0, s>>>(n, b, x, r.p, same() ? nullptr : rP.p, red, st.p, tol,
-                                         maxit, firstStep(0));
+                                         maxit, firstStep(0, tail));
     count_launch();
     level(0, rin(), z.p, s, nullptr);
     k_mg_init2<TK, TP><<<nb, VB, 0, s>>>(n, r.p, z.p, p.p, red, st.p);

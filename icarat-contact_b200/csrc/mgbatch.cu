@@ -500,7 +500,7 @@ template <typename TP> struct BatchMg
   /// is its tail or its coarsest solve)
   size_t ownLevels(int i) const
   {
-    return M[i]->useTail() ? size_t(M[i]->tail0) : M[i]->lv.size() - 1;
+    return M[i]->useTail(M[i]->batchTail) ? size_t(M[i]->batchTail.from) : M[i]->lv.size() - 1;
   }
 
   /// append the batched steps of level(l, b, out) for the problems `set`, `left`
@@ -533,15 +533,15 @@ template <typename TP> struct BatchMg
       for(const Inst &I : coarse)
       {
         MG &m = *M[I.i];
-        if(m.useTail())
+        if(m.useTail(m.batchTail))
         {
           size_t g = 0;
           while(g < tails.size() && std::memcmp(&tails[g].K, &m.tailK, sizeof m.tailK))
             g++;
           if(g == tails.size())
             tails.push_back(Group{m.tailK, {}, 0});
-          tails[g].recs.push_back(m.tailArgs(gate(I.i)));
-          tails[g].smem = std::max(tails[g].smem, m.tail.smem);
+          tails[g].recs.push_back(m.tailArgs(m.batchTail, gate(I.i)));
+          tails[g].smem = std::max(tails[g].smem, m.batchTail.args.smem);
           continue;
         }
         const Level<TP> &C = m.lv.back();
@@ -563,7 +563,7 @@ template <typename TP> struct BatchMg
                                  cudaMemcpyHostToDevice, s));
         ICB_CUDA(cudaStreamSynchronize(s));
         push([D, nt, smem, K = t.K](cudaStream_t cs) {
-          launch_mg_tail_batch<TP>(D->p, nt, 2, smem, K, cs);
+          launch_mg_tail_batch<TP>(D->p, nt, smem, K, cs);
         });
       }
     }
@@ -632,7 +632,7 @@ template <typename TP> struct BatchMg
         op.add(L.d, L.K, L.E, cs[t].cur, L.r.p, L.fix, res);
         const dim3 g3 = grid3(Cn.d);
         rs.add(RestrictL<TP>{{}, L.d, Cn.d, Cn.sh, L.r.p, Cn.b.p, Cn.fix, gate(I.i), g3.y,
-                            m.firstStep(I.l + 1)},
+                            m.firstStep(I.l + 1, m.batchTail)},
                g3.x,
                transfer_rows(g3.y, kR), g3.z);
         next.push_back(Inst{I.i, Cn.b.p, Cn.x.p, I.l + 1});
@@ -792,7 +792,7 @@ template <typename TP> struct BatchMg
       {
         MG &m = *M[i];
         in.add(InitL<double, TP>{{}, m.n, b[i], x[i], m.r.p, MG::same() ? nullptr : m.rP.p, m.red,
-                                 m.st.p, tol[i], maxit[i], m.firstStep(0)},
+                                 m.st.p, tol[i], maxit[i], m.firstStep(0, m.batchTail)},
                unsigned(vblocks(m.n)));
         all.push_back(Inst{i, m.rin(), m.z.p, 0});
       }
@@ -825,7 +825,7 @@ template <typename TP> struct BatchMg
         a.gate = m.st.p;
         op.add(m.lv[0].d, m.Kk, m.Ek, m.p.p, m.q.p, m.lv[0].fix, a);
         rb.add(RL<double, TP>{{}, m.n, m.r.p, MG::same() ? nullptr : m.rP.p, m.q.p, m.z.p,
-                              m.dots.p, m.red, m.st.p, m.firstStep(0)},
+                              m.dots.p, m.red, m.st.p, m.firstStep(0, m.batchTail)},
                unsigned(vblocks(m.n)));
       }
       push(iter, op.finish(s, qc.p));

@@ -35,7 +35,8 @@ namespace icb
 {
 namespace
 {
-/// threads of the CTA: as many as 64 (FP32) or 128 (FP64) registers each allow
+/// threads of the CTA: as many as 64 (FP32) or 128 (FP64) registers each allow.  (The 3D
+/// FP64 form spills 268 bytes a thread at that.)
 template <typename T> constexpr int kTailThreads = sizeof(T) == 4 ? 1024 : 512;
 
 template <typename T, int DIM> struct TailVec;
@@ -539,11 +540,11 @@ __global__ void __launch_bounds__(kTailThreads<T>)
 {
   tail_body<T, DIM>(A, K);
 }
-template <typename T, int DIM>
+template <typename T>
 __global__ void __launch_bounds__(kTailThreads<T>)
     k_mg_tail_batch(const TailArgs<T> *__restrict__ D, const __grid_constant__ TailK<T> K)
 {
-  tail_body<T, DIM>(D[blockIdx.x], K);
+  tail_body<T, 2>(D[blockIdx.x], K);
 }
 
 /// the shared-memory opt-in: a per-device function attribute shared by every
@@ -617,19 +618,16 @@ template void launch_mg_tail<float>(const TailArgs<float> &, const TailK<float> 
 template void launch_mg_tail<double>(const TailArgs<double> &, const TailK<double> &, cudaStream_t);
 
 template <typename T>
-void launch_mg_tail_batch(const TailArgs<T> *D, int n, int dim, int smem, const TailK<T> &K,
+void launch_mg_tail_batch(const TailArgs<T> *D, int n, int smem, const TailK<T> &K,
                           cudaStream_t s)
 {
-  auto run = [&](auto kern) {
-    tail_optin(kern);
-    kern<<<n, kTailThreads<T>, smem, s>>>(D, K);
-  };
-  dim == 2 ? run(k_mg_tail_batch<T, 2>) : run(k_mg_tail_batch<T, 3>);
+  tail_optin(k_mg_tail_batch<T>);
+  k_mg_tail_batch<T><<<n, kTailThreads<T>, smem, s>>>(D, K);
   ICB_CUDA(cudaGetLastError());
   count_launch();
 }
-template void launch_mg_tail_batch<float>(const TailArgs<float> *, int, int, int,
+template void launch_mg_tail_batch<float>(const TailArgs<float> *, int, int,
                                           const TailK<float> &, cudaStream_t);
-template void launch_mg_tail_batch<double>(const TailArgs<double> *, int, int, int,
+template void launch_mg_tail_batch<double>(const TailArgs<double> *, int, int,
                                            const TailK<double> &, cudaStream_t);
 } // namespace icb

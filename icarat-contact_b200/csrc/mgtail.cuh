@@ -7,15 +7,28 @@ namespace icb
 {
 /// levels of a tail at most, and smoothing steps it takes
 constexpr int kTailLevels = 12, kTailSmooth = 8;
-/// shared memory of a tail, and most nodes of its first level.  A phase of the
-/// largest first levels takes about 2.1 us (2D FP64, 1281 nodes), 2.9 us (2D FP32,
-/// 3321) or 1.6 us (3D FP32, 396) on its one SM, a launch over the whole GPU 3.7 to
-/// 5 us at any of these sizes; the next finer level has four (2D) or eight (3D)
-/// times the nodes and would be slower here.
+/// shared memory of a tail
 constexpr int kTailSmem = 200 << 10;
-template <typename T> constexpr long long tail_nodes(int dim)
+/// Whether a tail may begin at this level.  A phase on one SM grows with the rounds its
+/// warps make, a launch over the whole GPU takes 3.7 to 5 us at any of these sizes.  In
+/// 2D a warp takes 32 nodes of a row: two rounds of the FP32 tail's 32 warps pay, three
+/// of the FP64 tail's 16.  Microseconds a PCG iteration with the tail beginning at the
+/// level and one level below it: FP32, two rounds, 56x26 nodes 68.6 and 70.1, 51x26 82.4
+/// and 84.1; three, 46x43 73.7 and 71.1; four, 51x49 80.1 and 75.6, 81x41 86.4 and 78.3;
+/// FP64, two rounds, 51x16 71.6 and 74.7; three, 31x41 74.9 and 75.5, 61x21 72.4 and 72.5;
+/// four, 34x32 61.9 and 59.1; five, 34x33 79.1 and 74.3.  In 3D a thread takes a node: 343
+/// nodes FP32 77.2 and 78.6, FP64 85.2 and 86.1; 468 FP32 78.6 and 79.6; 512 81.8 and
+/// 80.2, FP64 equal.
+///
+/// In a batch (2D) the tails of all designs are one launch, and a level above them costs
+/// eight more for the few designs that have one of its size: up to 3400 (FP32) or 1400
+/// (FP64) nodes there (8 designs 19.0 ms, with the rule above 20.0; 32 designs equal).
+template <typename T> inline bool tail_level(const Dims &d, bool batch)
 {
-  return dim == 2 ? (sizeof(T) == 4 ? 3400 : 1400) : 512;
+  if(d.dim == 3)
+    return d.nnode <= 480;
+  return (d.sx + 31LL) / 32 * d.sy <= (sizeof(T) == 4 ? 64 : 48) ||
+         (batch && d.nnode <= (sizeof(T) == 4 ? 3400 : 1400));
 }
 
 /// the element matrix (2D, 64 entries) or its corner-mode form (3D, 45) of the
@@ -62,9 +75,9 @@ template <typename T> int tail_entry(const TailLevel<T> &L, int dim, int c, int 
 /// one V-cycle tail on stream s
 template <typename T>
 void launch_mg_tail(const TailArgs<T> &A, const TailK<T> &K, cudaStream_t s);
-/// n tails (device records of one dimension and element matrix) as one launch;
+/// n tails of 2D problems (device records of one element matrix) as one launch;
 /// smem: the largest of the records
 template <typename T>
-void launch_mg_tail_batch(const TailArgs<T> *D, int n, int dim, int smem, const TailK<T> &K,
+void launch_mg_tail_batch(const TailArgs<T> *D, int n, int smem, const TailK<T> &K,
                           cudaStream_t s);
 } // namespace icb

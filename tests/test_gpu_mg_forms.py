@@ -1,7 +1,7 @@
 """The V-cycle's forms that claim one another's bits: the coarse levels as one launch
 against their own launches, on grids whose first tail level is the largest it takes
-and one past it (1400 nodes in 2D FP64, 3400 in 2D FP32, 512 in 3D), thin and odd
-ones, and a problem that is all tail; and the 3D restriction with one, two, four and
+and one past it (in 2D 48 rows of up to 32 nodes in FP64 and 64 in FP32, 480 nodes in
+3D), thin and odd ones, and a problem that is all tail; and the 3D restriction with one, two, four and
 five coarse planes a thread, on every parity of the axes and on a grid past the size
 where it takes four by itself."""
 import numpy as np
@@ -42,9 +42,10 @@ def solves(p, option, values, smooth=(0,)):
     return out
 
 
-@pytest.mark.parametrize("dims", [(34, 39), (35, 39), (57, 57), (58, 57), (68, 78), (71, 79),
+@pytest.mark.parametrize("dims", [(63, 23), (63, 24), (31, 47), (31, 48), (64, 15), (64, 16),
+                                  (63, 31), (63, 32), (31, 63), (31, 64), (126, 62), (57, 57), (68, 78),
                                   (120, 40), (61, 1), (9, 33), (24, 13), (333, 222),
-                                  (7, 7, 7), (8, 7, 7), (15, 15, 15), (16, 15, 15), (20, 10, 10),
+                                  (7, 9, 5), (7, 9, 6), (7, 7, 7), (15, 15, 15), (16, 15, 15), (20, 10, 10),
                                   (33, 9, 1), (7, 6, 5), (40, 21, 18)])
 def test_tail_has_the_bits_of_its_levels_launches(ctx, dims):
     p = build(ctx, dims)
