@@ -790,6 +790,90 @@ __global__ void __launch_bounds__(VB)
   }
 }
 
+/// The column form launch by launch, for designs of more tiles than k_oc_update takes:
+/// h and the bounds of every element once an update (nel each in prep), then a launch a
+/// step, a block a tile
+struct OcCols
+{
+  Dims d;
+  ConeCols cols;
+  const double *aa, *vol, *prep;
+  unsigned gx, ntx; ///< tiles, and along x
+  OcParams P;
+  RedScratch red;
+  OcState *st;
+};
+__global__ void k_oc_prep(long long nel, const double *__restrict__ x, const double *__restrict__ df,
+                          const double *__restrict__ dg, const double *__restrict__ xmin,
+                          const double *__restrict__ xmax, OcParams P, double *__restrict__ prep)
+{
+  const long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+  if(e >= nel)
+    return;
+  double h, lo, hi;
+  oc_prep(x[e], df[e], dg[e], xmin[e], xmax[e], P, h, lo, hi);
+  prep[e] = h;
+  prep[nel + e] = lo;
+  prep[2 * nel + e] = hi;
+}
+/// one bisection step on tiles b0 .. b0 + n - 1 in the column form (k_oc_update's
+/// arithmetic and sums): the candidates of a tile and its halo into shared memory, the
+/// volume, and in the update's last block its bisection logic.  R: OcCols, or a batch's
+/// record
+template <class R>
+__device__ __forceinline__ void oc_step_cols_b(const R &r, int b0, int n, double *buf,
+                                               const LoopCtl &L)
+{
+  const Dims &d = r.d;
+  const ConeCols &C = r.cols;
+  const double c = 1.0 / oc_power(r.st->lam, r.P.eta), tb = r.st->tanhTb;
+  const int W = kOcTW + 2 * C.hx, cells = oc_up_cells(C);
+  sum_runs<1, VB, true>(
+      b0, n, r.gx, r.red,
+      [&](const Blk &B, double(&v)[1]) {
+        const int x0 = int(B.x % r.ntx) * kOcTW, y0 = int(B.x / r.ntx) * kOcTH;
+        double aav[4], volv[4];
+        oc_tile_weights(d, x0 + int(threadIdx.x & 31), y0 + 4 * int(threadIdx.x >> 5), r.aa, r.vol,
+                        aav, volv);
+        if(int(B.x) != b0)
+          __syncthreads(); // the tile before is summed
+        constexpr int U = 4;
+        for(int q0 = threadIdx.x; q0 < cells; q0 += VB * U)
+        {
+          double h[U], lo[U], hi[U];
+#pragma unroll
+          for(int u = 0; u < U; u++)
+          {
+            const int q = q0 + u * VB, ty = q / W, i = x0 - C.hx + q - ty * W, j = y0 - C.hz + ty;
+            const bool in = q < cells && unsigned(i) < unsigned(d.nx) && unsigned(j) < unsigned(d.ny);
+            const long long e = i + (long long)j * d.nx;
+            h[u] = in ? __ldg(r.prep + e) : 0.0;
+            lo[u] = in ? __ldg(r.prep + d.nel + e) : 0.0;
+            hi[u] = in ? __ldg(r.prep + 2 * d.nel + e) : 0.0;
+          }
+#pragma unroll
+          for(int u = 0; u < U; u++)
+            if(q0 + u * VB < cells)
+              buf[q0 + u * VB] = oc_bounded(h[u] * c, lo[u], hi[u]);
+        }
+        __syncthreads();
+        v[0] = oc_tile_volume(buf, W, C, aav, volv, r.P, tb);
+      },
+      FinOc{r.st, L});
+}
+
+__global__ void __launch_bounds__(VB) k_oc_step_cols(const __grid_constant__ OcCols r, LoopCtl L)
+{
+  extern __shared__ __align__(16) double oc_cols_dyn[];
+  if(r.st->done)
+  {
+    if(blockIdx.x == 0 && threadIdx.x == 0)
+      loop_stop(L);
+    return;
+  }
+  oc_step_cols_b(r, int(blockIdx.x), 1, oc_cols_dyn, L);
+}
+
 // ----------------------------------------------------------------- MMA ----
 /// GenSub (MMASolver.cpp:400-512) for m = 1: asymptotes, move bounds, p0,
 /// q0, p, q; the constraint constant b = -g + sum(p/(U-x) + q/(x-L)) is
@@ -1286,9 +1370,7 @@ int oc_update_tiles(const Dims &d)
 }
 /// the one-kernel update's CTAs (no more than tiles or SMs) and shared memory: two
 /// buffers of candidates and three values a cell of its tiles.  ctas 0: the update
-/// runs as a graph (3D, too many tiles, a stencil too large).  Batched updates
-/// take the column form where a run alone is this kernel, and only there, so that
-/// both form every volume by the same operations
+/// runs as a graph (3D, too many tiles, a stencil too large)
 struct OcOneKernel
 {
   int ctas = 0, smem = 0;
@@ -1303,6 +1385,12 @@ OcOneKernel oc_one_kernel(const Dims &d, const ConeFilter *cone)
   r.smem = int(sizeof(double)) * oc_up_cells(cone->cols) * (2 + 3 * ((tiles + ctas - 1) / ctas));
   r.ctas = r.smem <= kOcUpSmem ? ctas : 0;
   return r;
+}
+/// whether a design's updates take the column form, as one kernel, step by step or in a
+/// batch: all three form every volume by the same operations and add the tiles alike
+bool oc_columns(const Dims &d, const ConeFilter *cone)
+{
+  return d.dim == 2 && cone && cone->cols.ncol;
 }
 } // namespace
 
@@ -1386,6 +1474,17 @@ void OcUpdater::launch(const ConeFilter *cone, double *x, const double *df, cons
   Pp.useFilter = cone != nullptr;
   const OcTiling tl = oc_tiling(d, cone);
   const int sb = tl.tiled ? tl.blocks : nb;
+  const bool cols = oc_columns(d, cone);
+  const int colSmem = cols ? int(sizeof(double)) * oc_up_cells(cone->cols) : 0;
+  OcCols rc{};
+  if(cols)
+  {
+    if(!prep.p)
+      prep.alloc(3 * size_t(d.nel));
+    k_oc_prep<<<unsigned((d.nel + 255) / 256), 256, 0, s>>>(d.nel, x, df, dg, xmin, xmax, Pp, prep.p);
+    count_launch();
+    rc = OcCols{d, cone->cols, aa, vol, prep.p, unsigned(tl.blocks), tl.ntx, Pp, red, st.p};
+  }
   // graph of the bisection: one step as the body of a conditional WHILE node
   // that the device repeats until done (at most maxiter = 100 steps), rebuilt
   // when anything it bakes in changes -- the stencil's device buffers and
@@ -1394,12 +1493,17 @@ void OcUpdater::launch(const ConeFilter *cone, double *x, const double *df, cons
   const bool dev = device_loops_enabled();
   GraphKey k;
   k.add(off).add(w).add(aa).add((long long)nnb).add(x).add(df).add(dg).add(xmin).add(xmax);
-  k.add(vol).add(cand.p).add((const void *)s).addBytes(Pp).add((long long)kernel_switches());
+  k.add(vol).add(cand.p).add(prep.p).add((const void *)s).addBytes(Pp).add((long long)kernel_switches());
   if(loop.exec == nullptr || loop.device != dev || k != key)
   {
     // host form: all of ICARAT's 100 steps in one launch, gated after done
     loop.build(
         [&](cudaStream_t cs, const LoopCtl &L) {
+          if(cols)
+          {
+            k_oc_step_cols<<<sb, VB, colSmem, cs>>>(rc, L);
+            return;
+          }
           if(Pp.useFilter)
             k_oc_cand<<<nb, VB, 0, cs>>>(d.nel, x, df, dg, xmin, xmax, Pp, st.p, cand.p);
           if(tl.tiled)
@@ -1471,49 +1575,6 @@ __global__ void __launch_bounds__(VB)
         }
       });
 }
-/// one bisection step on tiles b0 .. b0 + n - 1 in the column form (k_oc_update's
-/// arithmetic): the candidates of a tile and its halo into shared memory, the
-/// volume, and in a problem's last block its bisection logic
-__device__ __forceinline__ void oc_step_cols_b(const OcBatch::Rec &r, int b0, int n, double *buf)
-{
-  const Dims &d = r.d;
-  const ConeCols &C = r.cols;
-  const double c = 1.0 / oc_power(r.st->lam, r.P.eta), tb = r.st->tanhTb;
-  const int W = kOcTW + 2 * C.hx, cells = oc_up_cells(C);
-  sum_runs<1, VB, true>(
-      b0, n, r.gx, r.red,
-      [&](const Blk &B, double(&v)[1]) {
-        const int x0 = int(B.x % r.ntx) * kOcTW, y0 = int(B.x / r.ntx) * kOcTH;
-        double aav[4], volv[4];
-        oc_tile_weights(d, x0 + int(threadIdx.x & 31), y0 + 4 * int(threadIdx.x >> 5), r.aa, r.vol,
-                        aav, volv);
-        if(int(B.x) != b0)
-          __syncthreads(); // the tile before is summed
-        constexpr int U = 4;
-        for(int q0 = threadIdx.x; q0 < cells; q0 += VB * U)
-        {
-          double h[U], lo[U], hi[U];
-#pragma unroll
-          for(int u = 0; u < U; u++)
-          {
-            const int q = q0 + u * VB, ty = q / W, i = x0 - C.hx + q - ty * W, j = y0 - C.hz + ty;
-            const bool in = q < cells && unsigned(i) < unsigned(d.nx) && unsigned(j) < unsigned(d.ny);
-            const long long e = i + (long long)j * d.nx;
-            h[u] = in ? __ldg(r.prep + e) : 0.0;
-            lo[u] = in ? __ldg(r.prep + d.nel + e) : 0.0;
-            hi[u] = in ? __ldg(r.prep + 2 * d.nel + e) : 0.0;
-          }
-#pragma unroll
-          for(int u = 0; u < U; u++)
-            if(q0 + u * VB < cells)
-              buf[q0 + u * VB] = oc_bounded(h[u] * c, lo[u], hi[u]);
-        }
-        __syncthreads();
-        v[0] = oc_tile_volume(buf, W, C, aav, volv, r.P, tb);
-      },
-      FinOc{r.st, LoopCtl{}});
-}
-
 __global__ void k_oc_init_batch(const OcBatch::Rec *__restrict__ R, int n)
 {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -1541,7 +1602,7 @@ __global__ void __launch_bounds__(VB, 4)
       [](const OcBatch::Rec &r, int b0, int n) {
         if(r.cols.ncol)
         {
-          oc_step_cols_b(r, b0, n, reinterpret_cast<double *>(oc_batch_dyn));
+          oc_step_cols_b(r, b0, n, reinterpret_cast<double *>(oc_batch_dyn), LoopCtl{});
           return;
         }
         for(int b = b0; b < b0 + n; b++)
@@ -1609,7 +1670,7 @@ void OcBatch::build(const std::vector<OcBatchItem> &items, cudaStream_t s)
   std::vector<int2> ms, mc, mp, mf;
   smemStep = 0;
   size_t np = 0;
-  auto columns = [](const OcBatchItem &it) { return oc_one_kernel(it.oc->d, it.cone).ctas > 0; };
+  auto columns = [](const OcBatchItem &it) { return oc_columns(it.oc->d, it.cone); };
   for(const OcBatchItem &it : items)
     np += columns(it) ? 3 * size_t(it.oc->d.nel) : 0;
   prep.alloc(std::max<size_t>(np, 1));

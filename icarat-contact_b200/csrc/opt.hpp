@@ -60,6 +60,7 @@ struct OcUpdater
   DevBuf<unsigned> counter;
   RedScratch red;
   DevBuf<double> cand; ///< the candidates x+(lambda) of the current step
+  DevBuf<double> prep; ///< what the column form's steps read, when it runs launch by launch
   OcState *hst = nullptr;
   WhileGraph loop; ///< one bisection step, repeated on the device until done
   GraphKey key;     ///< what `loop` bakes in
@@ -90,7 +91,8 @@ struct OcBatchItem
 /// The OC updates of many problems as batched launches (opt.cu): the init,
 /// every bisection step and the final candidate each launched once for all
 /// problems through the work queue; each problem's blocks run exactly its own
-/// update's blocks, so its design is bitwise that of OcUpdater::update.
+/// update's blocks or, in the column form, its tiles in the same order, so its design is
+/// bitwise that of OcUpdater::update.
 struct OcBatch
 {
   struct Rec; ///< one problem's step launch (opt.cu)
