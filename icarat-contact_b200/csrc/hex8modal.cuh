@@ -13,7 +13,7 @@
 // are its null rows.  So  K0 u = H (Kt (H u))  costs two butterflies and 45
 // FMAs instead of 576.  The host builds Kt from K0 and checks that every entry
 // outside the blocks vanishes (to rounding); an element matrix that fails the
-// check runs on the dense kernel above.
+// check runs on the dense kernel (operator.cu).
 //
 // The marching column shares the butterflies between layers: the x-y half of
 // the transform is applied once per node plane (the top plane of element k is

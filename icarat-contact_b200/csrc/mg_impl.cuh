@@ -503,8 +503,9 @@ constexpr int kInvThreads = 512; ///< its CTA: 16 warps
 /// one barrier -- the warp that owns row k divides it by the pivot and puts it
 /// in shared memory, every warp takes column k's entries of its own rows by
 /// shuffle and updates them (with the matrix in shared memory and three
-/// barriers a step it took 333 us at n = 132; now 127 us.  Dividing the next
-/// row ahead of the other rows' updates took 139 us: more registers, spills).
+/// barriers a step it took 333 us at n = 132; now 127 us, though 128 registers a
+/// thread spill 460 bytes of the largest form.  Dividing the next row ahead of the
+/// other rows' updates took 139 us: it spills more).
 /// The loops over column blocks and row halves are unrolled, so every index
 /// into a is a constant.
 template <int NB>

@@ -1592,6 +1592,7 @@ __global__ void __launch_bounds__(VB, 4)
                       (long long)b * VB * kCandPerThread);
       });
 }
+/// (at four CTAs an SM 64 registers a thread spill 108 bytes)
 __global__ void __launch_bounds__(VB, 4)
     k_oc_step_batch(const OcBatch::Rec *__restrict__ R, const int2 *__restrict__ map, BatchQueue q)
 {

@@ -49,7 +49,7 @@ namespace icb
 namespace
 {
 /// threads of a CTA: one a node in 2D; in 3D two, one for the four elements
-/// below the node and one for the four above
+/// below the node and one for the four above (168 registers a thread: 160 bytes spill)
 template <int DIM> constexpr int kThreads = DIM == 3 ? 384 : 256;
 template <int DIM> constexpr int kNodeThreads = DIM == 3 ? 192 : 256;
 /// of the scalar form: one a node, as many as an exchange takes
