@@ -55,8 +55,10 @@ template <int DIM> constexpr int kNodeThreads = DIM == 3 ? 192 : 256;
 /// of the scalar form: one a node, as many as an exchange takes
 constexpr int kScalarThreads = 512;
 constexpr int kTileSmem = 200 << 10, kScalarSmem = 226 << 10;
-/// boxes of a CTA at most, and their shared memory (their sums take some more)
-constexpr int kTileShare = 8, kShareSmem = 222 << 10;
+/// boxes of a CTA at most, and their shared memory (their sums take some more).  With
+/// more solves in flight than that some wait, which beats more boxes: eight solves on
+/// 60x20x20 5.0 us an iteration and solve with up to four, 5.7 with up to eight
+constexpr int kTileShare = 4, kShareSmem = 222 << 10;
 
 template <int DIM> struct ElemK;
 template <> struct ElemK<2>
@@ -656,12 +658,12 @@ PcgTiles pcg_tiles(const Dims &d)
 /// SMs.  The cut for one solve fills the chip, so that a second one would wait for it.
 /// Microseconds an iteration and solve, with 1, 2, 4 and 8 threads solving: one box a
 /// CTA always, this rule, and three kernels an iteration
-///   40x15x15   7.2 7.0 6.9 6.9    7.0  5.2  3.4  3.9   16.5  9.4  5.4  3.4
-///   60x20x20   7.8 7.6 7.5 7.5    7.8  6.6  5.4  5.6   18.1 11.0  6.3  4.5
+///   40x15x15   7.2 7.0 6.9 6.9    7.0  5.2  3.4  3.4   16.5  9.4  5.4  3.4
+///   60x20x20   7.8 7.6 7.5 7.5    7.8  6.6  5.4  5.0   18.1 11.0  6.3  4.5
 ///   50x30x30  10.4 10.1 10.0 10.0 10.3  8.8  8.7  8.3  21.9 13.0  8.1  6.8
 ///   40x40x40  12.5 12.2 12.2 12.2 12.5 10.5 10.5 10.0  24.2 14.7 10.5 10.3
-///   300x100    5.8 5.6 5.6 5.6    5.8  5.2  3.8  4.0   16.6  9.0  5.3  3.5
-///   120x40     5.0 2.6 1.7 1.7    4.8  2.5  1.8  1.7   15.9  8.4  4.3  2.4
+///   300x100    5.8 5.6 5.6 5.6    5.8  5.2  3.8  3.9   16.6  9.0  5.3  3.5
+///   120x40     5.0 2.6 1.7 1.7    4.8  2.5  1.8  1.8   15.9  8.4  4.3  2.4
 /// Boxes of more than half of kShareSmem (3D grids of more than 70k nodes or so, 2D ones
 /// of more than 150k) stay alone on an SM: 48x46x45 16.4 with any number, three kernels
 /// 27.3, 17.0, 12.6 and 13.0; 540x540 10.2, three kernels 32.2, 18.8, 15.1, 16.6.
@@ -698,7 +700,9 @@ static void run_tiles(const PcgTiles &t, const Dims &d, const typename TileOp<DI
                       const double *E, const double *invdiag, double *x, double *r, double *p,
                       double *z, KState *st, int jobs, cudaStream_t s)
 {
-  const int share = tile_share(t, jobs);
+  // a filter call is more copies and host time than solve: half of those in flight are
+  // on the device at once (80x40x40, 2 threads: 250 us a call, 293 counting all)
+  const int share = tile_share(t, NC == DIM ? jobs : jobs / 2);
   (share > 1 ? run_tiles_as<DIM, NC, true> : run_tiles_as<DIM, NC, false>)(
       t, share, d, K, E, invdiag, x, r, p, z, st, s);
 }
